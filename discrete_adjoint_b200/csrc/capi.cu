@@ -467,6 +467,8 @@ int da_selftest_barrier(da_ctx *ctx, int32_t limit_us) {
     const int st3 = cuda_check(ctx, cudaStreamSynchronize(ctx->stream), "sync");
     return st2 ? st2 : (st3 ? st3 : code);
 }
+    if (ctx->stats_mem) cudaFree(ctx->stats_mem);
+    if (ctx->stats_host) cudaFreeHost(ctx->stats_host);
 
 int da_set_params(da_ctx *ctx, const da_params *p) {
     if (!ctx) return DA_ERR_INVALID;

@@ -198,6 +198,8 @@ struct da_ctx {
     int ntiles = 0;                  // tiles of 256 consecutive cells
     int nblocks = 0;                 // grid of the seed kernel (fixed at allocation)
     int grid = 0;                    // grid of the tiled step kernels (da_params.grid_blocks)
+    double *stats_mem = nullptr;      // partial sums and result of the flow statistics (stats.cu)
+    double *stats_host = nullptr;     // pinned copy of the result
     // resident blocks of k_steps [FP32, FP64] x [single, ensemble] x [2, 3 per SM] x [staged] x
     // [checkpoint stores inside the launch]
     int coop_cap[32] = {};

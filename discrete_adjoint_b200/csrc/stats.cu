@@ -1,9 +1,12 @@
 // Flow statistics of the current state (calc_stats, src/geoflow/stats.C:31-360) and the
 // discharge through planes (DISCHARGE::update, src/header/properties.h:964-1133), on the device.
 //
-// One pass over the cells: block b of kParts sums a fixed contiguous range of cells (thread-strided,
-// then thread 0 over the threads in order), a final block adds the parts in order: FP64 sums in a
-// fixed order (the reference sums in hash-table order, so the two agree to rounding).
+// One launch, one pass over the cells: block b of kParts sums a fixed contiguous range of cells
+// (thread-strided, then a shuffle tree per warp, then the warps in order), the last block to finish
+// adds the parts (a warp per value): FP64 sums in a fixed order (the reference sums in hash-table
+// order, so the two agree to rounding).  The pass is a latency chain at ordinary sizes, not
+// bandwidth; summing the block's 256 values by one thread, and the 256 parts by one thread of a
+// second launch, took most of it.
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -22,7 +25,39 @@ constexpr int kParts = 256;
 constexpr int kSums = 14;   // xC yC rC area v_ave vx_ave vy_ave slope_ave energy slopevol testvol xVar yVar u_ave
 constexpr int kMax = 3;     // max_height v_max u_max
 constexpr int kMin = 4;     // xmin, -xmax, ymin, -ymax (over h >= hxyminmax)
-constexpr int kPartLen = kSums + kMax + kMin + 2 + DA_MAX_PLANES;  // + test point (dist2, reach)
+constexpr int kPoint = kSums + kMax + kMin;  // test point: squared distance, reach
+constexpr int kPlane0 = kPoint + 2;          // discharge per plane
+constexpr int kPartLen = kPlane0 + DA_MAX_PLANES;
+constexpr int kResPlane0 = 24;               // the result: 23 statistics, then the planes
+constexpr int kResLen = kResPlane0 + DA_MAX_PLANES;
+
+enum SlotOp { kAdd, kTakeMax, kTakeMin };
+__device__ __forceinline__ int slot_op(int q) {
+    return q < kSums ? kAdd : (q < kSums + kMax ? kTakeMax : (q < kPoint ? kTakeMin : kAdd));
+}
+__device__ __forceinline__ double combine(int op, double a, double b) {
+    return op == kAdd ? a + b : (op == kTakeMax ? (b > a ? b : a) : (b < a ? b : a));
+}
+// the nearer test-point candidate (a tie takes the higher reach)
+__device__ __forceinline__ void take_point(double &d, double &r, double d2, double r2) {
+    if (d2 < d || (d2 == d && r2 > r)) {
+        d = d2;
+        r = r2;
+    }
+}
+template <int OP>
+__device__ __forceinline__ double warp_pick(double v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = combine(OP, v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+__device__ __forceinline__ void warp_point(double &d, double &r) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const double d2 = __shfl_xor_sync(0xffffffffu, d, o), r2 = __shfl_xor_sync(0xffffffffu, r, o);
+        take_point(d, r, d2, r2);
+    }
+}
 
 struct StatArgs {
     double min_height, hxyminmax, heightifreach, tx, ty;
@@ -40,7 +75,7 @@ __device__ double plane_flux(const double nodes[9][2], double hu, double hv, con
                          fabs(nodes[7][0] - nodes[5][0]) + fabs(nodes[7][1] - nodes[5][1])) *
                         0.25;
     const double half2 = half * half;
-    const double err = half / pow(2.0, 19.0);
+    const double err = half / 524288.0;
     for (int c1 = 0; c1 < 4; ++c1) {
         const int c2 = (c1 + 1) % 4;
         dxn[c1] = nodes[c2][0] - nodes[c1][0];
@@ -105,18 +140,18 @@ __device__ double plane_flux(const double nodes[9][2], double hu, double hv, con
 }
 
 template <class R>
-__global__ void __launch_bounds__(kBlock) k_stats_parts(MeshArgs m, StateRef<R> U, StatArgs a, double *parts) {
-    __shared__ double sh[kBlock];
+__global__ void __launch_bounds__(kBlock) k_stats(MeshArgs m, StateRef<R> U, StatArgs a, double vslump, double *parts,
+                                                  unsigned *done, double *res) {
     // the owned cells (a subdomain's ghosts are another subdomain's)
     const int per = (m.n_owned + kParts - 1) / kParts;
     const int i0 = blockIdx.x * per, i1 = min(m.n_owned, i0 + per);
     double s[kSums] = {}, mx[kMax] = {}, mn[kMin], dis[DA_MAX_PLANES] = {};
     for (int q = 0; q < kMin; ++q) mn[q] = HUGE_VAL;
-    double tdist = pow(2.0, 30.0), treach = 0.0;  // stats.C:58
+    double tdist = 1073741824.0, treach = 0.0;  // stats.C:58
     for (int i = i0 + threadIdx.x; i < i1; i += kBlock) {
         const double h = double(U.h[i]), hu = double(U.hu[i]), hv = double(U.hv[i]);
         const double x = m.x[i], y = m.y[i], dx = m.dx ? m.dx[i] : double(m.fdx[i]), dy = m.dy ? m.dy[i] : double(m.fdy[i]);
-        if (a.n_planes > 0) {
+        if (a.n_planes > 0 && (hu != 0.0 || hv != 0.0)) {  // no momentum, no flux through a plane
             double nodes[9][2] = {{x - 0.5 * dx, y - 0.5 * dy}, {x + 0.5 * dx, y - 0.5 * dy}, {x + 0.5 * dx, y + 0.5 * dy},
                                   {x - 0.5 * dx, y + 0.5 * dy}, {x, y - 0.5 * dy},             {x + 0.5 * dx, y},
                                   {x, y + 0.5 * dy},             {x - 0.5 * dx, y},             {x, y}};
@@ -167,96 +202,134 @@ __global__ void __launch_bounds__(kBlock) k_stats_parts(MeshArgs m, StateRef<R> 
             s[9] += dV;
         }
     }
-    // the block's values in thread order
-    double *out = parts + (size_t)blockIdx.x * kPartLen;
-    auto reduce = [&](double v, int slot, int op) {
-        __syncthreads();
-        sh[threadIdx.x] = v;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double r = sh[0];
-            for (int t = 1; t < kBlock; ++t)
-                r = op == 0 ? r + sh[t] : (op == 1 ? (sh[t] > r ? sh[t] : r) : (sh[t] < r ? sh[t] : r));
-            out[slot] = r;
-        }
-    };
-    for (int q = 0; q < kSums; ++q) reduce(s[q], q, 0);
-    for (int q = 0; q < kMax; ++q) reduce(mx[q], kSums + q, 1);
-    for (int q = 0; q < kMin; ++q) reduce(mn[q], kSums + kMax + q, 2);
-    for (int p = 0; p < a.n_planes; ++p) reduce(dis[p], kSums + kMax + kMin + 2 + p, 0);
-    // test point: the smallest distance; its reach (a tie takes the higher reach)
+    // The block's values: each warp by shuffles, then the warps' values in order.  parts[slot][block].
+    __shared__ double sh[kPartLen + 1][kBlock / 32];
+    __shared__ bool last;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int q = 0; q < kSums; ++q) {
+        const double v = warp_sum(s[q]);
+        if (lane == 0) sh[q][warp] = v;
+    }
+#pragma unroll
+    for (int q = 0; q < kMax; ++q) {
+        const double v = warp_pick<kTakeMax>(mx[q]);
+        if (lane == 0) sh[kSums + q][warp] = v;
+    }
+#pragma unroll
+    for (int q = 0; q < kMin; ++q) {
+        const double v = warp_pick<kTakeMin>(mn[q]);
+        if (lane == 0) sh[kSums + kMax + q][warp] = v;
+    }
+    warp_point(tdist, treach);
+    if (lane == 0) {
+        sh[kPoint][warp] = tdist;
+        sh[kPoint + 1][warp] = treach;
+    }
+    for (int p = 0; p < a.n_planes; ++p) {
+        const double v = warp_sum(dis[p]);
+        if (lane == 0) sh[kPlane0 + p][warp] = v;
+    }
     __syncthreads();
-    sh[threadIdx.x] = tdist;
-    __shared__ double rr[kBlock];
-    rr[threadIdx.x] = treach;
+    const int nslot = kPlane0 + a.n_planes;
+    for (int q = threadIdx.x; q < nslot; q += kBlock) {
+        if (q == kPoint + 1) continue;  // with its distance
+        double v = sh[q][0], r = q == kPoint ? sh[q + 1][0] : 0.0;
+        for (int w = 1; w < kBlock / 32; ++w) {
+            if (q == kPoint)
+                take_point(v, r, sh[q][w], sh[q + 1][w]);
+            else
+                v = combine(slot_op(q), v, sh[q][w]);
+        }
+        parts[(size_t)q * kParts + blockIdx.x] = v;
+        if (q == kPoint) parts[(size_t)(q + 1) * kParts + blockIdx.x] = r;
+    }
+    // the last block to finish adds the blocks' parts (a warp per slot: lane l takes parts l, l + 32,
+    // ... in order, then a shuffle tree) and forms the statistics
     __syncthreads();
     if (threadIdx.x == 0) {
-        double d = sh[0], r = rr[0];
-        for (int t = 1; t < kBlock; ++t)
-            if (sh[t] < d || (sh[t] == d && rr[t] > r)) {
-                d = sh[t];
-                r = rr[t];
-            }
-        out[kSums + kMax + kMin] = d;
-        out[kSums + kMax + kMin + 1] = r;
+        __threadfence();
+        last = atomicAdd(done, 1u) == gridDim.x - 1;
     }
-}
-
-__global__ void k_stats_final(const double *parts, int n_planes, double vslump, double d_time, double *res,
-                              double *discharge) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    double s[kSums] = {}, mx[kMax] = {}, mn[kMin], dis[DA_MAX_PLANES] = {};
-    for (int q = 0; q < kMin; ++q) mn[q] = HUGE_VAL;
-    double d = pow(2.0, 30.0), reach = 0.0;
-    for (int b = 0; b < kParts; ++b) {
-        const double *p = parts + (size_t)b * kPartLen;
-        for (int q = 0; q < kSums; ++q) s[q] += p[q];
-        for (int q = 0; q < kMax; ++q) mx[q] = p[kSums + q] > mx[q] ? p[kSums + q] : mx[q];
-        for (int q = 0; q < kMin; ++q) mn[q] = p[kSums + kMax + q] < mn[q] ? p[kSums + kMax + q] : mn[q];
-        const double pd = p[kSums + kMax + kMin], pr = p[kSums + kMax + kMin + 1];
-        if (pd < d || (pd == d && pr > reach)) {
-            d = pd;
-            reach = pr;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    for (int q = warp; q < nslot; q += kBlock / 32) {
+        if (q == kPoint + 1) continue;
+        const double *pq = parts + (size_t)q * kParts;
+        double v = __ldcg(pq + lane), r = q == kPoint ? __ldcg(pq + kParts + lane) : 0.0;
+        for (int b = lane + 32; b < kParts; b += 32) {
+            if (q == kPoint)
+                take_point(v, r, __ldcg(pq + b), __ldcg(pq + kParts + b));
+            else
+                v = combine(slot_op(q), v, __ldcg(pq + b));
         }
-        for (int q = 0; q < n_planes; ++q) dis[q] += p[kSums + kMax + kMin + 2 + q];
+        const int op = slot_op(q);
+        if (q == kPoint)
+            warp_point(v, r);
+        else if (op == kTakeMax)
+            v = warp_pick<kTakeMax>(v);
+        else if (op == kTakeMin)
+            v = warp_pick<kTakeMin>(v);
+        else
+            v = warp_sum(v);
+        if (lane == 0) {
+            sh[q][0] = v;
+            if (q == kPoint) sh[q + 1][0] = r;
+        }
     }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    *done = 0u;
+    auto S = [&](int q) { return sh[q][0]; };
     // stats.C:271-302 with LENGTH_SCALE = HEIGHT_SCALE = velocity scale = 1
-    const double tv = s[10];
-    res[0] = s[0] / tv;                      // xcen
-    res[1] = s[1] / tv;                      // ycen
-    res[2] = s[11] / tv - res[0] * res[0];   // xvar
-    res[3] = s[12] / tv - res[1] * res[1];   // yvar
-    res[4] = s[2] / tv;                      // rmean
-    res[5] = s[3];                           // area
-    res[6] = s[4] / tv;                      // vmean
-    res[7] = s[13] / tv;                     // umean
-    res[8] = s[5] / tv;                      // vxmean
-    res[9] = s[6] / tv;                      // vymean
-    res[10] = s[9] > 0 ? s[7] / s[9] : 0.0;  // slopemean
+    const double tv = S(10);
+    res[0] = S(0) / tv;                      // xcen
+    res[1] = S(1) / tv;                      // ycen
+    res[2] = S(11) / tv - res[0] * res[0];   // xvar
+    res[3] = S(12) / tv - res[1] * res[1];   // yvar
+    res[4] = S(2) / tv;                      // rmean
+    res[5] = S(3);                           // area
+    res[6] = S(4) / tv;                      // vmean
+    res[7] = S(13) / tv;                     // umean
+    res[8] = S(5) / tv;                      // vxmean
+    res[9] = S(6) / tv;                      // vymean
+    res[10] = S(9) > 0 ? S(7) / S(9) : 0.0;  // slopemean
     res[11] = tv;                            // statvolume
     res[12] = 3.0 * sqrt(res[2] + res[3]);   // piler
-    res[13] = mx[0];                         // hmax
-    res[14] = mx[1];                         // vmax
-    res[15] = mx[2];                         // umax
-    res[16] = vslump != 0 ? res[6] / vslump : 0.0;  // vstar
-    res[17] = mn[0];
-    res[18] = -mn[1];
-    res[19] = mn[2];
-    res[20] = -mn[3];
-    res[21] = reach;
-    res[22] = s[8];                          // the energy sum stats.C reduces in its "adjoint" slot
-    for (int q = 0; q < n_planes; ++q) discharge[q] += d_time * dis[q];
+    for (int q = 0; q < kMax; ++q) res[13 + q] = S(kSums + q);  // hmax vmax umax
+    res[16] = vslump != 0 ? res[6] / vslump : 0.0;              // vstar
+    for (int q = 0; q < kMin; ++q) res[17 + q] = q & 1 ? -S(kSums + kMax + q) : S(kSums + kMax + q);
+    res[21] = S(kPoint + 1);
+    res[22] = S(8);  // the energy sum stats.C reduces in its "adjoint" slot
+    for (int p = 0; p < a.n_planes; ++p) res[kResPlane0 + p] = S(kPlane0 + p);
 }
 
 template <class R>
-int stats_t(da_ctx *ctx, const StatArgs &a, double vslump, double d_time, double *dev) {
+int stats_t(da_ctx *ctx, const StatArgs &a, double vslump) {
     const MeshArgs m = mesh_args(ctx);
     const int c = ctx->cur;
     StateRef<R> U{(const R *)ctx->U[c][0], (const R *)ctx->U[c][1], (const R *)ctx->U[c][2]};
-    double *parts = dev, *res = dev + (size_t)kParts * kPartLen, *dis = res + 32;
-    k_stats_parts<R><<<kParts, kBlock, 0, ctx->stream>>>(m, U, a, parts);
-    k_stats_final<<<1, 32, 0, ctx->stream>>>(parts, a.n_planes, vslump, d_time, res, dis);
+    double *parts = ctx->stats_mem, *res = parts + (size_t)kParts * kPartLen;
+    k_stats<R><<<kParts, kBlock, 0, ctx->stream>>>(m, U, a, vslump, parts, (unsigned *)(res + kResLen), res);
     return cuda_check(ctx, cudaGetLastError(), "stats launch");
+}
+
+// The partial sums, the result and the block counter, kept with the context; the result's pinned copy.
+int stats_alloc(da_ctx *ctx) {
+    if (ctx->stats_mem) return DA_OK;
+    const size_t words = (size_t)kParts * kPartLen + kResLen + 1;
+    int st = DA_OK;
+    if (!ctx->stats_host)
+        st = cuda_check(ctx, cudaMallocHost((void **)&ctx->stats_host, sizeof(double) * kResLen), "cudaMallocHost(stats)");
+    double *dev = nullptr;
+    if (!st) st = cuda_check(ctx, cudaMalloc((void **)&dev, sizeof(double) * words), "cudaMalloc(stats)");
+    if (!st) st = cuda_check(ctx, cudaMemsetAsync(dev, 0, sizeof(double) * words, ctx->stream), "memset");
+    if (!st)
+        ctx->stats_mem = dev;
+    else if (dev)
+        cudaFree(dev);
+    return st;
 }
 
 // OutLine::update (properties.h:726-790) for every cell: the maximum depth so far over the grid
@@ -382,24 +455,13 @@ int da_compute_stats(da_ctx *ctx, const da_stats_props *props, double d_time, da
         pl[9] = 0.0;
         if (!(pl[6] > 0)) return set_error(ctx, DA_ERR_INVALID, "da_compute_stats: degenerate discharge plane");
     }
-    const size_t words = (size_t)kParts * kPartLen + 32 + DA_MAX_PLANES;
-    double *dev = nullptr;
-    int st = cuda_check(ctx, cudaMalloc((void **)&dev, sizeof(double) * words), "cudaMalloc(stats)");
-    double *dis = dev + (size_t)kParts * kPartLen + 32;
-    // the state the statistics read may still be in flight on the context's stream
-    if (!st) st = cuda_check(ctx, cudaStreamSynchronize(ctx->stream), "sync");
-    if (!st && props->n_planes > 0)
-        st = copy_h2d(ctx, dis, discharge, sizeof(double) * props->n_planes, "copy");
-    if (!st) st = ctx->p.precision == DA_PREC_FP64 ? stats_t<double>(ctx, a, props->vslump, d_time, dev)
-                                                   : stats_t<float>(ctx, a, props->vslump, d_time, dev);
-    double res[32];
-    // the context's stream does not synchronise with the legacy stream of cudaMemcpy
-    if (!st) st = cuda_check(ctx, cudaStreamSynchronize(ctx->stream), "sync");
-    if (!st) st = copy_d2h(ctx, res, dev + (size_t)kParts * kPartLen, sizeof(res), "copy");
-    if (!st && props->n_planes > 0)
-        st = copy_d2h(ctx, discharge, dis, sizeof(double) * props->n_planes, "copy");
-    if (dev) cudaFree(dev);
+    int st = stats_alloc(ctx);
+    if (!st) st = ctx->p.precision == DA_PREC_FP64 ? stats_t<double>(ctx, a, props->vslump)
+                                                   : stats_t<float>(ctx, a, props->vslump);
+    const double *res = ctx->stats_host;
+    if (!st) st = copy_d2h(ctx, ctx->stats_host, ctx->stats_mem + (size_t)kParts * kPartLen, sizeof(double) * kResLen, "copy");
     if (st) return st;
+    for (int p = 0; p < props->n_planes; ++p) discharge[p] = std::fma(d_time, res[kResPlane0 + p], discharge[p]);
     out->xcen = res[0];
     out->ycen = res[1];
     out->xvar = res[2];
