@@ -431,7 +431,7 @@ std::vector<unsigned char> sweep_key(const da_ctx *ctx, const double *box, int n
     put(iptr, sizeof(iptr));
     const void *ptrs[] = {ctx->U[0][0], ctx->U[0][1], ctx->U[0][2], ctx->U[1][0], ctx->U[1][1], ctx->U[1][2],
                           ctx->lam[0][0], ctx->lam[0][1], ctx->lam[0][2], ctx->lam[1][0], ctx->lam[1][1],
-                          ctx->lam[1][2], ctx->kact, ctx->active, ctx->seg_clean, ctx->seg_wet, ctx->seg_vol,
+                          ctx->lam[1][2], ctx->kact, ctx->slopes, ctx->fsign, ctx->active, ctx->seg_clean, ctx->seg_wet, ctx->seg_vol,
                           ctx->seg_dirty, ctx->mask, ctx->tile_epoch, ctx->seg_act, ctx->lam_clean, ctx->adjA,
                           ctx->adjB, ctx->gbed, ctx->gint, ctx->dk_tab, ctx->red_out, ctx->red_part, ctx->inst_J,
                           ctx->seg_J, ctx->dh0, ctx->dsc};

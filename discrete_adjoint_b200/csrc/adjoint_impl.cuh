@@ -284,8 +284,7 @@ __device__ __forceinline__ InstTables inst_tables(const AdjArgs &aa, const InstA
 // parameter sensitivities, from its own recorded branches (mask) and lambda^{n+1}.  Reads U^n
 // at the cell and its neighbours; writes only the cell's own entries.
 // adj_src_wet: wet cell i with U^n = prev, g_z, branch byte mi, boundary flags bf, lambda^{n+1}
-// = lnext and source coefficients cs; v and vi give the neighbour values of the slopes (global
-// arrays with vi = i, or the tile staged in shared memory with vi the cell's slot).
+// = lnext and source coefficients cs.
 // The forward's slopes, velocities and friction signs of wet cell vi (update_cell's arithmetic).
 template <class R, class V>
 __device__ __forceinline__ SrcFwd<R> src_fwd(const V &v, int vi, uint8_t bf, const R prev[3], R gamma, R ft) {
@@ -307,12 +306,25 @@ __device__ __forceinline__ SrcFwd<R> src_fwd(const V &v, int vi, uint8_t bf, con
     return f;
 }
 
-// get_f() gives the forward's quantities of the cell (computed, or handed over by the update).
-template <class R, class V, class GetF>
-__device__ __forceinline__ void adj_src_wet(const V &v, int vi, const MeshArgs &m, const R prev[3], R gz,
+// d (depth slope) / d h at the neighbour across each side: the slope's derivative by dp or dm over
+// the centre distance.
+template <class R, class V>
+__device__ __forceinline__ void slope_quotients(const V &v, int vi, uint8_t bf, R gamma, R h, R q[4]) {
+    SlopeD<R> sd[2];
+    h_slope_deriv<R>(v, vi, bf, gamma, h, sd);
+    q[0] = sd[0].g_dp / sd[0].dxp;
+    q[2] = sd[0].g_dm / sd[0].dxm;
+    q[1] = sd[1].g_dp / sd[1].dxp;
+    q[3] = sd[1].g_dm / sd[1].dxm;
+}
+
+// get_f() gives the forward's quantities of the cell (computed, or handed over by the update), get_q(q)
+// its slope_quotients (called for a cell without a domain edge).
+template <class R, class GetF, class GetQ>
+__device__ __forceinline__ void adj_src_wet(const MeshArgs &m, const R prev[3], R gz,
                                             uint8_t mi, uint8_t bf, const R lnext[3], const CellSrc<R> &cs,
-                                            const MatConsts &mc, const AdjArgs &aa, const InstTables &it, R dt, R ft,
-                                            int i, const GetF &get_f) {
+                                            const MatConsts &mc, const AdjArgs &aa, const InstTables &it, R dt,
+                                            int i, const GetF &get_f, const GetQ &get_q) {
     double A[3] = {0, 0, 0}, B[4] = {0, 0, 0, 0};
     {
         // lambda_eff: the depth row dropped where the forward step clamped h at zero
@@ -343,13 +355,11 @@ __device__ __forceinline__ void adj_src_wet(const V &v, int vi, const MeshArgs &
             A[2] = double(nu_v * (-sg3 * tan_bed * py * R(2) * vel1 * ky));
             // the limited depth slopes of this cell (zero on boundary cells)
             if (!(bf & 0x0F)) {
-                SlopeD<R> sd[2];
-                h_slope_deriv<R>(v, vi, bf, R(mc.gamma), h, sd);
+                R q[4];
+                get_q(q);
                 const R cx = -nu_v * sg1 * h * k * gz * sin_int;  // on d h / dx
                 const R cy = -nu_u * sg0 * h * k * gz * sin_int;  // on d h / dy
-                // d slope / d h at the neighbours: g / (centre distance)
-                const R qp0 = sd[0].g_dp / sd[0].dxp, qm0 = sd[0].g_dm / sd[0].dxm;
-                const R qp1 = sd[1].g_dp / sd[1].dxp, qm1 = sd[1].g_dm / sd[1].dxm;
+                const R qp0 = q[0], qm0 = q[2], qp1 = q[1], qm1 = q[3];
                 A[0] += double(cx * (-qp0 + qm0) + cy * (-qp1 + qm1));
                 B[0] = double(cx * qp0);
                 B[2] = double(-cx * qm0);
@@ -385,8 +395,9 @@ __device__ __forceinline__ void adj_src_cell(const MeshArgs &m, const StateRef<R
     const R lnext[3] = {Lnext.h[i], Lnext.hu[i], Lnext.hv[i]};
     const GlobalView<R> v = global_view<R>(m, U, (const R *)nullptr);
     const uint8_t bf = m.bflag[i];
-    adj_src_wet<R>(v, i, m, prev, grav<R>(m, 2, i), aa.mask[i], bf, lnext, cell_src<R>(m, i), mc, aa, it, dt, ft, i,
-                   [&]() { return src_fwd<R>(v, i, bf, prev, R(mc.gamma), ft); });
+    adj_src_wet<R>(m, prev, grav<R>(m, 2, i), aa.mask[i], bf, lnext, cell_src<R>(m, i), mc, aa, it, dt, i,
+                   [&]() { return src_fwd<R>(v, i, bf, prev, R(mc.gamma), ft); },
+                   [&](R q[4]) { slope_quotients<R>(v, i, bf, R(mc.gamma), h_i, q); });
 }
 
 template <class R, bool BATCH = false>

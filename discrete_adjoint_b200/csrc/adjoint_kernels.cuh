@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(kBlock, OCC) k_youturn(MeshArgs m, fwd::StateP
     unsigned long long my_min = 0x7FF0000000000000ull, my_max = 0ull;
     if (STAGED)
         fwd::coef_phase_staged<R, true, BATCH>(m, ha, U, kact, active, seg_wet, ntiles, cull, mc, sc, mask, list, my_min,
-                                               my_max, ia, stg);
+                                               my_max, ia, stg, fwd::sign_threshold<R>(iter, tc, mc));
     else
         fwd::coef_phase<R, true, BATCH>(m, U, kact, active, seg_wet, ntiles, cull, mc, sc, mask, list, my_min, my_max,
                                         ia);
@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(kBlock, OCC) k_youturn(MeshArgs m, fwd::StateP
         // the source adjoint of each wet cell right after its update, from the tile and halo
         // staged for it (its own branches and lambda^{n+1}, U^n around it: nothing another cell
         // writes in this phase), so the reverse step needs no source phase of its own
-        const SrcEpilogue<R, BATCH> src{m, Ln, mc, aa, ia, R(dt), ftr};
+        const SrcEpilogue<R, BATCH> src{m, Ln, mc, aa, ia, R(dt), (const R *)ha.kept};
         fwd::update_phase_staged<R, true, BATCH>(m, ha, U, O, kact, active, seg_clean, seg_wet, seg_vol, seg_dirty,
                                                  ntiles, cull, mc, sc, R(dt), ftr, mask, tile_epoch, seg_act, rec_id,
                                                  list, ia, stg, src);

@@ -101,6 +101,30 @@ void fill_consts(const da_params &p, MatConsts *mc, TimeConsts *tc) {
     tc->frict_tiny_iters = p.frict_tiny_iters;
 }
 
+bool kact_ordinary(const MatConsts &mc) {
+    auto ok = [](double k) { return k == 0.0 || (k >= 0x1p-60 && k <= 0x1p60); };
+    bool all = ok(mc.kact_rest);
+    for (int m = 0; m < mc.n_materials; ++m)
+        for (double k : mc.kact_sgn[m]) all = all && ok(k);
+    return all;
+}
+
+// The mesh's share of what quot.cuh asks for: the distances between a cell's centre and its
+// neighbours' (cells with four neighbours), the sizes and g_z all within [2^-40, 2^40].
+static bool mesh_ordinary(const da_mesh_soa *m) {
+    auto ok = [](double v) { return v >= 0x1p-40 && v <= 0x1p40; };
+    const int n = m->n_cells;
+    for (int i = 0; i < n; ++i) {
+        if (!ok(m->dx[i]) || !ok(m->dy[i]) || !ok(m->gravity[(size_t)2 * n + i])) return false;
+        const int e[4] = {m->nbr[i], m->nbr[(size_t)n + i], m->nbr[(size_t)2 * n + i], m->nbr[(size_t)3 * n + i]};
+        if (e[0] < 0 || e[1] < 0 || e[2] < 0 || e[3] < 0) continue;
+        if (!ok(m->x[e[0]] - m->x[i]) || !ok(m->x[i] - m->x[e[2]]) || !ok(m->y[e[1]] - m->y[i]) ||
+            !ok(m->y[i] - m->y[e[3]]))
+            return false;
+    }
+    return true;
+}
+
 static bool params_ok(const da_params *p) {
     if (!p) return false;
     if (p->precision != DA_PREC_FP64 && p->precision != DA_PREC_FP32_SPLIT) return false;
@@ -137,6 +161,7 @@ static void free_state(da_ctx *ctx) {
         for (int v = 0; v < 3; ++v) dfree(ctx->U[b][v]);
     dfree(ctx->kact);
     dfree(ctx->slopes);
+    dfree(ctx->fsign);
     dfree(ctx->seg_vol);
     dfree(ctx->vol_parts);
     dfree(ctx->active);
@@ -442,6 +467,8 @@ void da_destroy(da_ctx *ctx) {
     trace_flush(ctx);
     for (cudaEvent_t e : ctx->trace.pool) cudaEventDestroy(e);
     if (ctx->dt_replay) cudaFree(ctx->dt_replay);
+    if (ctx->stats_mem) cudaFree(ctx->stats_mem);
+    if (ctx->stats_host) cudaFreeHost(ctx->stats_host);
     if (ctx->dsc) cudaFree(ctx->dsc);
     if (ctx->hsc) cudaFreeHost(ctx->hsc);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
@@ -467,8 +494,6 @@ int da_selftest_barrier(da_ctx *ctx, int32_t limit_us) {
     const int st3 = cuda_check(ctx, cudaStreamSynchronize(ctx->stream), "sync");
     return st2 ? st2 : (st3 ? st3 : code);
 }
-    if (ctx->stats_mem) cudaFree(ctx->stats_mem);
-    if (ctx->stats_host) cudaFreeHost(ctx->stats_host);
 
 int da_set_params(da_ctx *ctx, const da_params *p) {
     if (!ctx) return DA_ERR_INVALID;
@@ -539,6 +564,7 @@ int da_upload_mesh(da_ctx *ctx, const da_mesh_soa *m, int32_t epoch) {
     d.n_owned = n;
     d.epoch = epoch;
     const bool fp64 = ctx->p.precision == DA_PREC_FP64;
+    d.ordinary = fp64 && mesh_ordinary(m);
     if (!st) st = upload(ctx, &d.nbr, m->nbr, (size_t)8 * n);
     if (!st) st = upload(ctx, &d.bflag, bflag.data(), npad);
     if (!st) st = upload(ctx, &d.mat, mat.data(), npad);

@@ -131,6 +131,8 @@ struct DevMesh {
     int32_t *halo_idx = nullptr;    // halo cells of every tile, tile after tile
     int16_t *nloc = nullptr;        // [n][8] tile-local slot of each neighbour entry
     int32_t halo_max = 0;           // largest halo of a tile
+    // FP64: centre distances, sizes and g_z all within [2^-40, 2^40] (quot.cuh)
+    bool ordinary = false;
 };
 
 // Tracing: CUDA events around every launch of the step and the adjoint, summed per kernel
@@ -167,7 +169,11 @@ struct da_ctx {
     void *U[2][3] = {{nullptr, nullptr, nullptr}, {nullptr, nullptr, nullptr}};
     int cur = 0;
     void *kact = nullptr;            // [n] Real
-    void *slopes = nullptr;          // [6][n] Real: wet cells' limited slopes from the coefficient phase
+    // what the staged coefficient phase keeps of each wet cell for the update phase (staged_impl.cuh):
+    // FP64 [9][n] (depth slopes, velocities, wave speed, the depth slopes' derivatives) and the friction
+    // signs, FP32 [4][n] (slopes)
+    void *slopes = nullptr;
+    uint8_t *fsign = nullptr;        // [n] FP64 only
     // segments: 32 consecutive cells (one warp), 8 per tile; arrays padded to whole tiles
     int nseg = 0;                    // ntiles * 8
     double *seg_vol = nullptr;       // [nseg] volume partial of each segment after its last update
@@ -182,6 +188,7 @@ struct da_ctx {
     // ensemble mode (ninst > 0): device tables of InstArgs, host copies of the member layout
     int ninst = 0;
     da::InstArgs ia{};
+    bool inst_ordinary = false;       // every member's k act/pass table within quot.cuh's range
     std::vector<int32_t> inst_cell0;  // [ninst + 1] first cell of each member (multiple of 256)
     std::vector<int32_t> inst_ncell;  // [ninst] cells of each member before padding
     std::vector<int32_t> inst_nmat;   // [ninst] materials of each member
@@ -191,6 +198,8 @@ struct da_ctx {
     std::vector<double> inst_init;    // [3][n] members' initial states, concatenated (restart)
     da::DwrState dwr;                 // error grid of the DWR indicator (da_dwr_setup)
     da::OutlineGrid outline;          // maximum-depth map (da_outline_init)
+    double *stats_mem = nullptr;      // partial sums and result of the flow statistics (stats.cu)
+    double *stats_host = nullptr;     // pinned copy of the result
     int *tile_epoch = nullptr;       // [ntiles] id of the last recording step that listed the tile
     uint8_t *seg_act = nullptr;      // [nseg] the segment had an active cell in that step
     uint8_t *lam_clean = nullptr;    // [nseg] both adjoint buffers hold the same segment
@@ -198,8 +207,6 @@ struct da_ctx {
     int ntiles = 0;                  // tiles of 256 consecutive cells
     int nblocks = 0;                 // grid of the seed kernel (fixed at allocation)
     int grid = 0;                    // grid of the tiled step kernels (da_params.grid_blocks)
-    double *stats_mem = nullptr;      // partial sums and result of the flow statistics (stats.cu)
-    double *stats_host = nullptr;     // pinned copy of the result
     // resident blocks of k_steps [FP32, FP64] x [single, ensemble] x [2, 3 per SM] x [staged] x
     // [checkpoint stores inside the launch]
     int coop_cap[32] = {};
@@ -264,6 +271,8 @@ int cuda_check(da_ctx *ctx, cudaError_t e, const char *what);
 int copy_h2d(da_ctx *ctx, void *dev, const void *host, size_t bytes, const char *what);
 int copy_d2h(da_ctx *ctx, void *host, const void *dev, size_t bytes, const char *what);
 void fill_consts(const da_params &p, MatConsts *mc, TimeConsts *tc);
+// every k act/pass value of the table zero or within [2^-60, 2^60] (quot.cuh)
+bool kact_ordinary(const MatConsts &mc);
 
 // forward_fp64.cu / forward_fp32.cu
 // record_mask (optional): branch codes of the step for the adjoint (listed tiles; tile_epoch)

@@ -172,6 +172,7 @@ int da_ensemble_upload(da_ctx *ctx, const da_member *members, int32_t n_members)
     double *sec2 = (double *)(host.data() + o_sec2), *cosi = (double *)(host.data() + o_cos);
     double *dk = (double *)(host.data() + o_dk), *box = (double *)(host.data() + o_box);
     int32_t *seg0 = (int32_t *)(host.data() + o_seg0);
+    bool ordinary = true;
     for (int k = 0; k < nm; ++k) {
         da_params pk = ctx->p;
         pk.n_materials = members[k].n_materials;
@@ -179,6 +180,7 @@ int da_ensemble_upload(da_ctx *ctx, const da_member *members, int32_t n_members)
         pk.intfrict = members[k].intfrict;
         TimeConsts tc;
         fill_consts(pk, &mcs[k], &tc);
+        ordinary = ordinary && kact_ordinary(mcs[k]);
         for (int m = 0; m < DA_MAX_MATERIALS; ++m) {
             const double t = m < pk.n_materials ? std::tan(pk.bedfrict[m]) : 0.0;
             sec2[k * DA_MAX_MATERIALS + m] = 1.0 + t * t;
@@ -208,6 +210,7 @@ int da_ensemble_upload(da_ctx *ctx, const da_member *members, int32_t n_members)
     ia.box = (const double *)(b + o_box);
     ia.seg0 = (const int32_t *)(b + o_seg0);
     ctx->ninst = nm;
+    ctx->inst_ordinary = ordinary;
     ctx->inst_cell0 = cell0;
     for (int k = 0; k < nm; ++k) {
         ctx->inst_ncell.push_back(members[k].mesh.n_cells);

@@ -62,6 +62,13 @@ __device__ __forceinline__ void step_dt(double min_dxe, double hmax, double time
     ft_out = iter < tc.frict_tiny_iters ? tc.frict_tiny_early : tc.frict_tiny_late;
 }
 
+// The friction sign threshold of the step after iter steps (step_dt's ft, not below the FP32 floor).
+template <class R>
+__device__ __forceinline__ R sign_threshold(long long iter, const TimeConsts &tc, const MatConsts &mc) {
+    const double ft = iter < tc.frict_tiny_iters ? tc.frict_tiny_early : tc.frict_tiny_late;
+    return R(ft) > R(mc.sign_floor) ? R(ft) : R(mc.sign_floor);
+}
+
 constexpr unsigned long long kMinDxeStart = 0x416312D000000000ull;  // bits of 1e7, get_coef_and_eigen.C:36
 
 __device__ void finalize_dt(DevScalars *sc, const TimeConsts &tc) {
@@ -607,7 +614,7 @@ __global__ void __launch_bounds__(kBlock, OCC) k_steps(MeshArgs m, StatePair<R> 
         unsigned long long my_min = 0x7FF0000000000000ull, my_max = 0ull;
         if (STAGED)
             coef_phase_staged<R, false, BATCH>(m, ha, U, kact, active, seg_wet, ntiles, cull, mc, sc, nullptr, list,
-                                               my_min, my_max, ia, stg);
+                                               my_min, my_max, ia, stg, sign_threshold<R>(iter, tc, mc));
         else
             coef_phase<R, false, BATCH>(m, U, kact, active, seg_wet, ntiles, cull, mc, sc, nullptr, list, my_min,
                                         my_max, ia);

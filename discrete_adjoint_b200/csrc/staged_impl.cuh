@@ -10,11 +10,27 @@
 // identical; only where the operands come from changes.  Each cell's neighbour entries come from
 // the host-built table of tile-local slots (one 16-byte load per cell).
 //
+// FP64: what both phases need of a wet cell and of its wet neighbours is formed once per cell, in the
+// coefficient phase: the velocities hu / h and hv / h and the flux's wave speed sqrt(k h g_z) go to
+// global memory, are staged with the tile, and replace k act/pass and g_z there, so the four side
+// fluxes of a cell take no division and no square root besides the HLL quotients; the four friction
+// signs (a byte) and the two depth slopes are all that the sources take from the slopes.  Quotients
+// that share a divisor are formed branch-free (quot.cuh) as long as every staged state is ordinary
+// there (tested as the copies land, folded into the tile's barrier); a tile with any other value, and
+// a mesh or material outside the range, takes the division operator.  The results are the
+// reference's bits either way.  Bound: not memory (740k wet cells: a third of HBM's rate) but the
+// instructions and the latency of one warp's FP64 chain.  46 divisions and 6 square roots per cell and
+// step became 13 divisors and 2 square roots: 2894 -> 2050 instructions per warp and step, 125 -> 95 us
+// per step on 740k wet cells (2 x 296 blocks), 14.0 -> 10.7 us on a flow of 18 tiles.  Three blocks
+// per SM with one buffer each (80 registers) took 100 us.
+//
 // Activity: a cell is updated when it or a face neighbour is wet.  The global path marks every
 // neighbour of a wet cell in the active bitmask with atomics; here the update phase recomputes
 // that set from the staged depths of the tile and its halo, and the coefficient phase only marks
 // neighbours in other tiles (and each warp's own wet cells), which the tile listing needs.
 #pragma once
+
+#include "quot.cuh"
 
 namespace da {
 namespace fwd {
@@ -31,10 +47,12 @@ struct StageBuf {
     R src[6][kTileCells];                      // update phase: g_x, g_y, the gravity derivatives, curvatures
     // every slot
     R h[kSlots], hu[kSlots], hv[kSlots];
-    R k[kSlots];   // k act/pass (update phase)
-    R gz[kSlots];  // g_z
-    R c0[kSlots];  // FP64: x centre; FP32: dx
-    R c1[kSlots];  // FP64: y centre; FP32: dy
+    R c0[kSlots];  // FP64: x centre (coefficient phase), hu / h of wet cells (update phase); FP32: dx
+    R c1[kSlots];  // FP64: y centre, hv / h; FP32: dy
+    R a[sizeof(R) == 8 ? kSlots : 1];  // FP64: wave speed of wet cells (update phase)
+    // FP64: the tile's own cells only
+    R k[sizeof(R) == 8 ? kTileCells : kSlots];   // k act/pass (update phase)
+    R gz[sizeof(R) == 8 ? kTileCells : kSlots];  // g_z
 };
 
 template <class R>
@@ -54,12 +72,18 @@ struct HaloArgs {
     const int32_t *off;   // [ntiles + 1]
     const int32_t *idx;   // halo cells, tile after tile
     const int16_t *nloc;  // [n][8] tile-local neighbour slots
-    void *slopes;         // [6][n] reals: the limited slopes of each wet cell (h > GEOFLOW_TINY), written
-                          // by the coefficient phase and read by the same step's update phase
+    // written by the coefficient phase for each wet cell and read by the same step's update phase:
+    void *kept;           // FP64 [5][n]: d h / dx, d h / dy, hu / h, hv / h, sqrt(k h g_z), and when recording
+                          // [4][n] more, the derivatives of d h / dx and d h / dy by the neighbours' depths;
+                          // FP32 [4][n]: the limited slopes d h / dx, d hv / dx, d h / dy, d hu / dy
+    uint8_t *fsign;       // FP64 [n]: the four friction signs of the sources, two bits each (sign + 1)
+    int fast;             // FP64: the mesh and the materials allow quot.cuh's quotients
 };
 
 inline HaloArgs halo_args(const da_ctx *ctx) {
-    return HaloArgs{ctx->mesh.halo_off, ctx->mesh.halo_idx, ctx->mesh.nloc, ctx->slopes};
+    const bool kact = ctx->ninst > 0 ? ctx->inst_ordinary : kact_ordinary(ctx->mc);
+    return HaloArgs{ctx->mesh.halo_off, ctx->mesh.halo_idx, ctx->mesh.nloc,
+                    ctx->slopes,        ctx->fsign,         ctx->mesh.ordinary && kact ? 1 : 0};
 }
 
 // The staged phases run when the parameters ask for them, the mesh's halo tables exist and the
@@ -102,25 +126,30 @@ __device__ __forceinline__ void load_slots(const int16_t *nloc, int i, int nl[8]
     }
 }
 
-// Copies of one slot's values.  UPD: also k act/pass and g_z (the update phase reads them at
-// neighbours; the coefficient phase reads g_z at the cell itself only).  XY (FP64): the centres,
-// which only the limited slopes read (the coefficient phase, and the reverse step's source
-// adjoint inside its update phase).
-template <class R, bool UPD, bool XY = true>
+// Copies of one slot's values.  UPD: also what the update phase reads at neighbours (FP64: the
+// velocities and the wave speed, at the cell itself k act/pass and g_z; FP32: k act/pass and g_z).
+// The coefficient phase reads the centres instead (FP64).
+template <class R, bool UPD>
 __device__ __forceinline__ void stage_slot(StageBuf<R> &b, int s, int e, bool own, const MeshArgs &m,
-                                           const StateRef<R> &U, const R *kact) {
+                                           const StateRef<R> &U, const R *kact, const HaloArgs &ha) {
     constexpr int B = sizeof(R);
     cp_async<B>(&b.h[s], U.h + e);
     cp_async<B>(&b.hu[s], U.hu + e);
     cp_async<B>(&b.hv[s], U.hv + e);
-    if (UPD) cp_async<B>(&b.k[s], kact + e);
     if constexpr (sizeof(R) == 8) {
-        if (UPD || own) cp_async<B>(&b.gz[s], m.g + (size_t)2 * m.n + e);
-        if (XY) {
+        if (own) cp_async<B>(&b.gz[s], m.g + (size_t)2 * m.n + e);
+        if (UPD) {
+            const R *kept = (const R *)ha.kept;
+            if (own) cp_async<B>(&b.k[s], kact + e);
+            cp_async<B>(&b.c0[s], kept + (size_t)2 * m.n + e);
+            cp_async<B>(&b.c1[s], kept + (size_t)3 * m.n + e);
+            cp_async<B>(&b.a[s], kept + (size_t)4 * m.n + e);
+        } else {
             cp_async<B>(&b.c0[s], m.x + e);
             cp_async<B>(&b.c1[s], m.y + e);
         }
     } else {
+        if (UPD) cp_async<B>(&b.k[s], kact + e);
         if (UPD || own) cp_async<B>(&b.gz[s], m.fg + (size_t)2 * m.n + e);
         cp_async<B>(&b.c0[s], m.fdx + e);
         cp_async<B>(&b.c1[s], m.fdy + e);
@@ -185,14 +214,24 @@ __device__ __forceinline__ void staged_slots(const StageBuf<R> &b, int c, int nl
 }
 
 // Tile t's own cells and its halo (halo list already in shared memory) into buffer b.
-template <class R, bool UPD, bool XY = true>
+template <class R, bool UPD>
 __device__ __forceinline__ void stage_tile(StageBuf<R> &b, int t, const int *hidx, int hcnt, const MeshArgs &m,
-                                           const StateRef<R> &U, const R *kact, const int16_t *nloc) {
+                                           const StateRef<R> &U, const R *kact, const HaloArgs &ha) {
     const int i = t * kTileCells + (int)threadIdx.x;
-    if (i < m.n) stage_slot<R, UPD, XY>(b, threadIdx.x, i, true, m, U, kact);
-    stage_own<R, UPD>(b, t, m, nloc);
+    if (i < m.n) stage_slot<R, UPD>(b, threadIdx.x, i, true, m, U, kact, ha);
+    stage_own<R, UPD>(b, t, m, ha.nloc);
     for (int k = threadIdx.x; k < hcnt; k += kTileCells)
-        stage_slot<R, UPD, XY>(b, kTileCells + k, hidx[k], false, m, U, kact);
+        stage_slot<R, UPD>(b, kTileCells + k, hidx[k], false, m, U, kact, ha);
+}
+
+// Whether a state this thread staged (its own cell of tile t, its halo cells) is outside the range
+// of quot.cuh; after the thread's copies have landed.
+__device__ __forceinline__ bool staged_odd(const StageBuf<double> &b, int t, int hcnt, int n) {
+    auto odd = [&](int s) { return !(quot::ordinary(b.h[s]) && quot::ordinary(b.hu[s]) && quot::ordinary(b.hv[s])); };
+    const int c = (int)threadIdx.x;
+    bool r = t * kTileCells + c < n && odd(c);
+    for (int k = c; k < hcnt; k += kTileCells) r = r || odd(kTileCells + k);
+    return r;
 }
 
 __device__ __forceinline__ void stage_halo_list(int *dst, const int32_t *src, int cnt) {
@@ -210,23 +249,24 @@ __device__ __forceinline__ void halo_range(const HaloArgs &ha, int tq, int ntile
     }
 }
 
-// The listed tiles of a round, pipelined: fn(t, buffer, halo list) computes tile t from shared
-// memory.  Needs blockDim.x == kTileCells; every thread of the block calls it with the same cnt;
-// S.hoff / S.hcnt hold the listed tiles' halo ranges (compact_tiles).  The first tile's halo
-// cells are read by the threads that copy them; later tiles' lists arrive two tiles ahead.
-template <class R, bool UPD, bool XY = true, class F>
+// The listed tiles of a round, pipelined: fn(t, buffer, halo list, fast) computes tile t from shared
+// memory (fast: FP64 quotients by quot.cuh).  Needs blockDim.x == kTileCells; every thread of the
+// block calls it with the same cnt; S.hoff / S.hcnt hold the listed tiles' halo ranges
+// (compact_tiles).  The first tile's halo cells are read by the threads that copy them; later
+// tiles' lists arrive two tiles ahead.
+template <class R, bool UPD, class F>
 __device__ __forceinline__ void staged_tiles(const MeshArgs &m, const HaloArgs &ha, const StateRef<R> &U,
                                              const R *kact, int cnt, const int *list, StageSmem<R> &S, F &&fn) {
     {
         const int t0 = list[0], hc = S.hcnt[0];
         const int32_t *src = ha.idx + S.hoff[0];
         const int i = t0 * kTileCells + (int)threadIdx.x;
-        if (i < m.n) stage_slot<R, UPD, XY>(S.buf[0], threadIdx.x, i, true, m, U, kact);
+        if (i < m.n) stage_slot<R, UPD>(S.buf[0], threadIdx.x, i, true, m, U, kact, ha);
         stage_own<R, UPD>(S.buf[0], t0, m, ha.nloc);
         for (int k = threadIdx.x; k < hc; k += kTileCells) {
             const int e = src[k];
             S.hidx[0][k] = e;
-            stage_slot<R, UPD, XY>(S.buf[0], kTileCells + k, e, false, m, U, kact);
+            stage_slot<R, UPD>(S.buf[0], kTileCells + k, e, false, m, U, kact, ha);
         }
     }
     if (cnt > 1) stage_halo_list(S.hidx[1], ha.idx + S.hoff[1], S.hcnt[1]);
@@ -234,16 +274,257 @@ __device__ __forceinline__ void staged_tiles(const MeshArgs &m, const HaloArgs &
     for (int q = 0; q < cnt; ++q) {
         // tile q's values and tile q + 1's halo list have landed; every thread is past tile q - 1
         cp_async_wait_all();
-        __syncthreads();
+        bool fast = false;
+        if constexpr (sizeof(R) == 8)
+            fast = !__syncthreads_or(!ha.fast || staged_odd(S.buf[q & 1], list[q], S.hcnt[q], m.n));
+        else
+            __syncthreads();
         if (q + 1 < cnt) {
-            stage_tile<R, UPD, XY>(S.buf[(q + 1) & 1], list[q + 1], S.hidx[(q + 1) % 3], S.hcnt[q + 1], m, U,
-                                   kact, ha.nloc);
+            stage_tile<R, UPD>(S.buf[(q + 1) & 1], list[q + 1], S.hidx[(q + 1) % 3], S.hcnt[q + 1], m, U, kact, ha);
             if (q + 2 < cnt) stage_halo_list(S.hidx[(q + 2) % 3], ha.idx + S.hoff[q + 2], S.hcnt[q + 2]);
         }
         cp_async_commit();
-        fn(list[q], S.buf[q & 1], S.hidx[q % 3]);
+        fn(list[q], S.buf[q & 1], S.hidx[q % 3], fast);
     }
     __syncthreads();
+}
+
+// ------------------------------------------------------------------------------- FP64 arithmetic
+// The cold path's division, out of line (the kernels stay small).
+__device__ __noinline__ double div_operator(double a, double b) { return a / b; }
+
+// A divisor and its quotients: FAST by quot.cuh, else the operator.
+template <bool FAST>
+struct Divisor {
+    quot::Recip r;
+    __device__ __forceinline__ explicit Divisor(double b) {
+        if constexpr (FAST)
+            r = quot::recip(b);
+        else
+            r.b = b;
+    }
+    __device__ __forceinline__ double operator()(double a) const {
+        if constexpr (FAST)
+            return quot::div(a, r);
+        else
+            return div_operator(a, r.b);
+    }
+};
+
+// cell_slopes (fv_device.cuh, FP64) with one divisor per centre distance.  DERIV: also the derivatives
+// of the depth slopes by the depth across each side, q[s] (h_slope_deriv, adjoint_impl.cuh: the
+// slope's derivative by dp or dm over the centre distance).
+template <bool FAST, bool DERIV>
+__device__ __forceinline__ void staged_slopes64(const StagedView<double> &v, int i, uint8_t bf, double gamma,
+                                                const double ui[3], double out[6], double q[4]) {
+    if (bf & 0x0F) {
+#pragma unroll
+        for (int j = 0; j < 6; ++j) out[j] = 0.0;
+        if (DERIV) q[0] = q[1] = q[2] = q[3] = 0.0;
+        return;
+    }
+#pragma unroll
+    for (int dir = 0; dir < 2; ++dir) {
+        const int ep = v.nb(dir, i), em = v.nb(dir + 2, i);
+        const bool two_p = bf & (0x10 << dir), two_m = bf & (0x10 << (dir + 2));
+        const double ci = v.coord(dir, i);
+        const double dxp = v.coord(dir, ep) - ci, dxm = ci - v.coord(dir, em);
+        const Divisor<FAST> dvp(dxp), dvm(dxm), dvs(dxm + dxp);
+        const double up[3] = {v.h(ep), v.hu(ep), v.hv(ep)}, um[3] = {v.h(em), v.hu(em), v.hv(em)};
+        double dp[3], dm[3];
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            dp[j] = dvp(up[j] - ui[j]);
+            dm[j] = dvm(ui[j] - um[j]);
+        }
+        if (two_p) {
+            const int e = v.nb(dir + 4, i);
+            const double u2[3] = {v.h(e), v.hu(e), v.hv(e)};
+#pragma unroll
+            for (int j = 0; j < 3; ++j) dp[j] = .5 * (dp[j] + dvp(u2[j] - ui[j]));
+        }
+        if (two_m) {
+            const int e = v.nb(dir + 6, i);
+            const double u2[3] = {v.h(e), v.hu(e), v.hv(e)};
+#pragma unroll
+            for (int j = 0; j < 3; ++j) dm[j] = .5 * (dm[j] + dvm(ui[j] - u2[j]));
+        }
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            const double dc = dvs(dp[j] * dxm + dm[j] * dxp);
+            double mn = gamma * dabs(dp[j]);
+            const double b = gamma * dabs(dm[j]), c = dabs(dc);
+            int sel = 0;
+            if (mn > b) { mn = b; sel = 1; }
+            if (mn > c) { mn = c; sel = 2; }
+            const double fac = .5 * (c_sgn(dp[j]) + c_sgn(dm[j]));
+            out[j + 3 * dir] = fac * mn;
+            if (DERIV && j == 0) {
+                const auto sgnf = [](double x) { return x > 0.0 ? 1.0 : (x < 0.0 ? -1.0 : 0.0); };
+                const double gc = dvs(fac * sgnf(dc));
+                const double gp = sel == 0 ? fac * gamma * sgnf(dp[0]) : (sel == 1 ? 0.0 : gc * dxm);
+                const double gm = sel == 1 ? fac * gamma * sgnf(dm[0]) : (sel == 0 ? 0.0 : gc * dxp);
+                q[dir] = dvp(gp);
+                q[dir + 2] = dvm(gm);
+            }
+        }
+    }
+}
+
+// What the coefficient phase forms of a wet cell (FP64).
+struct Coef64 {
+    double s[6];        // limited slopes
+    double vx, vy, a;   // hu / h, hv / h, sqrt(k h g_z)
+    double k, ev;       // k act/pass, largest wave speed
+    uint8_t code;       // branch of k act/pass
+    uint8_t sgn;        // friction signs, two bits each
+    double q[4];        // recording: derivatives of the depth slopes by the neighbours' depths
+};
+
+// A cell with h > GEOFLOW_TINY: get_slopes, gmfggetcoef, eigen, and the velocities, wave speed and
+// friction signs that the corrector forms from the same values (update_cell).
+template <bool FAST, bool DERIV>
+__device__ __forceinline__ void staged_coef64(const StagedView<double> &v, int c, uint8_t bf, int mat, double gz,
+                                              const MatConsts &mc, double ft, const double ui[3], Coef64 &o) {
+    staged_slopes64<FAST, DERIV>(v, c, bf, mc.gamma, ui, o.s, o.q);
+    const double *s = o.s;
+    const double h = ui[0], hu = ui[1], hv = ui[2];
+    const Divisor<FAST> dh(h), dhh(h * h);
+    o.vx = dh(hu);
+    o.vy = dh(hv);
+    const double vel = dh(s[1]) - dhh(hu * s[0]) + dh(s[5]) - dhh(hv * s[3]);
+    const int sg = fsgn(vel, DA_TINY);
+    o.k = mc.kact_sgn[mat][sg + 1];
+    o.code = uint8_t(sg + 2);
+    if (dabs(o.vx) < DA_TINY && dabs(o.vy) < DA_TINY) {
+        o.k = mc.kact_rest;
+        o.code = 0;
+    }
+    const double cc = sqrt(o.k * gz * h);
+    o.a = sqrt(o.k * h * gz);
+    const double evx = dabs(o.vx) + cc, evy = dabs(o.vy) + cc;
+    o.ev = evx > evy ? evx : evy;
+    const double h_inv = dh(1.0);
+    const int s0 = int(tiny_sgn(h_inv * (s[4] - o.vx * s[3]), ft)), s2 = int(tiny_sgn(o.vx, ft));
+    const int s1 = int(tiny_sgn(h_inv * (s[2] - o.vy * s[0]), ft)), s3 = int(tiny_sgn(o.vy, ft));
+    o.sgn = uint8_t((s0 + 1) | (s1 + 1) << 2 | (s2 + 1) << 4 | (s3 + 1) << 6);
+}
+
+// A side of a Riemann problem from the staged values (dirflux): zero for a dry cell.
+struct Side64 {
+    double u[3], f[3], s0, s1, s2;
+};
+
+template <int DIR>
+__device__ __forceinline__ Side64 staged_side64(const StageBuf<double> &b, int e) {
+    Side64 o;
+    const double h = b.h[e];
+    const bool wet = !(h < DA_TINY);
+    o.u[0] = wet ? h : 0.0;
+    o.u[1] = wet ? b.hu[e] : 0.0;
+    o.u[2] = wet ? b.hv[e] : 0.0;
+    const double vel = wet ? (DIR == 0 ? b.c0[e] : b.c1[e]) : 0.0, a = wet ? b.a[e] : 0.0;
+    const double p = 0.5 * a * a * o.u[0];
+    if (DIR == 0) {
+        o.f[0] = o.u[1];
+        o.f[1] = o.u[1] * vel + p;
+        o.f[2] = o.u[2] * vel;
+    } else {
+        o.f[0] = o.u[2];
+        o.f[1] = o.u[1] * vel;
+        o.f[2] = o.u[2] * vel + p;
+    }
+    o.s0 = vel - a;
+    o.s1 = vel;
+    o.s2 = vel + a;
+    return o;
+}
+
+// riemann (fv_device.cuh) with one divisor for the three components.  Two dry sides give zero speeds,
+// hence the left flux, which is zero.
+template <bool FAST>
+__device__ __forceinline__ void riemann64(const Side64 &l, const Side64 &r, double F[3]) {
+    const bool ld = l.u[0] == 0.0, rd = r.u[0] == 0.0;
+    const double a0 = 2.0 * r.s0 - r.s1, a2 = 2.0 * r.s2 - r.s1;
+    const double b0 = 2.0 * l.s0 - l.s1, b2 = 2.0 * l.s2 - l.s1;
+    const double lo = ld ? a0 : (rd ? b0 : rmin(l.s0, r.s0));
+    const double hi = ld ? a2 : (rd ? b2 : rmax(l.s2, r.s2));
+    const double sl = rmin(0.0, lo), sr = rmax(0.0, hi);
+    if (sl >= 0.0) {
+        F[0] = l.f[0]; F[1] = l.f[1]; F[2] = l.f[2];
+    } else if (sr <= 0.0) {
+        F[0] = r.f[0]; F[1] = r.f[1]; F[2] = r.f[2];
+    } else {
+        const Divisor<FAST> den(sr - sl);
+#pragma unroll
+        for (int v = 0; v < 3; ++v) F[v] = den(sr * l.f[v] - sl * r.f[v] + sl * sr * (r.u[v] - l.u[v]));
+    }
+}
+
+// F(+side) - F(-side) in direction DIR of cell c (flux_div).
+template <bool FAST, int DIR>
+__device__ __forceinline__ void staged_div64(const StagedView<double> &v, int c, uint8_t bf, double div[3]) {
+    if (bf & ((1 << DIR) | (1 << (DIR + 2)))) {
+        div[0] = div[1] = div[2] = 0.0;
+        return;
+    }
+    const Side64 self = staged_side64<DIR>(v.b, c);
+    double Fm[3], Fp[3];
+    riemann64<FAST>(staged_side64<DIR>(v.b, v.nl[DIR + 2]), self, Fm);
+    riemann64<FAST>(self, staged_side64<DIR>(v.b, v.nl[DIR]), Fp);
+    if (bf & (0x10 << (DIR + 2))) {
+        double F2[3];
+        riemann64<FAST>(staged_side64<DIR>(v.b, v.nl[DIR + 6]), self, F2);
+#pragma unroll
+        for (int q = 0; q < 3; ++q) Fm[q] = 0.5 * (Fm[q] + F2[q]);
+    }
+    if (bf & (0x10 << DIR)) {
+        double F2[3];
+        riemann64<FAST>(self, staged_side64<DIR>(v.b, v.nl[DIR + 4]), F2);
+#pragma unroll
+        for (int q = 0; q < 3; ++q) Fp[q] = 0.5 * (Fp[q] + F2[q]);
+    }
+#pragma unroll
+    for (int q = 0; q < 3; ++q) div[q] = Fp[q] - Fm[q];
+}
+
+// What the update phase loads of a cell ahead of the fluxes.
+struct Kept64 {
+    double sx, sy;  // depth slopes
+    uint8_t sgn;
+};
+
+// update_cell (forward_impl.cuh) of an active cell from the staged and kept values.
+template <bool FAST, class Hook>
+__device__ __forceinline__ bool staged_update64(const StagedView<double> &v, int c, uint8_t bf, const CellSrc<double> &cs,
+                                                const MatConsts &mc, double dt, const double prev[3], double dxc,
+                                                double dyc, double st[3], const Kept64 &kp, const Hook &hook) {
+    double dx3[3], dy3[3];
+    staged_div64<FAST, 0>(v, c, bf, dx3);
+    staged_div64<FAST, 1>(v, c, bf, dy3);
+    const double dtdx = dt / dxc;
+    const double dtdy = dyc == dxc ? dtdx : dt / dyc;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) st[q] = prev[q] - dtdx * dx3[q] - dtdy * dy3[q];
+    const bool clamped = st[0] < 0.0;
+    if (clamped) st[0] = 0.0;
+    if (prev[0] > DA_TINY) {
+        const double vel0 = v.b.c0[c], vel1 = v.b.c1[c];
+        auto sg = [&](int q) { return double(int((kp.sgn >> (2 * q)) & 3) - 1); };
+        const double sg0 = sg(0), sg1 = sg(1), sg2 = sg(2), sg3 = sg(3);
+        hook(SrcFwd<double>{{kp.sx, 0.0, 0.0, kp.sy, 0.0, 0.0}, vel0, vel1, 0.0, sg0, sg1, sg2, sg3}, clamped);
+        const double ki = v.b.k[c], gz = v.b.gz[c];
+        const double sin_int = mc.sin_int, tan_bed = mc.tan_bed[cs.mat];
+        double s1 = cs.g[0] * prev[0];
+        double s2 = sg0 * prev[0] * ki * (gz * kp.sy + cs.dg[1] * prev[0]) * sin_int;
+        double s3 = sg2 * rmax(gz * prev[0] + vel0 * prev[1] * cs.cv[0], 0.0) * tan_bed;
+        st[1] += dt * (s1 - s2 - s3);
+        s1 = cs.g[1] * prev[0];
+        s2 = sg1 * prev[0] * ki * (gz * kp.sx + cs.dg[0] * prev[0]) * sin_int;
+        s3 = sg3 * rmax(gz * prev[0] + vel1 * prev[2] * cs.cv[1], 0.0) * tan_bed;
+        st[2] += dt * (s1 - s2 - s3);
+    }
+    return clamped;
 }
 
 // Coefficient phase (see coef_phase) with the tile and its halo staged.
@@ -252,7 +533,7 @@ __device__ __forceinline__ void coef_phase_staged(const MeshArgs &m, const HaloA
                                                   R *kact, unsigned *active, const uint8_t *seg_wet, int ntiles,
                                                   int cull, const MatConsts &mc0, DevScalars *sc, uint8_t *mask,
                                                   int *list, unsigned long long &my_min, unsigned long long &my_max,
-                                                  const InstArgs &ia, StageSmem<R> &S) {
+                                                  const InstArgs &ia, StageSmem<R> &S, R ft) {
     for (int round = 0; sched_more(round, ntiles); ++round) {
         const int tq = sched_tile(round);
         const bool need = tq < ntiles && (!cull || seg_flags(seg_wet, tq) != 0ull);
@@ -260,7 +541,7 @@ __device__ __forceinline__ void coef_phase_staged(const MeshArgs &m, const HaloA
         halo_range(ha, tq, ntiles, ho, hc);
         const int cnt = compact_tiles(need, tq, list, ho, hc, S.hoff, S.hcnt);
         if (cnt == 0) continue;
-        staged_tiles<R, false>(m, ha, U, kact, cnt, list, S, [&](int t, const StageBuf<R> &b, const int *hidx) {
+        staged_tiles<R, false>(m, ha, U, kact, cnt, list, S, [&](int t, const StageBuf<R> &b, const int *hidx, bool fast) {
             const int inst = BATCH ? ia.tile_inst[t] : 0;
             const MatConsts &mc = BATCH ? ia.mcs[inst] : mc0;
             const int c = threadIdx.x;
@@ -297,24 +578,52 @@ __device__ __forceinline__ void coef_phase_staged(const MeshArgs &m, const HaloA
                             }
                         }
                     }
+                    const R ui[3] = {h, b.hu[c], b.hv[c]};
+                    const R gz = b.gz[c];
                     if (!(h > R(DA_TINY))) {  // h == GEOFLOW_TINY: dry for get_coef_and_eigen, wet for the fluxes
                         kact[i] = R(mc.kact_rest);
-                    } else {
-                        const R ui[3] = {h, b.hu[c], b.hv[c]};
-                        R s[6];
-                        cell_slopes<R>(v, c, bf, R(mc.gamma), ui, s);
-                        if (ha.slopes) {  // kept for the update phase's source terms
-                            R *sl = (R *)ha.slopes;
-#pragma unroll
-                            for (int j = 0; j < 6; ++j) sl[(size_t)j * m.n + i] = s[j];
+                        if constexpr (sizeof(R) == 8) {
+                            R *kept = (R *)ha.kept;
+                            kept[(size_t)2 * m.n + i] = ui[1] / h;
+                            kept[(size_t)3 * m.n + i] = ui[2] / h;
+                            kept[(size_t)4 * m.n + i] = sqrt(mc.kact_rest * h * gz);
                         }
-                        const R k = cell_kact<R>(mc, mat, h, ui[1], ui[2], s, &code);
-                        kact[i] = k;
-                        const R gz = b.gz[c];
-                        const R vx = ui[1] / h, vy = ui[2] / h;
-                        const R cc = sqrt(k * gz * h);
-                        const R evx = dabs(vx) + cc, evy = dabs(vy) + cc;
-                        const R ev = evx > evy ? evx : evy;
+                    } else {
+                        R ev;
+                        R *kept = (R *)ha.kept;
+                        if constexpr (sizeof(R) == 8) {
+                            Coef64 o;
+                            if (fast)
+                                staged_coef64<true, RECORD>(v, c, bf, mat, gz, mc, ft, ui, o);
+                            else
+                                staged_coef64<false, RECORD>(v, c, bf, mat, gz, mc, ft, ui, o);
+                            code = o.code;
+                            kact[i] = o.k;
+                            kept[i] = o.s[0];
+                            kept[(size_t)m.n + i] = o.s[3];
+                            kept[(size_t)2 * m.n + i] = o.vx;
+                            kept[(size_t)3 * m.n + i] = o.vy;
+                            kept[(size_t)4 * m.n + i] = o.a;
+                            ha.fsign[i] = o.sgn;
+                            if (RECORD)
+#pragma unroll
+                                for (int q = 0; q < 4; ++q) kept[(size_t)(5 + q) * m.n + i] = o.q[q];
+                            ev = o.ev;
+                        } else {
+                            R s[6];
+                            cell_slopes<R>(v, c, bf, R(mc.gamma), ui, s);
+                            // kept for the update phase's source terms
+                            kept[i] = s[0];
+                            kept[(size_t)m.n + i] = s[2];
+                            kept[(size_t)2 * m.n + i] = s[3];
+                            kept[(size_t)3 * m.n + i] = s[4];
+                            const R k = cell_kact<R>(mc, mat, h, ui[1], ui[2], s, &code);
+                            kact[i] = k;
+                            const R vx = ui[1] / h, vy = ui[2] / h;
+                            const R cc = sqrt(k * gz * h);
+                            const R evx = dabs(vx) + cc, evy = dabs(vy) + cc;
+                            ev = evx > evy ? evx : evy;
+                        }
                         if (ev > R(1000000000.)) raise_err(sc, DA_ERR_EIGEN);
                         const unsigned long long rb = __double_as_longlong(double((dxm > dym ? dym : dxm) / ev));
                         const unsigned long long hb = __double_as_longlong(double(h));
@@ -374,10 +683,7 @@ __device__ __forceinline__ void update_phase_staged(const MeshArgs &m, const Hal
         const int cnt = compact_tiles(need, tq, list, ho, hc, S.hoff, S.hcnt);
         if (cnt == 0) continue;
         if (RECORD && threadIdx.x == 0) atomicAdd(&sc->listed, (unsigned)cnt);
-        // the centres only for an epilogue (the source adjoint's slope derivatives read them); the
-        // update itself takes the kept slopes
-        constexpr bool XY = !std::is_same<Epi, NoEpilogue>::value;
-        staged_tiles<R, true, XY>(m, ha, U, kact, cnt, list, S, [&](int t, const StageBuf<R> &b, const int *) {
+        staged_tiles<R, true>(m, ha, U, kact, cnt, list, S, [&](int t, const StageBuf<R> &b, const int *, bool fast) {
             const int inst = BATCH ? ia.tile_inst[t] : 0;
             const MatConsts &mc = BATCH ? ia.mcs[inst] : mc0;
             const R dt = BATCH ? R(ia.dt[inst]) : dt0;
@@ -389,15 +695,24 @@ __device__ __forceinline__ void update_phase_staged(const MeshArgs &m, const Hal
             bool wet_after = false, act = false;
             if (i < m.n) {
                 const R prev[3] = {b.h[c], b.hu[c], b.hv[c]};
-                // the slopes this step's coefficient phase left for a wet cell, loaded ahead of the fluxes
-                const bool own_s = ha.slopes != nullptr && prev[0] > R(DA_TINY);
-                R pre_s[6];
-                if (own_s) {
-                    const R *sl = (const R *)ha.slopes;
-#pragma unroll
-                    for (int j = 0; j < 6; ++j) pre_s[j] = sl[(size_t)j * m.n + i];
+                // what this step's coefficient phase left for a wet cell, loaded ahead of the fluxes
+                const bool wet = prev[0] > R(DA_TINY);
+                const R *kept = (const R *)ha.kept;
+                Kept64 kp{};
+                R pre_s[6] = {};
+                if (wet) {
+                    if constexpr (sizeof(R) == 8) {
+                        kp.sx = kept[i];
+                        kp.sy = kept[(size_t)m.n + i];
+                        kp.sgn = ha.fsign[i];
+                    } else {
+                        pre_s[0] = kept[i];
+                        pre_s[2] = kept[(size_t)m.n + i];
+                        pre_s[3] = kept[(size_t)2 * m.n + i];
+                        pre_s[4] = kept[(size_t)3 * m.n + i];
+                    }
                 }
-                const auto pre = epi.pre(i, prev[0] > R(DA_TINY));
+                const auto pre = epi.pre(i, wet);
                 const uint8_t bf = b.bf[c];
                 StagedView<R> v{b};
                 staged_slots(b, c, v.nl);
@@ -421,13 +736,21 @@ __device__ __forceinline__ void update_phase_staged(const MeshArgs &m, const Hal
                 const CellSrc<R> cs = staged_src(b, c);
                 // the k act/pass code the coefficient phase recorded
                 const uint8_t kcode = RECORD && prev[0] >= R(DA_TINY) ? uint8_t(mask[i] & 3) : uint8_t(0);
-                if (act)
-                    clamped = update_cell<R>(v, c, bf, cs, mc, dt, ft, prev, dxc, dyc, st, own_s ? pre_s : nullptr,
-                                             [&](const SrcFwd<R> &f, bool cl) {
-                                                 // a wet cell is active: its branch byte as recorded below
-                                                 epi(t, i, v, c, prev, bf, uint8_t(kcode | 8 | (cl ? 4 : 0)), b.gz[c],
-                                                     cs, pre, f);
-                                             });
+                // a wet cell is active: its branch byte as recorded below
+                const auto hook = [&](const SrcFwd<R> &f, bool cl) {
+                    epi(t, i, v, c, prev, bf, uint8_t(kcode | 8 | (cl ? 4 : 0)), b.gz[c], cs, pre, f);
+                };
+                if (act) {
+                    if constexpr (sizeof(R) == 8) {
+                        if (fast)
+                            clamped = staged_update64<true>(v, c, bf, cs, mc, dt, prev, dxc, dyc, st, kp, hook);
+                        else
+                            clamped = staged_update64<false>(v, c, bf, cs, mc, dt, prev, dxc, dyc, st, kp, hook);
+                    } else {
+                        clamped = update_cell<R>(v, c, bf, cs, mc, dt, ft, prev, dxc, dyc, st, wet ? pre_s : nullptr,
+                                                 hook);
+                    }
+                }
                 const uint8_t code = RECORD ? uint8_t(kcode | (act ? 8 : 0) | (clamped ? 4 : 0)) : 0;
                 if (RECORD) mask[i] = code;
                 if (!isfinite(st[0]) || !isfinite(st[1]) || !isfinite(st[2])) raise_err(sc, DA_ERR_NAN);
