@@ -281,6 +281,12 @@ static int sync_scalars(da_ctx *ctx) {
     return device_error(ctx, "forward step");
 }
 
+// The same after a launch_volume that wrote them into hsc.
+static int sync_volume(da_ctx *ctx) {
+    const int st = cuda_check(ctx, cudaStreamSynchronize(ctx->stream), "stream sync");
+    return st ? st : device_error(ctx, "forward step");
+}
+
 void update_grid(da_ctx *ctx) {
     const int per_sm4 = (ctx->sm_count > 0 ? ctx->sm_count : 148) * 4;
     int g = ctx->p.grid_blocks > 0 ? ctx->p.grid_blocks : per_sm4;
@@ -637,9 +643,9 @@ int da_forward_step(da_ctx *ctx, da_step_stats *out) {
     if (ctx->mesh.n <= 0) return set_error(ctx, DA_ERR_NO_MESH, "da_forward_step: no mesh");
     if (!ctx->have_state) return set_error(ctx, DA_ERR_INVALID, "da_forward_step: no state");
     cudaSetDevice(ctx->device);
-    int st = launch_forward_step(ctx);
-    if (!st) st = launch_volume(ctx);
-    if (!st) st = sync_scalars(ctx);
+    int st = launch_single_step(ctx);
+    if (!st) st = launch_volume(ctx, ctx->hsc);
+    if (!st) st = sync_volume(ctx);
     fill_stats(ctx, out);
     return st;
 }
@@ -671,8 +677,8 @@ int da_forward_run_timed(da_ctx *ctx, int32_t nsteps, da_step_stats *last, doubl
     }
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
-    if (!st) st = launch_volume(ctx);
-    if (!st) st = sync_scalars(ctx);
+    if (!st) st = launch_volume(ctx, ctx->hsc);
+    if (!st) st = sync_volume(ctx);
     fill_stats(ctx, last);
     return st;
 }

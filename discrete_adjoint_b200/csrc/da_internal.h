@@ -45,7 +45,7 @@ struct DevScalars {
     unsigned long long acc_min_dxe;  // running min, bit pattern of a positive double
     unsigned long long acc_hmax;     // running max, bit pattern of a non-negative double
     int err;              // sticky DA_ERR_* raised on the device
-    unsigned blocks_done[2];  // last-block counters of the coefficient and update kernels
+    unsigned blocks_done[2];  // last-block counters of the coefficient and volume kernels
     unsigned listed;      // tiles the reverse step's recording update listed (sets the gather's work split)
     unsigned long long acc_alt_min_dxe;  // the multi-step kernel's second accumulator pair
     unsigned long long acc_alt_hmax;     // (odd steps of a launch), same start values
@@ -279,8 +279,11 @@ bool kact_ordinary(const MatConsts &mc);
 int launch_forward_step(da_ctx *ctx, uint8_t *record_mask = nullptr);
 int launch_forward_step_fp64(da_ctx *ctx, uint8_t *record_mask);
 int launch_forward_step_fp32(da_ctx *ctx, uint8_t *record_mask);
-// the volume (sum dx dy h) of the current state into the device scalars
-int launch_volume(da_ctx *ctx);
+// one step without records, by whichever of the two below is the faster
+int launch_single_step(da_ctx *ctx);
+// the volume (sum dx dy h) of the current state into the device scalars, and all of them into host
+// (pinned memory, valid once the stream is waited for) unless it is null
+int launch_volume(da_ctx *ctx, DevScalars *host = nullptr);
 // nsteps whole steps in one cooperative launch (k_steps); same results as nsteps single steps
 // nsteps steps in one cooperative launch; pre_slot / post_slot (checkpoint slots, or null): a
 // restore before the first step and a store after the last one inside the same launch.

@@ -432,10 +432,13 @@ __global__ void __launch_bounds__(kBlock) k_update(MeshArgs m, StateRef<R> U, St
 
 // ---------------------------------------------------------------------------- volume
 // sum of dx dy h over the mesh (step.C:205) from the segments' partials, in a fixed order: block
-// b of kVolParts sums a fixed contiguous range of segments, then one block adds the parts.
-// Launched only when the volume is asked for.
-__global__ void __launch_bounds__(kBlock) k_volume_parts(const double *__restrict__ seg_vol, int nseg,
-                                                         double *__restrict__ parts) {
+// b of kVolParts sums a fixed contiguous range of segments, then the last block to finish adds the
+// parts.  Launched only when the volume is asked for.  host (or null): pinned memory that receives all
+// the scalars, so that a caller who waits for the stream needs no copy after it (a step's two volume
+// launches and its copy cost about as much as one of its two kernels: 47 us a step before).
+__global__ void __launch_bounds__(kBlock) k_volume(const double *__restrict__ seg_vol, int nseg,
+                                                   double *__restrict__ parts, DevScalars *sc, DevScalars *host) {
+    static_assert(kVolParts == kBlock, "one thread per part");
     __shared__ double red[kBlock / 32];
     const int per = (nseg + kVolParts - 1) / kVolParts;
     const int s0 = blockIdx.x * per, s1 = min(nseg, s0 + per);
@@ -443,17 +446,12 @@ __global__ void __launch_bounds__(kBlock) k_volume_parts(const double *__restric
     for (int s = s0 + threadIdx.x; s < s1; s += kBlock) acc += seg_vol[s];
     acc = block_sum(acc, red);
     if (threadIdx.x == 0) parts[blockIdx.x] = acc;
-}
-
-__global__ void __launch_bounds__(kVolParts) k_volume_final(const double *__restrict__ parts, DevScalars *sc) {
-    __shared__ double red[kVolParts / 32];
-    const double v = warp_sum(parts[threadIdx.x]);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-    __syncthreads();
+    if (!last_block(&sc->blocks_done[1])) return;
+    const double v = block_sum(__ldcg(parts + threadIdx.x), red);
     if (threadIdx.x == 0) {
-        double t = 0.0;
-        for (int w = 0; w < kVolParts / 32; ++w) t += red[w];
-        sc->volume = t;
+        sc->volume = v;
+        sc->blocks_done[1] = 0u;
+        if (host) *host = *sc;
     }
 }
 
@@ -841,10 +839,9 @@ int launch_steps_t(da_ctx *ctx, int nsteps, void *pre_slot, void *post_slot, con
     return DA_OK;
 }
 
-// The volume of the current state into the scalars (two launches, fixed order).
-inline int launch_volume_t(da_ctx *ctx) {
-    k_volume_parts<<<kVolParts, kBlock, 0, ctx->stream>>>(ctx->seg_vol, ctx->nseg, ctx->vol_parts);
-    k_volume_final<<<1, kVolParts, 0, ctx->stream>>>(ctx->vol_parts, ctx->dsc);
+// The volume of the current state into the scalars, and those into host (pinned, or null).
+inline int launch_volume_t(da_ctx *ctx, DevScalars *host) {
+    k_volume<<<kVolParts, kBlock, 0, ctx->stream>>>(ctx->seg_vol, ctx->nseg, ctx->vol_parts, ctx->dsc, host);
     return cuda_check(ctx, cudaGetLastError(), "volume launch");
 }
 

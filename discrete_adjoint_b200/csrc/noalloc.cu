@@ -174,8 +174,7 @@ extern "C" int da_forward_step_noalloc(const da_params *p, const da_mesh_soa *me
     fwd::k_coef<double><<<grid, fwd::kBlock, 0, s>>>(m, U, kact, active, seg_wet, ntiles, 0, mc, tc, sc);
     fwd::k_update<double><<<grid, fwd::kBlock, 0, s>>>(m, U, O, kact, active, seg_clean, seg_wet, seg_vol, seg_dirty,
                                                        ntiles, 0, mc, sc);
-    fwd::k_volume_parts<<<fwd::kVolParts, fwd::kBlock, 0, s>>>(seg_vol, ntiles * (fwd::kBlock / 32), vol_parts);
-    fwd::k_volume_final<<<1, fwd::kVolParts, 0, s>>>(vol_parts, sc);
+    fwd::k_volume<<<fwd::kVolParts, fwd::kBlock, 0, s>>>(seg_vol, ntiles * (fwd::kBlock / 32), vol_parts, sc, nullptr);
     if (cudaGetLastError() != cudaSuccess) return DA_ERR_CUDA;
     if (cudaMemcpyAsync(&hs, sc, sizeof(DevScalars), cudaMemcpyDeviceToHost, s) != cudaSuccess) return DA_ERR_CUDA;
     if (cudaStreamSynchronize(s) != cudaSuccess) return DA_ERR_CUDA;
