@@ -174,40 +174,20 @@ struct Schedule {
     }
 };
 
-// DWR indicator along the reverse sweep (da_adjoint_run_dwr): after the reverse step of n -> n+1
-// (U^n, U^{n+1} and lambda^{n+1} all resident) the indicator of that step, as the reference's
-// dual_solver calls error_compute after each adjoint step (dual_solver.C:206-230).
-struct DwrAcc {
-    double *cell = nullptr;       // [n] device: el_error per coarse cell, summed over the steps
-    double *step_sums = nullptr;  // host [nsteps][2]: total el_error and correction of each step
-    long long iter_begin = 0;     // iteration of U^0
-    int nsteps = 0;
-};
-
-__global__ void k_accumulate(int n, const double *__restrict__ a, double *__restrict__ acc) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) acc[i] += a[i];
-}
-
-int dwr_after_reverse_step(da_ctx *ctx, DwrAcc &d, int lam_next) {
-    // the reverse step wrote the step's dt, time and iteration like a forward step
-    int st = copy_d2h(ctx, ctx->hsc, ctx->dsc, sizeof(DevScalars), "read scalars");
-    if (st) return st;
-    const double dt = ctx->hsc->dt;
-    const long long iter0 = ctx->hsc->iter - 1;
-    const double time0 = ctx->hsc->time - dt;  // enters the error grid's step only through clipping
-    st = dwr_indicator(ctx, ctx->cur ^ 1, ctx->cur, lam_next, dt, time0, iter0);
-    if (st) return st;
-    const int n = ctx->mesh.n, grid = (ctx->sm_count > 0 ? ctx->sm_count : 148) * 4;
-    k_accumulate<<<grid, 256, 0, ctx->stream>>>(n, ctx->dwr.cell, d.cell);
-    st = cuda_check(ctx, cudaGetLastError(), "dwr accumulate");
-    const long long k = iter0 - d.iter_begin;
-    if (!st && k >= 0 && k < d.nsteps) st = copy_d2h(ctx, d.step_sums + 2 * k, ctx->dwr.sums, 16, "dwr sums");
-    return st;
-}
-
 struct Runner {
     da_ctx *ctx;
-    DwrAcc *dwr = nullptr;
+    // DWR indicator along the reverse sweep (da_adjoint_run_dwr): after the reverse step of n -> n+1
+    // (U^n, U^{n+1} and lambda^{n+1} all resident) the indicator of that step, as the reference's
+    // dual_solver calls error_compute after each adjoint step (dual_solver.C:206-230).
+    bool dwr = false;
+    long long iter_begin = 0;  // iteration of U^0
+    int left = 0;              // reverse steps still to come
+    int dwr_step() {
+        --left;
+        if (!dwr) return DA_OK;
+        return dwr_indicator(ctx, ctx->cur ^ 1, ctx->cur, lam_cur, iter_begin + left, ctx->dwr.acc,
+                             ctx->dwr.step_sums + 2 * (size_t)left);
+    }
     Schedule sch;
     std::vector<int> free_slots;
     int lam_cur = 0;  // buffer holding lambda^{n+1}
@@ -272,7 +252,7 @@ struct Runner {
         if (ctx->p.jacobian_mode == DA_JAC_REFERENCE) return youturn_reference();
         // the first reverse step (the horizon's last step) also seeds lambda^N from U^N
         int st = launch_youturn(ctx, lam_cur, 1 - lam_cur, sec2, cos_int, !seeded, box, take_pending());
-        if (!st && dwr) st = dwr_after_reverse_step(ctx, *dwr, lam_cur);
+        if (!st) st = dwr_step();
         seeded = true;
         lam_cur = 1 - lam_cur;
         return st;
@@ -286,7 +266,7 @@ struct Runner {
         if (!st) st = launch_forward_step(ctx, nullptr);
         if (!st && !seeded) st = launch_ref_seed(ctx, lam_cur, box);
         if (!st) st = launch_ref_adjoint_step(ctx, ctx->cur ^ 1, lam_cur, 1 - lam_cur);
-        if (!st && dwr) st = dwr_after_reverse_step(ctx, *dwr, lam_cur);
+        if (!st) st = dwr_step();
         seeded = true;
         lam_cur = 1 - lam_cur;
         return st;
@@ -444,17 +424,18 @@ std::vector<unsigned char> sweep_key(const da_ctx *ctx, const double *box, int n
 // over nsteps steps from the current state, reverse steps back to step 0, the state put back,
 // J and the gradient sums launched (single: red_out[n_mat + 1 + n_piles]; ensemble: per member).
 // lam0 receives the buffer that holds lambda^0.
-// Without the DWR indicator (which reads every reverse step on the host) and without tracing, the
-// sweep's thousand or so launches are captured once as a CUDA graph and replayed while nothing
+// Without tracing, the sweep's thousand or so launches (the DWR indicator's among them) are captured once as a CUDA graph and replayed while nothing
 // they depend on changes: a graph starts its cooperative kernels back to back, without the few
 // microseconds of idle GPU between stream launches.  The recording ids the capture gave the
 // reverse steps repeat on a replay, so the graph first clears the tiles' recording ids.
 int adjoint_sweep(da_ctx *ctx, const double *box, int32_t nsteps, int32_t nsnapshots, int32_t n_piles, int *lam0,
-                  long long *fsteps, float *dev_ms, void *dwr_acc, const double *lambda_end) {
+                  long long *fsteps, float *dev_ms, const long long *dwr_iter0, const double *lambda_end) {
     int st = adj_alloc(ctx, nsnapshots + 1);
     Runner r;
     r.ctx = ctx;
-    r.dwr = (DwrAcc *)dwr_acc;
+    r.dwr = dwr_iter0 != nullptr;
+    r.iter_begin = r.dwr ? *dwr_iter0 : 0;
+    r.left = nsteps;
     if (box)
         for (int q = 0; q < 4; ++q) r.box[q] = box[q];
     if (!st) st = upload_tables(ctx, r.sec2, &r.cos_int);
@@ -483,17 +464,23 @@ int adjoint_sweep(da_ctx *ctx, const double *box, int32_t nsteps, int32_t nsnaps
         if (!s) s = r.reverse(0, nsteps, 0);
         if (!s) s = r.flush();
         if (!s) s = restore(ctx, 0);
+        if (!s && r.dwr)
+            s = cuda_check(ctx, cudaMemsetAsync(ctx->dwr.acc, 0, sizeof(double) * (size_t)ctx->mesh.n, ctx->stream), "memset");
         if (!s) s = launch_functional(ctx, ctx->inst_J);
         if (!s) s = ctx->ninst > 0 ? launch_adjoint_reduce_inst(ctx, r.lam_cur) : launch_adjoint_reduce(ctx, r.lam_cur, n_piles);
         return s;
     };
-    bool graph = !r.dwr && !ctx->trace.on && ctx->p.jacobian_mode == DA_JAC_EXACT;
+    bool graph = !ctx->trace.on && ctx->p.jacobian_mode == DA_JAC_EXACT;
     if (graph) {
         std::vector<unsigned char> key = sweep_key(ctx, box, nsteps, nsnapshots, n_piles, r.seeded, r.sec2, r.cos_int);
         if (!ctx->sweep_graph || key != ctx->sweep_key) {
             if (ctx->sweep_graph) cudaGraphExecDestroy(ctx->sweep_graph);
             ctx->sweep_graph = nullptr;
             ctx->sweep_key.clear();
+        // the error grid's own tables are fixed until it is released, which drops the graph
+        const long long dwr_key[4] = {r.dwr, r.iter_begin, (long long)(uintptr_t)(r.dwr ? ctx->dwr.acc : nullptr),
+                                      (long long)(uintptr_t)(r.dwr ? ctx->dwr.step_sums : nullptr)};
+        key.insert(key.end(), (const unsigned char *)dwr_key, (const unsigned char *)(dwr_key + 4));
             // capture: nothing runs; the host-side state the launches leave is kept for replays
             const Runner r0 = r;
             const int cur0 = ctx->cur;
@@ -613,7 +600,7 @@ int da_adjoint_step(da_ctx *ctx, const double *lambda_next, double *lambda_out, 
 namespace {
 
 int adjoint_run_impl(da_ctx *ctx, const da_functional *f, int32_t nsteps, int32_t nsnapshots, const double *dh0_dpile,
-                     int32_t n_piles, da_gradient *out, double *lambda0, DwrAcc *dwr,
+                     int32_t n_piles, da_gradient *out, double *lambda0, const long long *dwr,
                      const double *lambda_end = nullptr) {
     if (!ctx || (!f && !lambda_end) || nsteps <= 0 || nsnapshots < 0 || n_piles < 0 || n_piles > DA_MAX_PILES ||
         (n_piles > 0 && !dh0_dpile) || (f && f->kind != DA_FUNC_H2_BOX))
@@ -675,18 +662,14 @@ int da_adjoint_run_dwr(da_ctx *ctx, const da_functional *f, int32_t nsteps, int3
     if (ctx->mesh.n <= 0 || nsteps <= 0) return da_adjoint_run(ctx, f, nsteps, nsnapshots, dh0_dpile, n_piles, out, lambda0);
     cudaSetDevice(ctx->device);
     const size_t n = (size_t)ctx->mesh.n;
-    DwrAcc acc;
-    acc.step_sums = step_sums;
-    acc.nsteps = nsteps;
     for (int k = 0; k < 2 * nsteps; ++k) step_sums[k] = 0.0;
     int st = cuda_check(ctx, cudaStreamSynchronize(ctx->stream), "sync");
     if (!st) st = copy_d2h(ctx, ctx->hsc, ctx->dsc, sizeof(DevScalars), "read scalars");
-    acc.iter_begin = ctx->hsc->iter;
-    if (!st) st = cuda_check(ctx, cudaMalloc((void **)&acc.cell, sizeof(double) * n), "cudaMalloc(dwr cells)");
-    if (!st) st = cuda_check(ctx, cudaMemsetAsync(acc.cell, 0, sizeof(double) * n, ctx->stream), "memset");
-    if (!st) st = adjoint_run_impl(ctx, f, nsteps, nsnapshots, dh0_dpile, n_piles, out, lambda0, &acc);
-    if (!st) st = copy_d2h(ctx, cell_error, acc.cell, sizeof(double) * n, "copy dwr cells");
-    if (acc.cell) cudaFree(acc.cell);
+    const long long iter_begin = ctx->hsc->iter;
+    if (!st) st = dwr_accumulators(ctx, nsteps);
+    if (!st) st = adjoint_run_impl(ctx, f, nsteps, nsnapshots, dh0_dpile, n_piles, out, lambda0, &iter_begin);
+    if (!st) st = copy_d2h(ctx, cell_error, ctx->dwr.acc, sizeof(double) * n, "copy dwr cells");
+    if (!st) st = copy_d2h(ctx, step_sums, ctx->dwr.step_sums, sizeof(double) * 2 * (size_t)nsteps, "copy dwr sums");
     return st;
 }
 

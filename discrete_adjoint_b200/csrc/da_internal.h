@@ -95,21 +95,24 @@ struct OutlineGrid {
 
 // Dual-weighted-residual indicator: the error grid's own context and the device tables (dwr.cu).
 struct DwrState {
-    da_ctx *fine = nullptr;      // context of the error grid (the mesh refined once)
+    da_ctx *fine = nullptr;      // context of the error grid (the mesh refined once), on the coarse stream
+    cudaStream_t fine_stream = nullptr;  // its own stream, unused meanwhile
     int nf = 0;
     void *mem = nullptr;         // one allocation for the tables below
-    int32_t *parent = nullptr;   // [nf]
     int32_t *children = nullptr; // [4][n] fine cells of each coarse cell, -1 unused
     int32_t *interp = nullptr;   // [4][nf] coarse interpolants, -1 unused
     double *weight = nullptr;    // [4][nf]
     double *ut_next = nullptr;   // [3][nf] reconstructed U^{n+1}
     double *lamt = nullptr;      // [3][nf] reconstructed adjoint
     double *err = nullptr;       // [nf] el_error
-    double *corr = nullptr;      // [nf] correction
     double *cell = nullptr;      // [n] el_error summed over each coarse cell's children
     double *parts = nullptr;     // compensated partial sums
     double *sums = nullptr;      // [2] total el_error, total correction
 };
+    unsigned *done = nullptr;    // last-block counter of the sums
+    double *acc = nullptr;       // [n] el_error per coarse cell over a sweep
+    double *step_sums = nullptr; // [step_cap][2] totals of each step of a sweep
+    int step_cap = 0;
 
 // Device copy of the flattened mesh.  FP64 path reads the double arrays; the FP32-split
 // path reads the float copies.
@@ -319,14 +322,19 @@ int forward_state_changed(da_ctx *ctx);
 // adjoint_host.cu: d kact / d phi_bed and d phi_int of each material's three branches
 void kact_derivatives(const da_params &p, double *dkb, double *dki);
 // adjoint_host.cu: the checkpointed reverse sweep (see there)
-// dwr_acc (or null): accumulate the DWR indicator of every reverse step (adjoint_host.cu DwrAcc)
+// dwr_iter0 (or null): also the DWR indicator of every reverse step, into the context's accumulators,
+// iteration *dwr_iter0 at the beginning
 // lambda_end (or null): lambda^N given instead of the functional's seed (host [3][n])
 int adjoint_sweep(da_ctx *ctx, const double *box, int32_t nsteps, int32_t nsnapshots, int32_t n_piles, int *lam0,
-                  long long *fsteps, float *dev_ms, void *dwr_acc = nullptr, const double *lambda_end = nullptr);
+                  long long *fsteps, float *dev_ms, const long long *dwr_iter0 = nullptr,
+                  const double *lambda_end = nullptr);
 int copy_lambda_out(da_ctx *ctx, int buf, double *host);
-// dwr.cu: the indicator of the step U[un] -> U[unext] with adjoint lam[lam] (coarse dt, time and
-// iteration before the step); release of the error grid
-int dwr_indicator(da_ctx *ctx, int un, int unext, int lam, double dt, double time0, long long iter0);
+// dwr.cu: the indicator of the step U[un] -> U[unext] with adjoint lam[lam], queued on the stream after
+// the kernel that made the step (iter0 the iteration before it; its dt and time are read from the
+// device scalars): the totals into out[2] (device), the estimate per coarse cell added to acc (or null);
+// the accumulators of a sweep; release of the error grid
+int dwr_indicator(da_ctx *ctx, int un, int unext, int lam, long long iter0, double *acc, double *out);
+int dwr_accumulators(da_ctx *ctx, int nsteps);
 void dwr_release(da_ctx *ctx);
 // adjoint_host.cu: adjoint buffers and one checkpoint slot
 int adj_alloc_for_dwr(da_ctx *ctx);

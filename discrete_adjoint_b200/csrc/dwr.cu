@@ -6,11 +6,16 @@
 //   1. the coarse step U^n -> U^{n+1} (its dt), the state put back afterwards;
 //   2. k_dwr_interp: on every fine cell the reconstructed U~^n (written as the error grid's state),
 //      U~^{n+1} and lambda~ from the coarse fields through the fixed (cell, weight) pairs;
-//   3. one step of the error grid from U~^n with the coarse dt (frozen-dt replay, same iteration);
+//   3. one step of the error grid from U~^n with the coarse dt (frozen-dt replay of the device's own
+//      value, same iteration);
 //   4. k_dwr_residual: r = step(U~^n) - U~^{n+1}; per fine cell |r . (lambda - lambda~)| summed
-//      over the three fields (el_error) and r . lambda (correction), lambda the parent's adjoint;
-//   5. per coarse cell the sum over its four children (fixed order), and the totals as
-//      compensated (Neumaier) FP64 sums in a fixed order.
+//      over the three fields (el_error) and r . lambda (correction), lambda the parent's adjoint; per
+//      coarse cell the sum over its four children (fixed order), and the totals as compensated FP64
+//      sums in a fixed order.
+// The error grid's context works on the coarse context's stream and nothing is read on the host, so
+// the reverse sweep's indicator steps queue up behind its kernels (three launches a step; with a
+// host round trip for dt, iteration and totals, a dt array allocated and freed and the sums' 256 parts
+// added by one thread, a step of 10k coarse cells took 210 us).
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -35,7 +40,19 @@ template <class R>
 __global__ void __launch_bounds__(kBlock) k_dwr_interp(int nf, const int32_t *__restrict__ idx,
                                                        const double *__restrict__ w, Fields<R> un, Fields<R> unext,
                                                        Fields<R> lam, R *fh, R *fhu, R *fhv,
-                                                       double *__restrict__ ut_next, double *__restrict__ lamt) {
+                                                       double *__restrict__ ut_next, double *__restrict__ lamt,
+                                                       uint8_t *__restrict__ seg_clean, uint8_t *__restrict__ seg_wet,
+                                                       int nseg, const DevScalars *__restrict__ coarse,
+                                                       DevScalars *__restrict__ fine) {
+    // the error grid's state is new everywhere, its time that of the step's beginning
+    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < nseg; s += gridDim.x * blockDim.x) {
+        seg_clean[s] = 0;
+        seg_wet[s] = 1;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        fine->time = coarse->time - coarse->dt;  // enters the step only through clipping, which the replay skips
+        fine->iter = coarse->iter - 1;
+    }
     for (int f = blockIdx.x * blockDim.x + threadIdx.x; f < nf; f += gridDim.x * blockDim.x) {
         double a[3] = {0, 0, 0}, b[3] = {0, 0, 0}, c[3] = {0, 0, 0};
         for (int q = 0; q < 4; ++q) {
@@ -58,38 +75,6 @@ __global__ void __launch_bounds__(kBlock) k_dwr_interp(int nf, const int32_t *__
     }
 }
 
-template <class R>
-__global__ void __launch_bounds__(kBlock) k_dwr_residual(int nf, const int32_t *__restrict__ parent, Fields<R> uf,
-                                                         const double *__restrict__ ut_next,
-                                                         const double *__restrict__ lamt, Fields<R> lam,
-                                                         double *__restrict__ err, double *__restrict__ corr) {
-    for (int f = blockIdx.x * blockDim.x + threadIdx.x; f < nf; f += gridDim.x * blockDim.x) {
-        const int p = parent[f];
-        double e = 0.0, c = 0.0;
-        for (int v = 0; v < 3; ++v) {
-            const double r = double(uf.get(v, f)) - ut_next[(size_t)v * nf + f];
-            const double l = double(lam.get(v, p));
-            e += fabs(r * (l - lamt[(size_t)v * nf + f]));
-            c += r * l;
-        }
-        err[f] = e;
-        corr[f] = c;
-    }
-}
-
-// Per coarse cell: the sum of its children's el_error in child order.
-__global__ void __launch_bounds__(kBlock) k_dwr_cells(int n, const int32_t *__restrict__ children,
-                                                      const double *__restrict__ err, double *__restrict__ cell) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        double s = 0.0;
-        for (int q = 0; q < 4; ++q) {
-            const int f = children[(size_t)q * n + i];
-            if (f >= 0) s += err[f];
-        }
-        cell[i] = s;
-    }
-}
-
 // Neumaier's compensated addition: (s, c) += x.
 __device__ __forceinline__ void neumaier(double &s, double &c, double x) {
     const double t = s + x;
@@ -100,45 +85,92 @@ __device__ __forceinline__ void neumaier(double &s, double &c, double x) {
     s = t;
 }
 
-// Block b sums its fixed contiguous range of a[] (both arrays) with compensation, thread by
-// thread and then thread 0 over the threads in order; then one block adds the parts.
-__global__ void __launch_bounds__(kBlock) k_dwr_sum_parts(int nf, const double *__restrict__ a,
-                                                          const double *__restrict__ b, double *__restrict__ parts) {
-    __shared__ double ss[2][kBlock], cc[2][kBlock];
-    const int per = (nf + kParts - 1) / kParts;
-    const int f0 = blockIdx.x * per, f1 = min(nf, f0 + per);
-    double s0 = 0, c0 = 0, s1 = 0, c1 = 0;
-    for (int f = f0 + threadIdx.x; f < f1; f += kBlock) {
-        neumaier(s0, c0, a[f]);
-        neumaier(s1, c1, b[f]);
-    }
-    ss[0][threadIdx.x] = s0;
-    cc[0][threadIdx.x] = c0;
-    ss[1][threadIdx.x] = s1;
-    cc[1][threadIdx.x] = c1;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int k = 0; k < 2; ++k) {
-            double s = 0, c = 0;
-            for (int t = 0; t < kBlock; ++t) {
-                neumaier(s, c, ss[k][t]);
-                neumaier(s, c, cc[k][t]);
-            }
-            parts[(size_t)4 * blockIdx.x + 2 * k] = s;
-            parts[(size_t)4 * blockIdx.x + 2 * k + 1] = c;
-        }
+// (s, c) += (s2, c2), both compensated sums: the rounding error of s + s2 goes to the compensation.
+__device__ __forceinline__ void add_sums(double &s, double &c, double s2, double c2) {
+    neumaier(s, c, s2);
+    c += c2;
+}
+__device__ __forceinline__ void warp_sums(double &s, double &c) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const double s2 = __shfl_down_sync(0xffffffffu, s, o), c2 = __shfl_down_sync(0xffffffffu, c, o);
+        add_sums(s, c, s2, c2);
     }
 }
+// Thread 0: the sum over the block's threads, warps in order.
+__device__ __forceinline__ void block_sums(double &s, double &c, double (*red)[2]) {
+    warp_sums(s, c);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) {
+        red[threadIdx.x >> 5][0] = s;
+        red[threadIdx.x >> 5][1] = c;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+        for (int w = 1; w < kBlock / 32; ++w) add_sums(s, c, red[w][0], red[w][1]);
+}
 
-__global__ void k_dwr_sum_final(const double *__restrict__ parts, double *__restrict__ out) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    for (int k = 0; k < 2; ++k) {
-        double s = 0, c = 0;
-        for (int b = 0; b < kParts; ++b) {
-            neumaier(s, c, parts[(size_t)4 * b + 2 * k]);
-            neumaier(s, c, parts[(size_t)4 * b + 2 * k + 1]);
+// One thread per coarse cell: its children's residuals and estimates in child order.  Block b takes a
+// fixed contiguous range of coarse cells; the last block adds the parts and writes the totals to
+// out[0..1].  acc (or null): the estimate per coarse cell is added there too.
+template <class R>
+__global__ void __launch_bounds__(kBlock) k_dwr_residual(int n, int nf, const int32_t *__restrict__ children, Fields<R> uf,
+                                                         const double *__restrict__ ut_next,
+                                                         const double *__restrict__ lamt, Fields<R> lam,
+                                                         double *__restrict__ err, double *__restrict__ cell,
+                                                         double *__restrict__ acc, double *parts, unsigned *done,
+                                                         double *__restrict__ out) {
+    __shared__ double red[kBlock / 32][2];
+    __shared__ bool last;
+    const int per = (n + kParts - 1) / kParts;
+    const int i0 = blockIdx.x * per, i1 = min(n, i0 + per);
+    double es = 0, ec = 0, cs = 0, cc = 0;
+    for (int i = i0 + threadIdx.x; i < i1; i += kBlock) {
+        const double l[3] = {double(lam.h[i]), double(lam.hu[i]), double(lam.hv[i])};
+        double sum = 0.0;
+        for (int q = 0; q < 4; ++q) {
+            const int f = children[(size_t)q * n + i];
+            if (f < 0) continue;
+            double e = 0.0, c = 0.0;
+            for (int v = 0; v < 3; ++v) {
+                const double r = double(uf.get(v, f)) - ut_next[(size_t)v * nf + f];
+                e += fabs(r * (l[v] - lamt[(size_t)v * nf + f]));
+                c += r * l[v];
+            }
+            err[f] = e;
+            sum += e;
+            neumaier(es, ec, e);
+            neumaier(cs, cc, c);
         }
-        out[k] = s + c;
+        cell[i] = sum;
+        if (acc) acc[i] += sum;
+    }
+    block_sums(es, ec, red);
+    block_sums(cs, cc, red);
+    double *p = parts + (size_t)4 * blockIdx.x;
+    if (threadIdx.x == 0) {
+        p[0] = es;
+        p[1] = ec;
+        p[2] = cs;
+        p[3] = cc;
+        __threadfence();
+        last = atomicAdd(done, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    static_assert(kParts == kBlock, "one thread per part");
+    p = parts + (size_t)4 * threadIdx.x;
+    es = __ldcg(p);
+    ec = __ldcg(p + 1);
+    cs = __ldcg(p + 2);
+    cc = __ldcg(p + 3);
+    block_sums(es, ec, red);
+    block_sums(cs, cc, red);
+    if (threadIdx.x == 0) {
+        out[0] = es + ec;
+        out[1] = cs + cc;
+        *done = 0u;
     }
 }
 
@@ -148,29 +180,28 @@ Fields<R> fields(void *const U[3]) {
 }
 
 template <class R>
-int run_t(da_ctx *ctx, DwrState &d, int un, int unext, int lam, double dt, double time0, long long iter0) {
+int run_t(da_ctx *ctx, DwrState &d, int un, int unext, int lam, long long iter0, double *acc, double *out) {
     da_ctx *fc = d.fine;
     const int nf = fc->mesh.n, grid = (ctx->sm_count > 0 ? ctx->sm_count : 148) * 8;
+    fc->cur = 0;  // every indicator step uses the same buffers
     k_dwr_interp<R><<<grid, kBlock, 0, ctx->stream>>>(nf, d.interp, d.weight, fields<R>(ctx->U[un]),
                                                       fields<R>(ctx->U[unext]), fields<R>(ctx->lam[lam]),
-                                                      (R *)fc->U[fc->cur][0], (R *)fc->U[fc->cur][1],
-                                                      (R *)fc->U[fc->cur][2], d.ut_next, d.lamt);
+                                                      (R *)fc->U[0][0], (R *)fc->U[0][1], (R *)fc->U[0][2], d.ut_next,
+                                                      d.lamt, fc->seg_clean, fc->seg_wet, fc->nseg, ctx->dsc, fc->dsc);
     int st = cuda_check(ctx, cudaGetLastError(), "dwr interpolation");
-    if (!st) st = cuda_check(ctx, cudaStreamSynchronize(ctx->stream), "sync");
-    // one step of the error grid from U~^n with the coarse dt and iteration
-    if (!st) st = forward_state_changed(fc);
-    if (!st) st = cuda_check(fc, cudaStreamSynchronize(fc->stream), "sync");
     fc->have_state = true;
-    if (!st) st = da_set_time(fc, time0, iter0);
-    if (!st) st = da_set_dt_replay(fc, &dt, 1, iter0);
-    if (!st) st = launch_forward_step(fc);
-    if (!st) st = cuda_check(fc, cudaStreamSynchronize(fc->stream), "sync");
+    // one step of the error grid from U~^n with the coarse dt, read where the coarse step left it
+    fc->tc.dt_replay = &ctx->dsc->dt;
+    fc->tc.iter0 = iter0;
+    fc->tc.n_replay = 1;
     if (!st) {
-        k_dwr_residual<R><<<grid, kBlock, 0, ctx->stream>>>(nf, d.parent, fields<R>(fc->U[fc->cur]), d.ut_next, d.lamt,
-                                                            fields<R>(ctx->lam[lam]), d.err, d.corr);
-        k_dwr_cells<<<grid, kBlock, 0, ctx->stream>>>(ctx->mesh.n, d.children, d.err, d.cell);
-        k_dwr_sum_parts<<<kParts, kBlock, 0, ctx->stream>>>(nf, d.err, d.corr, d.parts);
-        k_dwr_sum_final<<<1, 32, 0, ctx->stream>>>(d.parts, d.sums);
+        st = launch_single_step(fc);
+        if (st) set_error(ctx, st, std::string("dwr step of the error grid: ") + da_last_error(fc));
+    }
+    if (!st) {
+        k_dwr_residual<R><<<kParts, kBlock, 0, ctx->stream>>>(ctx->mesh.n, nf, d.children, fields<R>(fc->U[fc->cur]),
+                                                              d.ut_next, d.lamt, fields<R>(ctx->lam[lam]), d.err, d.cell,
+                                                              acc, d.parts, d.done, out);
         st = cuda_check(ctx, cudaGetLastError(), "dwr residual");
     }
     return st;
@@ -185,8 +216,18 @@ int read_scalars(da_ctx *ctx) {
 
 void free_dwr(da_ctx *ctx) {
     DwrState &d = ctx->dwr;
-    if (d.fine) da_destroy(d.fine);
+    if (d.fine) {
+        if (ctx->stream) cudaStreamSynchronize(ctx->stream);
+        d.fine->stream = d.fine_stream;  // its own again
+        da_destroy(d.fine);
+        // a captured sweep may hold launches on the error grid
+        if (ctx->sweep_graph) cudaGraphExecDestroy(ctx->sweep_graph);
+        ctx->sweep_graph = nullptr;
+        ctx->sweep_key.clear();
+    }
     if (d.mem) cudaFree(d.mem);
+    if (d.acc) cudaFree(d.acc);
+    if (d.step_sums) cudaFree(d.step_sums);
     d = DwrState{};
 }
 
@@ -194,9 +235,23 @@ void free_dwr(da_ctx *ctx) {
 
 void dwr_release(da_ctx *ctx) { free_dwr(ctx); }
 
-int dwr_indicator(da_ctx *ctx, int un, int unext, int lam, double dt, double time0, long long iter0) {
-    return ctx->p.precision == DA_PREC_FP64 ? run_t<double>(ctx, ctx->dwr, un, unext, lam, dt, time0, iter0)
-                                            : run_t<float>(ctx, ctx->dwr, un, unext, lam, dt, time0, iter0);
+int dwr_indicator(da_ctx *ctx, int un, int unext, int lam, long long iter0, double *acc, double *out) {
+    return ctx->p.precision == DA_PREC_FP64 ? run_t<double>(ctx, ctx->dwr, un, unext, lam, iter0, acc, out)
+                                            : run_t<float>(ctx, ctx->dwr, un, unext, lam, iter0, acc, out);
+}
+
+int dwr_accumulators(da_ctx *ctx, int nsteps) {
+    DwrState &d = ctx->dwr;
+    int st = DA_OK;
+    if (!d.acc) st = cuda_check(ctx, cudaMalloc((void **)&d.acc, sizeof(double) * (size_t)ctx->mesh.n), "cudaMalloc(dwr cells)");
+    if (!st && d.step_cap < nsteps) {
+        if (d.step_sums) cudaFree(d.step_sums);
+        d.step_sums = nullptr;
+        d.step_cap = 0;
+        st = cuda_check(ctx, cudaMalloc((void **)&d.step_sums, sizeof(double) * 2 * (size_t)nsteps), "cudaMalloc(dwr sums)");
+        if (!st) d.step_cap = nsteps;
+    }
+    return st;
 }
 
 }  // namespace da
@@ -236,32 +291,35 @@ int da_dwr_setup(da_ctx *ctx, const da_mesh_soa *fine, const int32_t *parent, co
         free_dwr(ctx);
         return st;
     }
-    // device tables: parent, children, interpolants, weights, work arrays
+    // the error grid's launches go out on the coarse context's stream, in order with its own
+    cudaStreamSynchronize(d.fine->stream);
+    d.fine_stream = d.fine->stream;
+    d.fine->stream = ctx->stream;
+    // device tables: children, interpolants, weights, work arrays
     size_t off = 0;
     auto take = [&](size_t bytes) { const size_t o = off; off = (off + bytes + 255) & ~size_t(255); return o; };
-    const size_t o_par = take(4 * (size_t)nf), o_ch = take(4 * (size_t)4 * n), o_idx = take(4 * (size_t)4 * nf),
+    const size_t o_ch = take(4 * (size_t)4 * n), o_idx = take(4 * (size_t)4 * nf),
                  o_w = take(8 * (size_t)4 * nf), o_ut = take(8 * (size_t)3 * nf), o_lt = take(8 * (size_t)3 * nf),
-                 o_err = take(8 * (size_t)nf), o_corr = take(8 * (size_t)nf), o_cell = take(8 * (size_t)n),
-                 o_parts = take(8 * (size_t)4 * kParts), o_sums = take(8 * 2);
+                 o_err = take(8 * (size_t)nf), o_cell = take(8 * (size_t)n),
+                 o_parts = take(8 * (size_t)4 * kParts), o_sums = take(8 * 2), o_done = take(sizeof(unsigned));
     st = cuda_check(ctx, cudaMalloc(&d.mem, off), "cudaMalloc(dwr)");
     if (st) {
         free_dwr(ctx);
         return st;
     }
     unsigned char *b = (unsigned char *)d.mem;
-    d.parent = (int32_t *)(b + o_par);
     d.children = (int32_t *)(b + o_ch);
     d.interp = (int32_t *)(b + o_idx);
     d.weight = (double *)(b + o_w);
     d.ut_next = (double *)(b + o_ut);
     d.lamt = (double *)(b + o_lt);
     d.err = (double *)(b + o_err);
-    d.corr = (double *)(b + o_corr);
     d.cell = (double *)(b + o_cell);
     d.parts = (double *)(b + o_parts);
     d.sums = (double *)(b + o_sums);
+    d.done = (unsigned *)(b + o_done);
     d.nf = nf;
-    st = copy_h2d(ctx, d.parent, parent, 4 * (size_t)nf, "copy");
+    st = cuda_check(ctx, cudaMemsetAsync(d.done, 0, sizeof(unsigned), ctx->stream), "memset");
     if (!st) st = copy_h2d(ctx, d.children, children.data(), 4 * (size_t)4 * n, "copy");
     if (!st) st = copy_h2d(ctx, d.interp, interp, 4 * (size_t)4 * nf, "copy");
     if (!st) st = copy_h2d(ctx, d.weight, weight, 8 * (size_t)4 * nf, "copy");
@@ -280,13 +338,11 @@ int da_dwr_step(da_ctx *ctx, const double *lambda_next, double *el_error, double
     // the coarse step n -> n+1 from a base checkpoint, put back afterwards
     if (!st) st = launch_snapshot(ctx, ctx->snaps[0], true);
     if (!st) st = read_scalars(ctx);
-    const double time0 = ctx->hsc->time;
     const long long iter0 = ctx->hsc->iter;
-    if (!st) st = launch_forward_step(ctx);
+    if (!st) st = launch_single_step(ctx);
     if (!st) st = read_scalars(ctx);
     if (!st) st = device_error(ctx, "da_dwr_step: the coarse step");
-    const double dt = ctx->hsc->dt;
-    if (!st) st = dwr_indicator(ctx, 1 - ctx->cur, ctx->cur, 0, dt, time0, iter0);
+    if (!st) st = dwr_indicator(ctx, 1 - ctx->cur, ctx->cur, 0, iter0, nullptr, ctx->dwr.sums);
     if (!st) st = launch_snapshot(ctx, ctx->snaps[0], false);
     if (!st) st = cuda_check(ctx, cudaStreamSynchronize(ctx->stream), "sync");
     const int nf = ctx->dwr.nf;
