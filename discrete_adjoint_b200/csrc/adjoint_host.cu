@@ -11,6 +11,7 @@
 // the recursion of binomial checkpointing (Griewank's revolve), solved by dynamic programming.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -88,6 +89,9 @@ int adj_alloc(da_ctx *ctx, int nsnap) {
     const size_t rs = rsize(ctx);
     int st = DA_OK;
     const int nouts = (ctx->ninst > 0 ? ctx->ninst : 1) * (DA_MAX_MATERIALS + 1 + DA_MAX_PILES);
+    // partial sums: the single instance's, or (n_materials + 2) outputs of every member
+    const size_t nparts = std::max((size_t)kAdjReduceParts * (DA_MAX_MATERIALS + 1 + DA_MAX_PILES),
+                                   (size_t)kAdjInstParts * ctx->ninst * (ctx->p.n_materials + 2));
     if (ctx->adj_n != (int)n || ctx->adj_ninst != ctx->ninst) {
         auto fr = [](void *p) { if (p) cudaFree(p); };
         fr(ctx->mask); fr(ctx->adjA); fr(ctx->adjB); fr(ctx->gbed); fr(ctx->gint); fr(ctx->dk_tab);
@@ -108,7 +112,7 @@ int adj_alloc(da_ctx *ctx, int nsnap) {
         if (!st) st = cuda_check(ctx, cudaMalloc((void **)&ctx->gint, sizeof(double) * n), "cudaMalloc(gint)");
         if (!st) st = cuda_check(ctx, cudaMalloc((void **)&ctx->dk_tab, sizeof(double) * 2 * DA_MAX_MATERIALS * 3), "cudaMalloc");
         if (!st) st = cuda_check(ctx, cudaMalloc((void **)&ctx->red_out, sizeof(double) * nouts), "cudaMalloc");
-        if (!st) st = cuda_check(ctx, cudaMalloc((void **)&ctx->red_part, sizeof(double) * kAdjReduceParts * (DA_MAX_MATERIALS + 1 + DA_MAX_PILES)), "cudaMalloc");
+        if (!st) st = cuda_check(ctx, cudaMalloc((void **)&ctx->red_part, sizeof(double) * nparts), "cudaMalloc");
         if (!st) st = cuda_check(ctx, cudaMalloc((void **)&ctx->inst_J, sizeof(double) * (ctx->ninst > 0 ? ctx->ninst : 1)), "cudaMalloc");
         if (!st) st = cuda_check(ctx, cudaMalloc((void **)&ctx->seg_J, sizeof(double) * ctx->nseg), "cudaMalloc");
         if (st) return st;
@@ -460,12 +464,12 @@ int adjoint_sweep(da_ctx *ctx, const double *box, int32_t nsteps, int32_t nsnaps
     // the launches of the sweep, from the base checkpoint to the gradient sums
     auto sweep = [&]() -> int {
         int s = store(ctx, 0);
+        if (!s && r.dwr)
+            s = cuda_check(ctx, cudaMemsetAsync(ctx->dwr.acc, 0, sizeof(double) * (size_t)ctx->mesh.n, ctx->stream), "memset");
         r.pos = 0;
         if (!s) s = r.reverse(0, nsteps, 0);
         if (!s) s = r.flush();
         if (!s) s = restore(ctx, 0);
-        if (!s && r.dwr)
-            s = cuda_check(ctx, cudaMemsetAsync(ctx->dwr.acc, 0, sizeof(double) * (size_t)ctx->mesh.n, ctx->stream), "memset");
         if (!s) s = launch_functional(ctx, ctx->inst_J);
         if (!s) s = ctx->ninst > 0 ? launch_adjoint_reduce_inst(ctx, r.lam_cur) : launch_adjoint_reduce(ctx, r.lam_cur, n_piles);
         return s;
@@ -473,14 +477,14 @@ int adjoint_sweep(da_ctx *ctx, const double *box, int32_t nsteps, int32_t nsnaps
     bool graph = !ctx->trace.on && ctx->p.jacobian_mode == DA_JAC_EXACT;
     if (graph) {
         std::vector<unsigned char> key = sweep_key(ctx, box, nsteps, nsnapshots, n_piles, r.seeded, r.sec2, r.cos_int);
-        if (!ctx->sweep_graph || key != ctx->sweep_key) {
-            if (ctx->sweep_graph) cudaGraphExecDestroy(ctx->sweep_graph);
-            ctx->sweep_graph = nullptr;
-            ctx->sweep_key.clear();
         // the error grid's own tables are fixed until it is released, which drops the graph
         const long long dwr_key[4] = {r.dwr, r.iter_begin, (long long)(uintptr_t)(r.dwr ? ctx->dwr.acc : nullptr),
                                       (long long)(uintptr_t)(r.dwr ? ctx->dwr.step_sums : nullptr)};
         key.insert(key.end(), (const unsigned char *)dwr_key, (const unsigned char *)(dwr_key + 4));
+        if (!ctx->sweep_graph || key != ctx->sweep_key) {
+            if (ctx->sweep_graph) cudaGraphExecDestroy(ctx->sweep_graph);
+            ctx->sweep_graph = nullptr;
+            ctx->sweep_key.clear();
             // capture: nothing runs; the host-side state the launches leave is kept for replays
             const Runner r0 = r;
             const int cur0 = ctx->cur;

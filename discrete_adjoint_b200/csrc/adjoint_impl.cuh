@@ -653,17 +653,23 @@ __global__ void __launch_bounds__(kBlock) k_adj_reduce(MeshArgs m, StateRef<R> L
     }
 }
 
-// Ensemble: block (k, o) sums output o of member k over the member's cells, in a fixed order:
-// o < n_mat the basal-friction sensitivities of material o, o == n_mat the internal friction,
-// o == n_mat + 1 the member's pile height (lambda_h dh0/dP).
+// Ensemble: output o of member k -- o < n_mat the basal-friction sensitivities of material o, o == n_mat
+// the internal friction, o == n_mat + 1 the member's pile height (lambda_h dh0/dP) -- in a fixed
+// order: block (b, k, o) sums the b-th of kInstParts contiguous cell ranges of the member, then a
+// warp per output adds the parts.  (One block per output left most of the GPU idle: 24 members of 75k
+// cells took 523 us.)
+constexpr int kInstParts = kAdjInstParts;
+
 template <class R>
 __global__ void __launch_bounds__(kBlock) k_adj_reduce_inst(MeshArgs m, StateRef<R> L0, const double *__restrict__ gbed,
                                                             const double *__restrict__ gint,
                                                             const double *__restrict__ dh0, int n_mat,
-                                                            const int32_t *__restrict__ seg0, double *__restrict__ out) {
+                                                            const int32_t *__restrict__ seg0, double *__restrict__ part) {
     __shared__ double red[kBlock / 32];
-    const int k = blockIdx.x, o = blockIdx.y;
-    const int i0 = seg0[k] * 32, i1 = min(m.n, seg0[k + 1] * 32);
+    const int k = blockIdx.y, o = blockIdx.z, nout = n_mat + 2;
+    const int first = seg0[k] * 32, last = min(m.n, seg0[k + 1] * 32);
+    const int per = (last - first + kInstParts - 1) / kInstParts;
+    const int i0 = first + (int)blockIdx.x * per, i1 = min(last, i0 + per);
     double acc = 0.0;
     for (int i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
         if (o < n_mat) {
@@ -680,8 +686,17 @@ __global__ void __launch_bounds__(kBlock) k_adj_reduce_inst(MeshArgs m, StateRef
     if (threadIdx.x == 0) {
         double t = 0.0;
         for (int w = 0; w < kBlock / 32; ++w) t += red[w];
-        out[(size_t)k * (n_mat + 2) + o] = t;
+        part[((size_t)k * nout + o) * kInstParts + blockIdx.x] = t;
     }
+}
+
+__global__ void __launch_bounds__(kBlock) k_adj_reduce_inst_final(const double *__restrict__ part, int n,
+                                                                  double *__restrict__ out) {
+    static_assert(kInstParts == 32, "a lane per part");
+    const int w = (blockIdx.x * kBlock + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (w >= n) return;
+    const double v = warp_sum(part[(size_t)w * kInstParts + lane]);
+    if (lane == 0) out[w] = v;
 }
 
 __global__ void __launch_bounds__(kReduceParts) k_adj_reduce_final(const double *__restrict__ part,

@@ -33,6 +33,7 @@ struct MatConsts {
 
 // Scalars that live on the device so that whole step loops run without host round trips.
 constexpr int kAdjReduceParts = 128;  // cell ranges of the gradient reduction
+constexpr int kAdjInstParts = 32;     // the same of each ensemble member
 
 struct DevScalars {
     double time;          // TimeProps::time
@@ -108,11 +109,11 @@ struct DwrState {
     double *cell = nullptr;      // [n] el_error summed over each coarse cell's children
     double *parts = nullptr;     // compensated partial sums
     double *sums = nullptr;      // [2] total el_error, total correction
-};
     unsigned *done = nullptr;    // last-block counter of the sums
     double *acc = nullptr;       // [n] el_error per coarse cell over a sweep
     double *step_sums = nullptr; // [step_cap][2] totals of each step of a sweep
     int step_cap = 0;
+};
 
 // Device copy of the flattened mesh.  FP64 path reads the double arrays; the FP32-split
 // path reads the float copies.
@@ -198,7 +199,7 @@ struct da_ctx {
     std::vector<int32_t> inst_npile;  // [ninst] piles of each member (0 or 1)
     void *inst_mem = nullptr;         // one allocation holding every InstArgs table
     double *inst_vol = nullptr;       // [ninst] members' volumes (stats)
-    std::vector<double> inst_init;    // [3][n] members' initial states, concatenated (restart)
+    void *inst_init[3] = {nullptr, nullptr, nullptr};  // [n] members' initial states, concatenated (restart)
     da::DwrState dwr;                 // error grid of the DWR indicator (da_dwr_setup)
     da::OutlineGrid outline;          // maximum-depth map (da_outline_init)
     double *stats_mem = nullptr;      // partial sums and result of the flow statistics (stats.cu)

@@ -29,7 +29,10 @@ void free_members(da_ctx *ctx) {
     ctx->inst_ncell.clear();
     ctx->inst_nmat.clear();
     ctx->inst_npile.clear();
-    ctx->inst_init.clear();
+    for (void *&p : ctx->inst_init) {
+        if (p) cudaFree(p);
+        p = nullptr;
+    }
 }
 
 namespace {
@@ -47,30 +50,25 @@ int member_ok(const da_member &m) {
     return 1;
 }
 
-// Starting values of a member's step scalars (the same as a fresh single-instance context).
-void reset_member_scalars(std::vector<double> &time, std::vector<unsigned long long> &acc_min,
-                          std::vector<unsigned long long> &acc_max) {
+// Starting values of the members' step scalars (the same as a fresh single-instance context); dt,
+// min_dxe and hmax of a member that has not stepped yet are zero.
+__global__ void k_member_start(InstArgs ia, unsigned long long acc_min0) {
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < ia.ninst; k += gridDim.x * blockDim.x) {
+        ia.time[k] = 0.0;
+        ia.dt[k] = 0.0;
+        ia.min_dxe[k] = 0.0;
+        ia.hmax[k] = 0.0;
+        ia.acc_min[k] = acc_min0;
+        ia.acc_max[k] = 0ull;
+    }
+}
+
+int start_member_scalars(da_ctx *ctx) {
     const double init = 10000000.0;  // min_dx_dy_evalue start value, get_coef_and_eigen.C:36
     unsigned long long bits;
     std::memcpy(&bits, &init, sizeof(bits));
-    std::fill(time.begin(), time.end(), 0.0);
-    std::fill(acc_min.begin(), acc_min.end(), bits);
-    std::fill(acc_max.begin(), acc_max.end(), 0ull);
-}
-
-int upload_member_scalars(da_ctx *ctx) {
-    const int nm = ctx->ninst;
-    std::vector<double> time(nm);
-    std::vector<unsigned long long> amin(nm), amax(nm);
-    reset_member_scalars(time, amin, amax);
-    int st = copy_h2d(ctx, ctx->ia.time, time.data(), sizeof(double) * nm, "copy");
-    // dt, min_dxe, hmax of a member that has not stepped yet: zero
-    if (!st) st = copy_h2d(ctx, ctx->ia.dt, time.data(), sizeof(double) * nm, "copy");
-    if (!st) st = copy_h2d(ctx, ctx->ia.min_dxe, time.data(), sizeof(double) * nm, "copy");
-    if (!st) st = copy_h2d(ctx, ctx->ia.hmax, time.data(), sizeof(double) * nm, "copy");
-    if (!st) st = copy_h2d(ctx, ctx->ia.acc_min, amin.data(), sizeof(unsigned long long) * nm, "copy");
-    if (!st) st = copy_h2d(ctx, ctx->ia.acc_max, amax.data(), sizeof(unsigned long long) * nm, "copy");
-    return st;
+    k_member_start<<<(ctx->ninst + 255) / 256, 256, 0, ctx->stream>>>(ctx->ia, bits);
+    return cuda_check(ctx, cudaGetLastError(), "member scalars");
 }
 
 }  // namespace
@@ -217,8 +215,14 @@ int da_ensemble_upload(da_ctx *ctx, const da_member *members, int32_t n_members)
         ctx->inst_nmat.push_back(members[k].n_materials);
         ctx->inst_npile.push_back(members[k].dh0_dpile ? 1 : 0);
     }
-    ctx->inst_init.swap(init);
-    if (!st) st = upload_member_scalars(ctx);
+    // the initial states stay on the device for da_ensemble_restart
+    const size_t rs = ctx->p.precision == DA_PREC_FP64 ? sizeof(double) : sizeof(float);
+    for (int v = 0; v < 3 && !st; ++v) {
+        st = cuda_check(ctx, cudaMalloc(&ctx->inst_init[v], rs * N), "cudaMalloc(initial states)");
+        if (!st) st = upload_real(ctx, ctx->inst_init[v], init.data() + (size_t)v * N);
+        // the staging buffer and the host array are reused
+        if (!st) st = cuda_check(ctx, cudaStreamSynchronize(ctx->stream), "sync");
+    }
     if (!st && any_pile) {
         st = cuda_check(ctx, cudaMalloc((void **)&ctx->dh0, sizeof(double) * N), "cudaMalloc(dh0)");
         if (!st) ctx->dh0_bytes = sizeof(double) * N;
@@ -232,13 +236,16 @@ int da_ensemble_upload(da_ctx *ctx, const da_member *members, int32_t n_members)
 int da_ensemble_restart(da_ctx *ctx) {
     if (!ctx) return DA_ERR_INVALID;
     if (ctx->ninst <= 0) return set_error(ctx, DA_ERR_INVALID, "da_ensemble_restart: not an ensemble context");
-    const size_t N = (size_t)ctx->mesh.n;
-    const int nm = ctx->ninst;
-    ctx->ninst = 0;  // da_set_state is a single-context call; the layout is unchanged
-    int st = da_set_state(ctx, ctx->inst_init.data(), ctx->inst_init.data() + N, ctx->inst_init.data() + 2 * N);
-    ctx->ninst = nm;
+    cudaSetDevice(ctx->device);
+    const size_t N = (size_t)ctx->mesh.n, rs = ctx->p.precision == DA_PREC_FP64 ? sizeof(double) : sizeof(float);
+    int st = DA_OK;
+    for (int v = 0; v < 3 && !st; ++v)
+        st = cuda_check(ctx, cudaMemcpyAsync(ctx->U[ctx->cur][v], ctx->inst_init[v], rs * N, cudaMemcpyDeviceToDevice,
+                                             ctx->stream), "initial states");
+    if (!st) st = forward_state_changed(ctx);
+    if (!st) ctx->have_state = true;
     if (!st) st = da_set_time(ctx, 0.0, 0);
-    if (!st) st = upload_member_scalars(ctx);
+    if (!st) st = start_member_scalars(ctx);
     return st;
 }
 
