@@ -133,8 +133,14 @@ __device__ __forceinline__ void make_side(int dir, R h, R hu, R hv, R k, R gz, S
     }
 }
 
-// Reverse of dirflux for a wet side: adjoints of (u, f, s) -> adjoints of (h, hu, hv, k).
+// Quotients of the derivatives: the division operator.
 template <class R>
+struct OperatorQuot {
+    static __device__ __forceinline__ R div(R a, R b) { return a / b; }
+};
+
+// Reverse of dirflux for a wet side: adjoints of (u, f, s) -> adjoints of (h, hu, hv, k).
+template <class R, class Q = OperatorQuot<R>>
 __device__ __forceinline__ void dirflux_adj(int dir, const Side<R> &s, const R au[3], const R af[3], const R as[3],
                                             R g[3], R &gk) {
     if (s.h < R(DA_TINY)) {
@@ -144,9 +150,9 @@ __device__ __forceinline__ void dirflux_adj(int dir, const Side<R> &s, const R a
     }
     // derivatives only (no branch depends on them): one reciprocal of h serves all quotients
     const R vel = s.vel, a = s.a, h = s.h;
-    const R ih = R(1) / h;
+    const R ih = Q::div(R(1), h);
     const R da_dh = a > R(0) ? R(0.5) * a * ih : R(0);
-    const R da_dk = (a > R(0) && s.k > R(0)) ? R(0.5) * a / s.k : R(0);
+    const R da_dk = (a > R(0) && s.k > R(0)) ? Q::div(R(0.5) * a, s.k) : R(0);
     const R avel_s = as[0] + as[1] + as[2];
     const R aa = -as[0] + as[2];
     if (dir == 0) {
@@ -168,7 +174,7 @@ __device__ __forceinline__ void dirflux_adj(int dir, const Side<R> &s, const R a
 
 // mu^T dF/d(left, right) for F = riemannflux(left, right) (element2.C:2228-2264), with the
 // branch decisions of the forward evaluation.
-template <class R>
+template <class R, class Q = OperatorQuot<R>>
 __device__ __forceinline__ void riemann_adj(int dir, const Side<R> &L, const Side<R> &Rt, const R mu[3], R gL[3],
                                             R gR[3], R &gkL, R &gkR) {
     gL[0] = gL[1] = gL[2] = gR[0] = gR[1] = gR[2] = R(0);
@@ -211,7 +217,7 @@ __device__ __forceinline__ void riemann_adj(int dir, const Side<R> &L, const Sid
         afr[0] = mu[0]; afr[1] = mu[1]; afr[2] = mu[2];
     } else {
         // derivatives of F = (sr fl - sl fr + sl sr du) / D: one reciprocal of D serves them all
-        const R iD = R(1) / (sr - sl);
+        const R iD = Q::div(R(1), sr - sl);
         R a_sr = 0, a_sl = 0;
 #pragma unroll
         for (int v = 0; v < 3; ++v) {
@@ -237,8 +243,8 @@ __device__ __forceinline__ void riemann_adj(int dir, const Side<R> &L, const Sid
         }
     }
     // asl/asr above hold the speed adjoints of the left / right side respectively
-    dirflux_adj<R>(dir, L, aul, afl, asl, gL, gkL);
-    dirflux_adj<R>(dir, Rt, aur, afr, asr, gR, gkR);
+    dirflux_adj<R, Q>(dir, L, aul, afl, asl, gL, gkL);
+    dirflux_adj<R, Q>(dir, Rt, aur, afr, asr, gR, gkR);
 }
 
 // Arrays written and read within one launch of the fused step kernel carry no __restrict__

@@ -5,6 +5,7 @@
 #include "adjoint_impl.cuh"
 #include "forward_impl.cuh"
 #include "adjoint_staged.cuh"
+#include "adjoint_staged64.cuh"
 
 namespace da {
 namespace adj {
@@ -92,6 +93,25 @@ __device__ __forceinline__ bool gather_quarters(const DevScalars *sc, int split)
     return 4ull * __ldcg(&sc->listed) <= gridDim.x;
 }
 
+// The gather of a staged launch in its precision.
+template <class R, bool BATCH>
+__device__ __forceinline__ void gather_staged(const MeshArgs &m, const fwd::HaloArgs &ha, const StateRef<R> &U,
+                                              const StateRef<R> &Ln, const StateOut<R> &Lo, const MatConsts &mc,
+                                              const AdjArgs &aa, double dt, int *list, const InstArgs &ia, void *smem,
+                                              bool quarter) {
+    if constexpr (sizeof(R) == 8)
+        adj_gather_phase64<BATCH>(m, ha, U, Ln, Lo, mc, aa, dt, list, ia, *(GatherSmem64 *)smem, quarter);
+    else
+        adj_gather_phase_staged<R, BATCH>(m, ha, U, Ln, Lo, mc, aa, R(dt), list, ia, *(GatherSmem<R> *)smem, quarter);
+}
+template <class R>
+constexpr size_t gather_staged_bytes() {
+    if constexpr (sizeof(R) == 8)
+        return sizeof(GatherSmem64);
+    else
+        return gather_smem_bytes<R>();
+}
+
 // ------------------------------------------------------------------------ k_youturn
 // One whole reverse step in one cooperative launch: the forward step of U^n replayed with its
 // branch codes recorded (coefficient phase, barrier, dt, update phase), a barrier, the source
@@ -155,8 +175,7 @@ __global__ void __launch_bounds__(kBlock, OCC) k_youturn(MeshArgs m, fwd::StateP
                                                  ntiles, cull, mc, sc, R(dt), ftr, mask, tile_epoch, seg_act, rec_id,
                                                  list, ia, stg, src);
         if (!fwd::grid_sync(sc)) return;
-        adj_gather_phase_staged<R, BATCH>(m, ha, U, Ln, Lo, mc, aa, R(dt), list, ia,
-                                          *reinterpret_cast<GatherSmem<R> *>(dyn_smem), gather_quarters(sc, gsplit));
+        gather_staged<R, BATCH>(m, ha, U, Ln, Lo, mc, aa, dt, list, ia, dyn_smem, gather_quarters(sc, gsplit));
         if (blockIdx.x == 0 && threadIdx.x == 0) {
             sc->iter = iter + 1;
             sc->frict_tiny = ft;
@@ -187,8 +206,7 @@ __global__ void __launch_bounds__(kBlock, OCC) k_youturn(MeshArgs m, fwd::StateP
     adj_src_phase<R, BATCH>(m, U, Ln, mc, aa, R(dt), ftr, list, ia);
     if (!fwd::grid_sync(sc)) return;
     if (STAGED)
-        adj_gather_phase_staged<R, BATCH>(m, ha, U, Ln, Lo, mc, aa, R(dt), list, ia,
-                                          *reinterpret_cast<GatherSmem<R> *>(dyn_smem), gather_quarters(sc, gsplit));
+        gather_staged<R, BATCH>(m, ha, U, Ln, Lo, mc, aa, dt, list, ia, dyn_smem, gather_quarters(sc, gsplit));
     else
         adj_gather_phase<R, BATCH>(m, U, Ln, Lo, mc, aa, R(dt), list, ia);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -233,7 +251,7 @@ int youturn_t(da_ctx *ctx, int lam_in, int lam_out, const double *sec2, double c
     const bool staged = fwd::staged_ok(ctx);
     const void *kern = youturn_kernel<R>(batch, seed, occ3, staged);
     // the staged phases and the staged gather use the same dynamic shared memory in turn
-    const size_t smem = staged ? std::max(fwd::stage_smem_bytes<R>(), gather_smem_bytes<R>()) : 0;
+    const size_t smem = staged ? std::max(fwd::stage_smem_bytes<R>(), gather_staged_bytes<R>()) : 0;
     int &cap_ref = ctx->coop_cap_yt[pi + 2 * batch + 4 * seed + 8 * occ3 + 16 * staged];
     if (cap_ref <= 0) {
         int st = DA_OK;

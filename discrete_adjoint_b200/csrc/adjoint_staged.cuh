@@ -9,7 +9,8 @@
 // host-built halo lists as the forward phases), by asynchronous copies (cp.async) and plain byte
 // loads all in flight together; the faces then read shared memory.  The tile's own A, running
 // parameter sensitivities and neighbour slots come along.  The arithmetic and its order are
-// adj_gather_phase's, so results are identical.
+// adj_gather_phase's, so results are identical.  FP64 has its own gather (adjoint_staged64.cuh); this
+// one is instantiated for FP32 only.
 #pragma once
 
 namespace da {
@@ -27,7 +28,7 @@ struct GatherBuf {
     R h[kSlots], hu[kSlots], hv[kSlots];      // U^n
     R lh[kSlots], lhu[kSlots], lhv[kSlots];   // lambda^{n+1}
     R gz[kSlots];                             // g_z
-    R sx[kSlots], sy[kSlots];                 // cell sizes (FP64: dx, dy; FP32: the float sizes)
+    R sx[kSlots], sy[kSlots];                 // cell sizes
     uint8_t mask[kSlots];                     // recorded branch byte, 0 outside this recording
     uint8_t bf[kSlots];                       // boundary / two-neighbour flags
     uint8_t mat[kSlots];                      // material
@@ -58,15 +59,9 @@ __device__ __forceinline__ void gather_slot(GatherBuf<R> &g, int s, int e, const
     cp_async<B>(&g.lh[s], L.h + e);
     cp_async<B>(&g.lhu[s], L.hu + e);
     cp_async<B>(&g.lhv[s], L.hv + e);
-    if constexpr (sizeof(R) == 8) {
-        cp_async<B>(&g.gz[s], m.g + (size_t)2 * m.n + e);
-        cp_async<B>(&g.sx[s], m.dx + e);
-        cp_async<B>(&g.sy[s], m.dy + e);
-    } else {
-        cp_async<B>(&g.gz[s], m.fg + (size_t)2 * m.n + e);
-        cp_async<B>(&g.sx[s], m.fdx + e);
-        cp_async<B>(&g.sy[s], m.fdy + e);
-    }
+    cp_async<B>(&g.gz[s], m.fg + (size_t)2 * m.n + e);
+    cp_async<B>(&g.sx[s], m.fdx + e);
+    cp_async<B>(&g.sy[s], m.fdy + e);
 #pragma unroll
     for (int q = 0; q < 4; ++q) cp_async<8>(&g.b[q][s], aa.B + (size_t)q * m.n + e);
 }
@@ -184,9 +179,8 @@ __device__ __forceinline__ void gather_cell(const GatherBuf<R> &g, const AdjArgs
     const InstTables it = inst_tables<BATCH>(aa, ia, inst);
     const double dkb = dk_of(it.dk_dbed, mat, code), dki = dk_of(it.dk_dint, mat, code);
     double dJ_dkj = 0.0;
-    // faces f = 2 s + q in the order side s = 0..3, neighbour q = 0 (1 on a hanging side); in
-    // FP64 one loop body for all of them keeps the code small
-#pragma unroll(sizeof(R) == 8 ? 1 : 8)
+    // faces f = 2 s + q in the order side s = 0..3, neighbour q = 0 (1 on a hanging side)
+#pragma unroll
     for (int f = 0; f < 8; ++f) {
         double tb, tg[3], tk;
         face(f >> 1, f & 1, tb, tg, tk);
