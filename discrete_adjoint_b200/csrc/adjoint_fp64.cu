@@ -7,6 +7,9 @@ int launch_adjoint_step_fp64(da_ctx *ctx, int a, int b, const double *sec2, doub
     return adj::step_t<double>(ctx, a, b, sec2, c);
 }
 int launch_adjoint_reduce_fp64(da_ctx *ctx, int a, int np) { return adj::reduce_t<double>(ctx, a, np); }
+int launch_reverse_run_fp64(da_ctx *ctx, int a, const double *sec2, double c, void *const *slots, int n) {
+    return adj::reverse_run_t<double>(ctx, a, sec2, c, slots, n);
+}
 int launch_youturn_fp64(da_ctx *ctx, int a, int b, const double *sec2, double c, bool seed, const double *box,
                         void *pre) {
     return adj::youturn_t<double>(ctx, a, b, sec2, c, seed, box, pre);

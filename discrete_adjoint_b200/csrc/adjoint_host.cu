@@ -35,6 +35,12 @@ int launch_youturn(da_ctx *ctx, int a, int b, const double *sec2, double c, bool
     return ctx->p.precision == DA_PREC_FP64 ? launch_youturn_fp64(ctx, a, b, sec2, c, seed, box, pre_slot)
                                             : launch_youturn_fp32(ctx, a, b, sec2, c, seed, box, pre_slot);
 }
+int launch_reverse_run_fp64(da_ctx *, int, const double *, double, void *const *, int);
+int launch_reverse_run_fp32(da_ctx *, int, const double *, double, void *const *, int);
+int launch_reverse_run(da_ctx *ctx, int a, const double *sec2, double c, void *const *slots, int n) {
+    return ctx->p.precision == DA_PREC_FP64 ? launch_reverse_run_fp64(ctx, a, sec2, c, slots, n)
+                                            : launch_reverse_run_fp32(ctx, a, sec2, c, slots, n);
+}
 int launch_functional(da_ctx *ctx, double *out) {
     return ctx->p.precision == DA_PREC_FP64 ? launch_functional_fp64(ctx, out) : launch_functional_fp32(ctx, out);
 }
@@ -94,16 +100,17 @@ int adj_alloc(da_ctx *ctx, int nsnap) {
                                    (size_t)kAdjInstParts * ctx->ninst * (ctx->p.n_materials + 2));
     if (ctx->adj_n != (int)n || ctx->adj_ninst != ctx->ninst) {
         auto fr = [](void *p) { if (p) cudaFree(p); };
-        fr(ctx->mask); fr(ctx->adjA); fr(ctx->adjB); fr(ctx->gbed); fr(ctx->gint); fr(ctx->dk_tab);
+        fr(ctx->mask); fr(ctx->run_flags); fr(ctx->adjA); fr(ctx->adjB); fr(ctx->gbed); fr(ctx->gint); fr(ctx->dk_tab);
         fr(ctx->red_out); fr(ctx->red_part); fr(ctx->inst_J); fr(ctx->seg_J);
         for (int b = 0; b < 2; ++b)
             for (int v = 0; v < 3; ++v) { fr(ctx->lam[b][v]); ctx->lam[b][v] = nullptr; }
         for (void *s : ctx->snaps) fr(s);
         ctx->snaps.clear();
-        ctx->mask = nullptr; ctx->adjA = ctx->adjB = ctx->gbed = ctx->gint = ctx->dk_tab = nullptr;
+        ctx->mask = ctx->run_flags = nullptr; ctx->adjA = ctx->adjB = ctx->gbed = ctx->gint = ctx->dk_tab = nullptr;
         ctx->red_out = ctx->red_part = ctx->inst_J = ctx->seg_J = nullptr;
         ctx->adj_n = -1;
         st = cuda_check(ctx, cudaMalloc((void **)&ctx->mask, n), "cudaMalloc(mask)");
+        if (!st) st = cuda_check(ctx, cudaMalloc((void **)&ctx->run_flags, 4 * (size_t)ctx->nseg), "cudaMalloc(run flags)");
         for (int b = 0; b < 2 && !st; ++b)
             for (int v = 0; v < 3 && !st; ++v) st = cuda_check(ctx, cudaMalloc(&ctx->lam[b][v], rs * n), "cudaMalloc(lam)");
         if (!st) st = cuda_check(ctx, cudaMalloc((void **)&ctx->adjA, sizeof(double) * 3 * n), "cudaMalloc(A)");
@@ -226,6 +233,21 @@ struct Runner {
         def_mid.n = 0;
         return st;
     }
+    // Consecutive reverse steps of a single instance, each from its own checkpoint (the first perhaps from
+    // the live state), wait here in the same way and go out as one launch (k_reverse_run): until a
+    // forward advance, the end of the sweep or a full list.
+    static constexpr int kRun = 32;  // at most kRunMax of the kernel
+    void *run_slot[kRun];
+    int run_n = 0, run_lam = 0;
+    bool runs() const {
+        return seeded && !dwr && ctx->ninst == 0 && ctx->p.tile_staging >= 1 && ctx->mesh.nloc && ctx->slopes;
+    }
+    int flush_run() {
+        if (run_n == 0) return DA_OK;
+        const int n = run_n;
+        run_n = 0;
+        return launch_reverse_run(ctx, run_lam, sec2, cos_int, run_slot, n);
+    }
     void *take_pending() {
         void *p = pending >= 0 ? ctx->snaps[pending] : nullptr;
         pending = -1;
@@ -234,6 +256,7 @@ struct Runner {
     // k forward steps; store_slot >= 0: the state after them is stored, in the same launch
     int advance(int k, int store_slot = -1) {
         if (k == 0) return DA_OK;  // a pending restore waits for the next launch
+        if (const int st = flush_run()) return st;
         fsteps += k;
         pos += k;
         void *slot = store_slot >= 0 ? ctx->snaps[store_slot] : nullptr;
@@ -254,6 +277,16 @@ struct Runner {
         pos = -1;  // past the step that is being taken back
         if (const int st = flush()) return st;
         if (ctx->p.jacobian_mode == DA_JAC_REFERENCE) return youturn_reference();
+        if (runs()) {
+            void *pre = take_pending();
+            int st = DA_OK;
+            if (run_n == kRun || !pre) st = flush_run();
+            if (run_n == 0) run_lam = lam_cur;
+            run_slot[run_n++] = pre;
+            --left;
+            lam_cur = 1 - lam_cur;
+            return st;
+        }
         // the first reverse step (the horizon's last step) also seeds lambda^N from U^N
         int st = launch_youturn(ctx, lam_cur, 1 - lam_cur, sec2, cos_int, !seeded, box, take_pending());
         if (!st) st = dwr_step();
@@ -415,7 +448,7 @@ std::vector<unsigned char> sweep_key(const da_ctx *ctx, const double *box, int n
     put(iptr, sizeof(iptr));
     const void *ptrs[] = {ctx->U[0][0], ctx->U[0][1], ctx->U[0][2], ctx->U[1][0], ctx->U[1][1], ctx->U[1][2],
                           ctx->lam[0][0], ctx->lam[0][1], ctx->lam[0][2], ctx->lam[1][0], ctx->lam[1][1],
-                          ctx->lam[1][2], ctx->kact, ctx->slopes, ctx->fsign, ctx->active, ctx->seg_clean, ctx->seg_wet, ctx->seg_vol,
+                          ctx->lam[1][2], ctx->kact, ctx->slopes, ctx->fsign, ctx->run_flags, ctx->active, ctx->seg_clean, ctx->seg_wet, ctx->seg_vol,
                           ctx->seg_dirty, ctx->mask, ctx->tile_epoch, ctx->seg_act, ctx->lam_clean, ctx->adjA,
                           ctx->adjB, ctx->gbed, ctx->gint, ctx->dk_tab, ctx->red_out, ctx->red_part, ctx->inst_J,
                           ctx->seg_J, ctx->dh0, ctx->dsc};
@@ -469,6 +502,7 @@ int adjoint_sweep(da_ctx *ctx, const double *box, int32_t nsteps, int32_t nsnaps
         r.pos = 0;
         if (!s) s = r.reverse(0, nsteps, 0);
         if (!s) s = r.flush();
+        if (!s) s = r.flush_run();
         if (!s) s = restore(ctx, 0);
         if (!s) s = launch_functional(ctx, ctx->inst_J);
         if (!s) s = ctx->ninst > 0 ? launch_adjoint_reduce_inst(ctx, r.lam_cur) : launch_adjoint_reduce(ctx, r.lam_cur, n_piles);

@@ -97,12 +97,12 @@ __device__ __forceinline__ bool gather_quarters(const DevScalars *sc, int split)
 template <class R, bool BATCH>
 __device__ __forceinline__ void gather_staged(const MeshArgs &m, const fwd::HaloArgs &ha, const StateRef<R> &U,
                                               const StateRef<R> &Ln, const StateOut<R> &Lo, const MatConsts &mc,
-                                              const AdjArgs &aa, double dt, int *list, const InstArgs &ia, void *smem,
-                                              bool quarter) {
+                                              const AdjArgs &aa, int rec_id, double dt, int *list, const InstArgs &ia,
+                                              void *smem, bool quarter) {
     if constexpr (sizeof(R) == 8)
-        adj_gather_phase64<BATCH>(m, ha, U, Ln, Lo, mc, aa, dt, list, ia, *(GatherSmem64 *)smem, quarter);
+        adj_gather_phase64<BATCH>(m, ha, U, Ln, Lo, mc, aa, rec_id, dt, list, ia, *(GatherSmem64 *)smem, quarter);
     else
-        adj_gather_phase_staged<R, BATCH>(m, ha, U, Ln, Lo, mc, aa, R(dt), list, ia, *(GatherSmem<R> *)smem, quarter);
+        adj_gather_phase_staged<R, BATCH>(m, ha, U, Ln, Lo, mc, aa, rec_id, R(dt), list, ia, *(GatherSmem<R> *)smem, quarter);
 }
 template <class R>
 constexpr size_t gather_staged_bytes() {
@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(kBlock, OCC) k_youturn(MeshArgs m, fwd::StateP
                                                  ntiles, cull, mc, sc, R(dt), ftr, mask, tile_epoch, seg_act, rec_id,
                                                  list, ia, stg, src);
         if (!fwd::grid_sync(sc)) return;
-        gather_staged<R, BATCH>(m, ha, U, Ln, Lo, mc, aa, dt, list, ia, dyn_smem, gather_quarters(sc, gsplit));
+        gather_staged<R, BATCH>(m, ha, U, Ln, Lo, mc, aa, rec_id, dt, list, ia, dyn_smem, gather_quarters(sc, gsplit));
         if (blockIdx.x == 0 && threadIdx.x == 0) {
             sc->iter = iter + 1;
             sc->frict_tiny = ft;
@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(kBlock, OCC) k_youturn(MeshArgs m, fwd::StateP
     adj_src_phase<R, BATCH>(m, U, Ln, mc, aa, R(dt), ftr, list, ia);
     if (!fwd::grid_sync(sc)) return;
     if (STAGED)
-        gather_staged<R, BATCH>(m, ha, U, Ln, Lo, mc, aa, dt, list, ia, dyn_smem, gather_quarters(sc, gsplit));
+        gather_staged<R, BATCH>(m, ha, U, Ln, Lo, mc, aa, rec_id, dt, list, ia, dyn_smem, gather_quarters(sc, gsplit));
     else
         adj_gather_phase<R, BATCH>(m, U, Ln, Lo, mc, aa, R(dt), list, ia);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -222,6 +222,233 @@ __global__ void __launch_bounds__(kBlock, OCC) k_youturn(MeshArgs m, fwd::StateP
         }
     }
     fwd::grid_exit(sc);
+}
+
+// Blocks of a reverse step's launch, cap of them co-resident.
+// FP64: every co-resident block, at most four per tile, whatever the forward steps' tuned grid:
+// the gather spreads a sparse flow's quarter tiles over them, which outweighs the dearer
+// barriers (the forward phases split no tile and keep the tuned grid; in FP32 the shorter
+// gather gains less than the barriers cost).  FP32: the tuned grid, but never below one block
+// per SM (a forward grid of half the SMs leaves the reverse step short of memory parallelism).
+// Results do not depend on it.
+template <class R>
+int reverse_grid(const da_ctx *ctx, int cap) {
+    int want = ctx->grid;
+    const int per_sm1 = ctx->sm_count > 0 ? ctx->sm_count : 148;
+    if (want < per_sm1) want = per_sm1 < ctx->ntiles ? per_sm1 : ctx->ntiles;
+    if (sizeof(R) == 8 && want < 4 * ctx->ntiles) want = 4 * ctx->ntiles;
+    return want < cap ? want : cap;
+}
+
+// --------------------------------------------------------------------- k_reverse_run
+// Consecutive reverse steps, each from a checkpoint of its own state, in one cooperative launch (most
+// of a binomial schedule: after a chain of forward steps has stored its checkpoints they are taken
+// back one after another).  Per step three phases and barriers -- coefficients, update with the source
+// adjoint, gather -- where a launch per step has a fourth for the restore and a kernel boundary: the
+// next step's checkpoint goes into the state buffer that this step does not read, while its gather
+// runs, and the replayed steps write no state.  A step's chain of phases is latency (a flow of 18 tiles:
+// restore 2, coefficients 5, update 7, gather 6, each barrier 1.2, the launch 4 us), so what counts is
+// how many there are.  Against a launch per step: 200 steps of 37k cells with 16 checkpoints (runs of
+// 5 steps) 10.1 -> 9.6 ms, 512 steps of 1M cells with 32 (runs of 16) 28.3 -> 26.4 ms, 48 steps of 262k
+// cells in FP32 3.31 -> 3.14 ms, 24 steps of 191k wet cells 4.03 -> 3.88 ms.
+//
+// The two state buffers are tracked on their own: dirty[b] the segments of buffer b that may differ
+// from the base checkpoint, wet[b] those with a wet cell (of the base where they do not differ).
+// Afterwards the live dirty flags cover both buffers too, as the restore that follows every run expects.
+constexpr int kRunMax = 32;  // steps of a launch
+
+template <class R>
+struct RunArgs {
+    int n;                         // steps
+    unsigned char *slot[kRunMax];  // their checkpoints (slot[0] null: the live state in buffer cur)
+    size_t array_bytes;            // a slot's layout: three state arrays, the dirty flags, the scalars
+    size_t scalars_at;
+    const R *base[3];              // the base checkpoint
+    uint8_t *dirty[2], *wet[2];    // [nseg]
+    int nseg;
+};
+
+// Checkpoint k of the run into state buffer b (snap_segments' division of the work).
+template <class R>
+__device__ __forceinline__ void run_restore(const RunArgs<R> &ra, int k, int b, const fwd::StatePair<R> &S, int n) {
+    const int lane = threadIdx.x & 31;
+    const int W = (gridDim.x * blockDim.x) >> 5;
+    const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const unsigned char *slot = ra.slot[k];
+    const bool is_base = (const R *)slot == ra.base[0];  // whose cells all hold the base
+    const uint8_t *snap_dirty = slot + 3 * ra.array_bytes;
+    uint8_t *dirty = b ? ra.dirty[1] : ra.dirty[0], *wet = b ? ra.wet[1] : ra.wet[0];
+    R *dst[3] = {b ? S.h[1] : S.h[0], b ? S.hu[1] : S.hu[0], b ? S.hv[1] : S.hv[0]};
+    for (int s0 = 0; s0 < ra.nseg; s0 += 32 * W) {
+        const int s = s0 + lane * W + w;
+        bool flag = false, work = false;
+        if (s < ra.nseg) {
+            flag = !is_base && snap_dirty[s] != 0;
+            work = flag || dirty[s];
+            if (work) dirty[s] = flag;
+        }
+        unsigned bits = __ballot_sync(0xffffffffu, work);
+        const unsigned from = __ballot_sync(0xffffffffu, flag);
+        while (bits) {
+            const int q = __ffs(bits) - 1;
+            bits &= bits - 1;
+            const int seg = s0 + q * W + w, i = seg * 32 + lane;
+            R h = R(0);
+            if (i < n) {
+#pragma unroll
+                for (int v = 0; v < 3; ++v) {
+                    const R x = (from >> q) & 1u ? ((const R *)(slot + v * ra.array_bytes))[i] : ra.base[v][i];
+                    dst[v][i] = x;
+                    if (v == 0) h = x;
+                }
+            }
+            const bool any = __any_sync(0xffffffffu, h >= R(DA_TINY));
+            if (lane == 0) wet[seg] = any;
+        }
+    }
+}
+
+template <class R, int OCC>
+__global__ void __launch_bounds__(kBlock, OCC) k_reverse_run(MeshArgs m, fwd::StatePair<R> S, int cur, R *kact,
+                                                             unsigned *active, uint8_t *seg_wet, uint8_t *seg_dirty,
+                                                             int ntiles, int cull, MatConsts mc, TimeConsts tc,
+                                                             DevScalars *sc, uint8_t *mask, int *tile_epoch,
+                                                             uint8_t *seg_act, int rec_id0, fwd::StatePair<R> L,
+                                                             int lam_in, AdjArgs aa, RunArgs<R> ra, fwd::HaloArgs ha,
+                                                             int gsplit) {
+    __shared__ int list[kBlock];
+    extern __shared__ __align__(16) unsigned char dyn_smem[];
+    fwd::StageSmem<R> &stg = *reinterpret_cast<fwd::StageSmem<R> *>(dyn_smem);
+    const int t0 = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
+    for (int s = t0; s < ra.nseg; s += nt) {
+        const uint8_t d = seg_dirty[s], w = seg_wet[s];
+        ra.dirty[0][s] = ra.dirty[1][s] = d;
+        ra.wet[0][s] = ra.wet[1][s] = w;
+    }
+    // the first step's state: live (its wet flags too), or its checkpoint after a barrier
+    if (ra.slot[0]) {
+        if (!fwd::grid_sync(sc)) return;
+        run_restore<R>(ra, 0, cur, S, m.n);
+        if (!fwd::grid_sync(sc)) return;
+    }
+    for (int k = 0; k < ra.n; ++k) {
+        const int p = (cur + k) & 1, rec_id = rec_id0 + k;
+        const DevScalars *from = ra.slot[k] ? (const DevScalars *)(ra.slot[k] + ra.scalars_at) : sc;
+        const double time = __ldcg(&from->time);
+        const long long iter = __ldcg(&from->iter);
+        const R ftr = fwd::sign_threshold<R>(iter, tc, mc);
+        const StateRef<R> U{S.h[p], S.hu[p], S.hv[p]};
+        const int li = (lam_in + k) & 1;
+        const StateRef<R> Ln{L.h[li], L.hu[li], L.hv[li]};
+        const StateOut<R> Lo{L.h[li ^ 1], L.hu[li ^ 1], L.hv[li ^ 1]};
+        unsigned long long *acc_min = k & 1 ? &sc->acc_alt_min_dxe : &sc->acc_min_dxe;
+        unsigned long long *acc_max = k & 1 ? &sc->acc_alt_hmax : &sc->acc_hmax;
+        // the recording update counts its listed tiles from zero (the adds follow a barrier)
+        if (blockIdx.x == 0 && threadIdx.x == 0) sc->listed = 0u;
+        unsigned long long my_min = 0x7FF0000000000000ull, my_max = 0ull;
+        fwd::coef_phase_staged<R, true>(m, ha, U, kact, active, ra.slot[k] ? ra.wet[p] : seg_wet, ntiles, cull, mc, sc,
+                                        mask, list, my_min, my_max, InstArgs{}, stg, ftr);
+        fwd::push_minmax(my_min, my_max, acc_min, acc_max);
+        if (!fwd::grid_sync(sc)) return;
+        const double min_dxe = __longlong_as_double(__ldcg(acc_min)), hmax = __longlong_as_double(__ldcg(acc_max));
+        double dt, ft;
+        fwd::step_dt(min_dxe, hmax, time, iter, tc, dt, ft);
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            if (!isfinite(dt)) raise_err(sc, DA_ERR_NAN);
+            // the other pair was read by every block before the last step's second barrier
+            *(k & 1 ? &sc->acc_min_dxe : &sc->acc_alt_min_dxe) = fwd::kMinDxeStart;
+            *(k & 1 ? &sc->acc_hmax : &sc->acc_alt_hmax) = 0ull;
+        }
+        const SrcEpilogue<R, false> src{m, Ln, mc, aa, InstArgs{}, R(dt), (const R *)ha.kept};
+        fwd::update_phase_staged<R, true, false, false>(m, ha, U, StateOut<R>{}, kact, active, nullptr, nullptr, nullptr,
+                                                        nullptr, ntiles, cull, mc, sc, R(dt), ftr, mask, tile_epoch,
+                                                        seg_act, rec_id, list, InstArgs{}, stg, src);
+        if (!fwd::grid_sync(sc)) return;
+        gather_staged<R, false>(m, ha, U, Ln, Lo, mc, aa, rec_id, dt, list, InstArgs{}, dyn_smem,
+                                gather_quarters(sc, gsplit));
+        if (k + 1 < ra.n) {
+            run_restore<R>(ra, k + 1, p ^ 1, S, m.n);
+            if (!fwd::grid_sync(sc)) return;
+        } else if (blockIdx.x == 0 && threadIdx.x == 0) {
+            // the last step's scalars, as a launch of its own leaves them
+            sc->iter = iter + 1;
+            sc->frict_tiny = ft;
+            sc->time = time + dt;
+            sc->dt = dt;
+            sc->min_dxe = min_dxe;
+            sc->hmax = hmax;
+            sc->acc_min_dxe = sc->acc_alt_min_dxe = fwd::kMinDxeStart;
+            sc->acc_hmax = sc->acc_alt_hmax = 0ull;
+        }
+    }
+    // Every segment that either buffer or the flags of the live state differ on from the base (the last
+    // restores wrote theirs before a barrier).
+    for (int s = t0; s < ra.nseg; s += nt) seg_dirty[s] |= ra.dirty[0][s] | ra.dirty[1][s];
+    fwd::grid_exit(sc);
+}
+
+// The steps of slots[0..n) (slots[0] may be null: the live state), lambda from buffer lam_in; afterwards
+// it is in lam_in ^ (n & 1) and the state is to be restored.
+template <class R>
+int reverse_run_t(da_ctx *ctx, int lam_in, const double *sec2, double cos_int, void *const *slots, int n) {
+    if (n < 1 || n > kRunMax || ctx->ninst > 0 || !fwd::staged_ok(ctx))
+        return set_error(ctx, DA_ERR_INVALID, "reverse run: not for this context");
+    const int pi = sizeof(R) == 8, occ3 = ctx->p.blocks_per_sm == 3;
+    const void *kern = occ3 ? (const void *)k_reverse_run<R, 3> : (const void *)k_reverse_run<R, 2>;
+    const size_t smem = std::max(fwd::stage_smem_bytes<R>(), gather_staged_bytes<R>());
+    int &cap = ctx->coop_cap_run[pi + 2 * occ3];
+    if (cap <= 0) {
+        int st = cuda_check(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+                            "shared memory attribute");
+        int per_sm = 0;
+        if (!st)
+            st = cuda_check(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kBlock, smem), "occupancy");
+        if (st) return st;
+        cap = per_sm * (ctx->sm_count > 0 ? ctx->sm_count : 1);
+    }
+    if (cap <= 0) return set_error(ctx, DA_ERR_UNSUPPORTED, "reverse-run kernel cannot be resident");
+    const int grid = reverse_grid<R>(ctx, cap);
+    const int rec_id0 = ctx->rec_id + 1;
+    ctx->rec_id += n;
+    MeshArgs m = mesh_args(ctx);
+    fwd::StatePair<R> S, L;
+    for (int b = 0; b < 2; ++b) {
+        S.h[b] = (R *)ctx->U[b][0];
+        S.hu[b] = (R *)ctx->U[b][1];
+        S.hv[b] = (R *)ctx->U[b][2];
+        L.h[b] = (R *)ctx->lam[b][0];
+        L.hu[b] = (R *)ctx->lam[b][1];
+        L.hv[b] = (R *)ctx->lam[b][2];
+    }
+    const snap::SnapArgs<R> sa = snap::snap_args<R>(ctx, ctx->snaps[0], false, ctx->cur);
+    RunArgs<R> ra{};
+    ra.n = n;
+    for (int k = 0; k < n; ++k) ra.slot[k] = (unsigned char *)slots[k];
+    ra.array_bytes = (size_t)((unsigned char *)sa.snap[1] - (unsigned char *)sa.snap[0]);
+    ra.scalars_at = (size_t)((unsigned char *)sa.snap_sc - (unsigned char *)ctx->snaps[0]);
+    for (int v = 0; v < 3; ++v) ra.base[v] = sa.base[v];
+    ra.nseg = ctx->nseg;
+    for (int b = 0; b < 2; ++b) {
+        ra.dirty[b] = ctx->run_flags + (size_t)(2 * b) * ctx->nseg;
+        ra.wet[b] = ctx->run_flags + (size_t)(2 * b + 1) * ctx->nseg;
+    }
+    int cur = ctx->cur, ntiles = ctx->ntiles, cull = ctx->p.tile_culling, rid = rec_id0, li = lam_in;
+    R *kact = (R *)ctx->kact;
+    unsigned *active = ctx->active;
+    uint8_t *seg_wet = ctx->seg_wet, *seg_dirty = ctx->seg_dirty, *mask = ctx->mask, *seg_act = ctx->seg_act;
+    int *tile_epoch = ctx->tile_epoch;
+    MatConsts mc = ctx->mc;
+    TimeConsts tc = ctx->tc;
+    DevScalars *sc = ctx->dsc;
+    AdjArgs aa = adj_args<R>(ctx, sec2, cos_int);
+    fwd::HaloArgs ha = fwd::halo_args(ctx);
+    int gsplit = ctx->p.tile_staging >= 2 ? ctx->p.tile_staging - 1 : 0;
+    void *args[] = {&m,    &S,          &cur,     &kact, &active, &seg_wet, &seg_dirty, &ntiles, &cull, &mc, &tc,
+                    &sc,   &mask,       &tile_epoch, &seg_act, &rid, &L, &li, &aa, &ra, &ha, &gsplit};
+    trace_begin(ctx, TR_YOUTURN);
+    const cudaError_t e = cudaLaunchCooperativeKernel(kern, grid, kBlock, args, smem, ctx->stream);
+    trace_end(ctx, n);
+    return cuda_check(ctx, e, "reverse-run launch");
 }
 
 // The k_youturn instantiation for the launch's flags.
@@ -267,17 +494,7 @@ int youturn_t(da_ctx *ctx, int lam_in, int lam_out, const double *sec2, double c
     }
     const int cap = cap_ref;
     if (cap <= 0) return set_error(ctx, DA_ERR_UNSUPPORTED, "reverse-step kernel cannot be resident");
-    // FP64: every co-resident block, at most four per tile, whatever the forward steps' tuned grid:
-    // the gather spreads a sparse flow's quarter tiles over them, which outweighs the dearer
-    // barriers (the forward phases split no tile and keep the tuned grid; in FP32 the shorter
-    // gather gains less than the barriers cost).  FP32: the tuned grid, but never below one block
-    // per SM (a forward grid of half the SMs leaves the reverse step short of memory parallelism).
-    // Results do not depend on it.
-    int want = ctx->grid;
-    const int per_sm1 = ctx->sm_count > 0 ? ctx->sm_count : 148;
-    if (want < per_sm1) want = per_sm1 < ctx->ntiles ? per_sm1 : ctx->ntiles;
-    if (sizeof(R) == 8 && want < 4 * ctx->ntiles) want = 4 * ctx->ntiles;
-    const int grid = want < cap ? want : cap;
+    const int grid = reverse_grid<R>(ctx, cap);
     ++ctx->rec_id;
     MeshArgs m = mesh_args(ctx);
     fwd::StatePair<R> S;

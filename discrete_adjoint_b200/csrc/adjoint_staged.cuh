@@ -69,12 +69,12 @@ __device__ __forceinline__ void gather_slot(GatherBuf<R> &g, int s, int e, const
 // The byte fields of one slot (plain loads; the branch byte of a cell whose tile the recording
 // step did not list is 0).
 __device__ __forceinline__ void gather_bytes(uint8_t &mk, uint8_t &bf, uint8_t &mat, int e, const MeshArgs &m,
-                                             const AdjArgs &aa) {
+                                             const AdjArgs &aa, int rec_id) {
     const int ep = aa.tile_epoch[e >> 8];
     const uint8_t mv = aa.mask[e];
     bf = m.bflag[e];
     mat = m.mat[e];
-    mk = ep == aa.rec_id ? mv : uint8_t(0);
+    mk = ep == rec_id ? mv : uint8_t(0);
 }
 
 // Tile t and its halo (hc cells of the halo list from hoff) into g; returns with every value in
@@ -83,14 +83,14 @@ __device__ __forceinline__ void gather_bytes(uint8_t &mk, uint8_t &bf, uint8_t &
 template <class R>
 __device__ __forceinline__ void gather_stage(GatherBuf<R> &g, int t, int hoff, int hc, const fwd::HaloArgs &ha,
                                              const MeshArgs &m, const StateRef<R> &U, const StateRef<R> &L,
-                                             const AdjArgs &aa) {
+                                             const AdjArgs &aa, int rec_id) {
     static_assert(kHaloMax <= kTileCells, "one halo cell per thread");
     const int c = threadIdx.x;
     const int i = t * kTileCells + c;
     const bool own = i < m.n;
     const int e = c < hc ? ha.idx[hoff + c] : -1;
     uint8_t mk = 0, bf = 0, mat = 0, hmk = 0, hbf = 0, hmat = 0;
-    if (own) gather_bytes(mk, bf, mat, i, m, aa);
+    if (own) gather_bytes(mk, bf, mat, i, m, aa, rec_id);
     if (own) {
         gather_slot<R>(g, c, i, m, U, L, aa);
         fwd::cp_async<16>(&g.nl[c], ha.nloc + (size_t)i * 8);
@@ -100,7 +100,7 @@ __device__ __forceinline__ void gather_stage(GatherBuf<R> &g, int t, int hoff, i
         fwd::cp_async<8>(&g.gi[c], aa.gint + i);
     }
     if (e >= 0) {
-        gather_bytes(hmk, hbf, hmat, e, m, aa);
+        gather_bytes(hmk, hbf, hmat, e, m, aa, rec_id);
         gather_slot<R>(g, kTileCells + c, e, m, U, L, aa);
     }
     fwd::cp_async_commit();
@@ -213,8 +213,8 @@ template <class R, bool BATCH>
 __device__ __forceinline__ void adj_gather_phase_staged(const MeshArgs &m, const fwd::HaloArgs &ha,
                                                         const StateRef<R> &U, const StateRef<R> &Lnext,
                                                         const StateOut<R> &Lout, const MatConsts &mc0,
-                                                        const AdjArgs &aa, R dt0, int *list, const InstArgs &ia,
-                                                        GatherSmem<R> &S, bool quarter) {
+                                                        const AdjArgs &aa, int rec_id, R dt0, int *list,
+                                                        const InstArgs &ia, GatherSmem<R> &S, bool quarter) {
     GatherBuf<R> &g = S.g;
     const int lane = threadIdx.x & 31;
     const int nunits = quarter ? 4 * aa.ntiles : aa.ntiles;
@@ -229,10 +229,10 @@ __device__ __forceinline__ void adj_gather_phase_staged(const MeshArgs &m, const
                 const size_t o = (size_t)tq * 8 + 2 * (uq & 3);
                 const unsigned sa = *reinterpret_cast<const uint16_t *>(aa.seg_act + o);
                 const unsigned lc = *reinterpret_cast<const uint16_t *>(aa.lam_clean + o);
-                need = (ep == aa.rec_id && sa != 0u) || lc != 0x0101u;
+                need = (ep == rec_id && sa != 0u) || lc != 0x0101u;
             } else {
                 const unsigned long long sa = seg_flags8(aa.seg_act, tq), lc = seg_flags8(aa.lam_clean, tq);
-                need = (ep == aa.rec_id && sa != 0ull) || lc != 0x0101010101010101ull;
+                need = (ep == rec_id && sa != 0ull) || lc != 0x0101010101010101ull;
             }
         }
         int ho, hc;
@@ -241,7 +241,7 @@ __device__ __forceinline__ void adj_gather_phase_staged(const MeshArgs &m, const
         for (int q = 0; q < cnt; ++q) {
             const int u = list[q];
             const int t = quarter ? u >> 2 : u;
-            gather_stage<R>(g, t, S.hoff[q], S.hcnt[q], ha, m, U, Lnext, aa);
+            gather_stage<R>(g, t, S.hoff[q], S.hcnt[q], ha, m, U, Lnext, aa, rec_id);
             const int inst = BATCH ? ia.tile_inst[t] : 0;
             const MatConsts &mc = BATCH ? ia.mcs[inst] : mc0;
             const R dt = BATCH ? R(ia.dt[inst]) : dt0;

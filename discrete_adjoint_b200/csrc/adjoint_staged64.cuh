@@ -57,7 +57,7 @@ __device__ __forceinline__ void gather_slot64(GatherBuf64 &g, int s, int e, cons
 // and halo cell c.
 __device__ __forceinline__ bool gather_stage64(GatherBuf64 &g, int t, int hoff, int hc, const fwd::HaloArgs &ha,
                                                const MeshArgs &m, const StateRef<double> &U, const StateRef<double> &L,
-                                               const AdjArgs &aa, double dt) {
+                                               const AdjArgs &aa, int rec_id, double dt) {
     static_assert(kHaloMax <= kTileCells, "one halo cell per thread");
     const int c = threadIdx.x;
     const int i = t * kTileCells + c;
@@ -66,7 +66,7 @@ __device__ __forceinline__ bool gather_stage64(GatherBuf64 &g, int t, int hoff, 
     const double *kept = (const double *)ha.kept;
     uint8_t mk = 0, bf = 0, mat = 0, hmk = 0, hbf = 0, hmat = 0;
     if (own) {
-        gather_bytes(mk, bf, mat, i, m, aa);
+        gather_bytes(mk, bf, mat, i, m, aa, rec_id);
         gather_slot64(g, c, i, m, U, L, aa, kept);
         fwd::cp_async<16>(&g.nl[c], ha.nloc + (size_t)i * 8);
 #pragma unroll
@@ -75,7 +75,7 @@ __device__ __forceinline__ bool gather_stage64(GatherBuf64 &g, int t, int hoff, 
         fwd::cp_async<8>(&g.gi[c], aa.gint + i);
     }
     if (e >= 0) {
-        gather_bytes(hmk, hbf, hmat, e, m, aa);
+        gather_bytes(hmk, hbf, hmat, e, m, aa, rec_id);
         gather_slot64(g, kTileCells + c, e, m, U, L, aa, kept);
     }
     fwd::cp_async_commit();
@@ -177,8 +177,8 @@ __device__ __forceinline__ void gather_face64(const GatherBuf64 &g, const MatCon
 template <bool BATCH>
 __device__ __forceinline__ void adj_gather_phase64(const MeshArgs &m, const fwd::HaloArgs &ha, const StateRef<double> &U,
                                                    const StateRef<double> &Lnext, const StateOut<double> &Lout,
-                                                   const MatConsts &mc0, const AdjArgs &aa, double dt0, int *list,
-                                                   const InstArgs &ia, GatherSmem64 &S, bool quarter) {
+                                                   const MatConsts &mc0, const AdjArgs &aa, int rec_id, double dt0,
+                                                   int *list, const InstArgs &ia, GatherSmem64 &S, bool quarter) {
     const GatherBuf64 &g = S.g;
     const int lane = threadIdx.x & 31, s = lane & 3;
     const int nunits = quarter ? 4 * aa.ntiles : aa.ntiles;
@@ -193,10 +193,10 @@ __device__ __forceinline__ void adj_gather_phase64(const MeshArgs &m, const fwd:
                 const size_t o = (size_t)tq * 8 + 2 * (uq & 3);
                 const unsigned sa = *reinterpret_cast<const uint16_t *>(aa.seg_act + o);
                 const unsigned lc = *reinterpret_cast<const uint16_t *>(aa.lam_clean + o);
-                need = (ep == aa.rec_id && sa != 0u) || lc != 0x0101u;
+                need = (ep == rec_id && sa != 0u) || lc != 0x0101u;
             } else {
                 const unsigned long long sa = seg_flags8(aa.seg_act, tq), lc = seg_flags8(aa.lam_clean, tq);
-                need = (ep == aa.rec_id && sa != 0ull) || lc != 0x0101010101010101ull;
+                need = (ep == rec_id && sa != 0ull) || lc != 0x0101010101010101ull;
             }
         }
         int ho, hc;
@@ -208,11 +208,11 @@ __device__ __forceinline__ void adj_gather_phase64(const MeshArgs &m, const fwd:
             const int inst = BATCH ? ia.tile_inst[t] : 0;
             const MatConsts &mc = BATCH ? ia.mcs[inst] : mc0;
             const double dt = BATCH ? ia.dt[inst] : dt0;
-            const bool fast = gather_stage64(S.g, t, S.hoff[q], S.hcnt[q], ha, m, U, Lnext, aa, dt);
+            const bool fast = gather_stage64(S.g, t, S.hoff[q], S.hcnt[q], ha, m, U, Lnext, aa, rec_id, dt);
             // a recorded tile's segment activity is the OR of its cells' active bits
             if (threadIdx.x < (quarter ? 2 : 8)) {
                 const int seg = t * 8 + (quarter ? 2 * (u & 3) : 0) + (int)threadIdx.x;
-                aa.lam_clean[seg] = aa.tile_epoch[t] == aa.rec_id && aa.seg_act[seg] ? 0 : 1;
+                aa.lam_clean[seg] = aa.tile_epoch[t] == rec_id && aa.seg_act[seg] ? 0 : 1;
             }
             const int c = quarter ? (u & 3) * 64 + ((int)threadIdx.x >> 2) : (int)threadIdx.x;
             const int j = t * kTileCells + c;

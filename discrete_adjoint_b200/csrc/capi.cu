@@ -178,7 +178,7 @@ static void free_state(da_ctx *ctx) {
 
 static void free_adjoint(da_ctx *ctx) {
     auto fr = [](void *p) { if (p) cudaFree(p); };
-    fr(ctx->mask); fr(ctx->adjA); fr(ctx->adjB); fr(ctx->gbed); fr(ctx->gint); fr(ctx->dk_tab);
+    fr(ctx->mask); fr(ctx->run_flags); fr(ctx->adjA); fr(ctx->adjB); fr(ctx->gbed); fr(ctx->gint); fr(ctx->dk_tab);
     fr(ctx->red_out); fr(ctx->red_part); fr(ctx->inst_J); fr(ctx->seg_J); fr(ctx->dh0);
     for (int b = 0; b < 2; ++b)
         for (int v = 0; v < 3; ++v) { fr(ctx->lam[b][v]); ctx->lam[b][v] = nullptr; }
@@ -187,7 +187,7 @@ static void free_adjoint(da_ctx *ctx) {
     if (ctx->sweep_graph) cudaGraphExecDestroy(ctx->sweep_graph);
     ctx->sweep_graph = nullptr;
     ctx->sweep_key.clear();
-    ctx->mask = nullptr; ctx->adjA = ctx->adjB = ctx->gbed = ctx->gint = ctx->dk_tab = nullptr;
+    ctx->mask = ctx->run_flags = nullptr; ctx->adjA = ctx->adjB = ctx->gbed = ctx->gint = ctx->dk_tab = nullptr;
     ctx->red_out = ctx->red_part = ctx->inst_J = ctx->seg_J = ctx->dh0 = nullptr;
     ctx->dh0_bytes = 0;
     fr(ctx->refadj_mem);

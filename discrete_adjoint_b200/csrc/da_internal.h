@@ -216,6 +216,7 @@ struct da_ctx {
     int coop_cap[32] = {};
     // of k_youturn [FP32, FP64] x [single, ensemble] x [seed] x [2, 3 per SM] x [staged]
     int coop_cap_yt[32] = {};
+    int coop_cap_run[4] = {};        // of k_reverse_run [FP32, FP64] x [2, 3 per SM]
     int sm_count = 0;
     da::DevScalars *dsc = nullptr;   // device scalars
     da::DevScalars *hsc = nullptr;   // pinned host mirror
@@ -227,6 +228,7 @@ struct da_ctx {
     // adjoint workspace (allocated on first use)
     uint8_t *mask = nullptr;         // [n] branch codes of the replayed forward step
     void *lam[2][3] = {{nullptr, nullptr, nullptr}, {nullptr, nullptr, nullptr}};
+    uint8_t *run_flags = nullptr;    // [4][nseg] dirty and wet flags of the two state buffers in a reverse run
     double *adjA = nullptr;          // [3][n]
     double *adjB = nullptr;          // [4][n]
     double *gbed = nullptr, *gint = nullptr;  // [n] running parameter sensitivities

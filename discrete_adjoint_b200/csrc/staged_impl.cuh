@@ -659,7 +659,9 @@ struct NoEpilogue {
 // signs f (the reverse step's source adjoint, which needs exactly these), with the staged view v
 // of the cell (slot c), its U^n, boundary flags, recorded branch byte, g_z and source coefficients,
 // and what epi.pre(i, wet) loaded before the update (so that those loads overlap it).
-template <class R, bool RECORD, bool BATCH = false, class Epi = NoEpilogue>
+// STATE false: a reverse step whose new state nobody reads -- the state, the segments' volumes and their
+// wet, clean and dirty flags are left alone, and only active tiles are listed.
+template <class R, bool RECORD, bool BATCH = false, bool STATE = true, class Epi = NoEpilogue>
 __device__ __forceinline__ void update_phase_staged(const MeshArgs &m, const HaloArgs &ha, const StateRef<R> &U,
                                                     const StateOut<R> &O, const R *kact, unsigned *active,
                                                     uint8_t *seg_clean, uint8_t *seg_wet, double *seg_vol,
@@ -673,7 +675,7 @@ __device__ __forceinline__ void update_phase_staged(const MeshArgs &m, const Hal
         bool need = false;
         if (tq < ntiles) {
             // the clean flags and the bitmask words of the tile, loaded together
-            const unsigned long long cf = seg_flags(seg_clean, tq);
+            const unsigned long long cf = STATE ? seg_flags(seg_clean, tq) : kAllSegs;
             const uint4 *w4 = reinterpret_cast<const uint4 *>(active + (size_t)tq * (kTileCells / 32));
             const uint4 a = w4[0], b = w4[1];
             need = !cull || cf != kAllSegs || (a.x | a.y | a.z | a.w | b.x | b.y | b.z | b.w) != 0u;
@@ -754,21 +756,25 @@ __device__ __forceinline__ void update_phase_staged(const MeshArgs &m, const Hal
                 const uint8_t code = RECORD ? uint8_t(kcode | (act ? 8 : 0) | (clamped ? 4 : 0)) : 0;
                 if (RECORD) mask[i] = code;
                 if (!isfinite(st[0]) || !isfinite(st[1]) || !isfinite(st[2])) raise_err(sc, DA_ERR_NAN);
-                O.h[i] = st[0];
-                O.hu[i] = st[1];
-                O.hv[i] = st[2];
+                if (STATE) {
+                    O.h[i] = st[0];
+                    O.hu[i] = st[1];
+                    O.hv[i] = st[2];
+                }
                 vol = double(dxc) * double(dyc) * double(st[0]);
                 wet_after = st[0] >= R(DA_TINY);
             }
             const unsigned wet_bits = __ballot_sync(0xffffffffu, wet_after);
             const unsigned act_bits = __ballot_sync(0xffffffffu, act);
-            vol = warp_sum(vol);
+            if (STATE) vol = warp_sum(vol);
             if (lane == 0) {
                 if (word) active[seg] = 0u;
-                if (act_bits) seg_dirty[seg] = 1;  // changed since the base checkpoint
-                seg_vol[seg] = vol;
-                seg_clean[seg] = act_bits ? 0 : 1;
-                seg_wet[seg] = wet_bits ? 1 : 0;
+                if (STATE) {
+                    if (act_bits) seg_dirty[seg] = 1;  // changed since the base checkpoint
+                    seg_vol[seg] = vol;
+                    seg_clean[seg] = act_bits ? 0 : 1;
+                    seg_wet[seg] = wet_bits ? 1 : 0;
+                }
                 if (RECORD) seg_act[seg] = act_bits ? 1 : 0;
             }
             if (RECORD && threadIdx.x == 0) tile_epoch[t] = rec_id;

@@ -280,3 +280,32 @@ def test_fp32_split_adjoint_close_to_fp64():
     lam_err = np.linalg.norm(b.lambda0 - a.lambda0) / np.linalg.norm(a.lambda0)
     print("fp32-split gradient rel errors", errs, "lambda0", lam_err, "J", rel(b.J, a.J))
     assert max(errs) < 1e-4 and lam_err < 1e-4
+
+
+@pytest.mark.parametrize("precision", [_ffi.DA_PREC_FP64, _ffi.DA_PREC_FP32_SPLIT])
+@pytest.mark.parametrize("nsteps,snaps,culling,per_sm", [(70, 80, 1, 2), (33, 33, 0, 2), (34, 5, 1, 3), (2, 1, 1, 2),
+                                                         (1, 4, 1, 2)])
+def test_reverse_runs_match_single_reverse_steps(precision, nsteps, snaps, culling, per_sm):
+    # consecutive reverse steps in one launch (lists longer than a launch takes, a checkpoint for
+    # every step, runs of one) against one launch per step: lambda^0, gradients, the state put back
+    # and the steps after it bit for bit
+    w = inputs.test_case(seed=5)
+    m = w.mesh
+    out = []
+    for staging in (0, 1):
+        with GeoflowContext(w.mat, TimeProps(), precision=precision, tile_staging=staging, tile_culling=culling,
+                            blocks_per_sm=per_sm) as c:
+            c.upload_mesh(m)
+            c.set_state(m.h0, m.hu0, m.hv0)
+            c.run(3)
+            got = [adjoint_run(c, box_of(w), nsteps, snaps, m.dh0_dpile, want_lambda0=True) for _ in range(2)]
+            back = np.stack(c.get_state())
+            st = c.run(5)
+            out.append((got, back, np.stack(c.get_state()), st.time, st.volume))
+    (ga, *ra), (gb, *rb) = out
+    for a, b in zip(ga, gb):
+        assert np.array_equal(a.lambda0, b.lambda0)
+        assert a.J == b.J and a.dJ_dintfrict == b.dJ_dintfrict and a.forward_steps == b.forward_steps
+        assert np.array_equal(a.dJ_dbedfrict, b.dJ_dbedfrict) and np.array_equal(a.dJ_dpile, b.dJ_dpile)
+    for a, b in zip(ra, rb):
+        assert np.array_equal(a, b)
