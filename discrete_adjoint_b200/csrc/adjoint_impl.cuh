@@ -57,62 +57,6 @@ __device__ __forceinline__ void lam_eff(const StateRef<R> &L, uint8_t mk, int i,
 }
 
 
-// Derivative data of the limited depth slope in one direction (Element::get_slopes for j = 0):
-// slope = fac * min(gamma|dp|, gamma|dm|, |dc|); g_dp, g_dm = d slope / d dp, d dm.
-template <class R>
-struct SlopeD {
-    R g_dp, g_dm, dxp, dxm;
-};
-
-// v: where the depths, neighbours and centres / sizes come from (global arrays, or a tile staged
-// in shared memory with i the cell's slot); the arithmetic is the same either way.
-template <class R, class V>
-__device__ __forceinline__ void h_slope_deriv(const V &v, int i, uint8_t bf, R gamma, R hi, SlopeD<R> out[2]) {
-#pragma unroll
-    for (int dir = 0; dir < 2; ++dir) {
-        const int ep = v.nb(dir, i);
-        const int em = v.nb(dir + 2, i);
-        const bool two_p = bf & (0x10 << dir), two_m = bf & (0x10 << (dir + 2));
-        R dxp, dxm, dp, dm;
-        if constexpr (sizeof(R) == 8) {
-            const double ci = v.coord(dir, i);
-            dxp = v.coord(dir, ep) - ci;
-            dxm = ci - v.coord(dir, em);
-            dp = (v.h(ep) - hi) / dxp;
-            if (two_p) dp = .5 * (dp + (v.h(v.nb(dir + 4, i)) - hi) / dxp);
-            dm = (hi - v.h(em)) / dxm;
-            if (two_m) dm = .5 * (dm + (hi - v.h(v.nb(dir + 6, i))) / dxm);
-        } else {
-            const float si = v.size(dir, i);
-            dxp = 0.5f * (v.size(dir, ep) + si);
-            dxm = 0.5f * (v.size(dir, em) + si);
-            const float ip = 1.0f / dxp, im = 1.0f / dxm;
-            dp = (v.h(ep) - hi) * ip;
-            if (two_p) dp = 0.5f * (dp + (v.h(v.nb(dir + 4, i)) - hi) * ip);
-            dm = (hi - v.h(em)) * im;
-            if (two_m) dm = 0.5f * (dm + (hi - v.h(v.nb(dir + 6, i))) * im);
-        }
-        const R dc = (dp * dxm + dm * dxp) / (dxm + dxp);
-        const R fac = R(.5) * (c_sgn(dp) + c_sgn(dm));
-        const R a = gamma * dabs(dp), b = gamma * dabs(dm), c = dabs(dc);
-        // selection order of c_dmin1(a, b, c) (geoflow.h:112-120)
-        int sel = 0;
-        R mn = a;
-        if (mn > b) { mn = b; sel = 1; }
-        if (mn > c) { mn = c; sel = 2; }
-        const auto sgnf = [](R v) { return v > R(0) ? R(1) : (v < R(0) ? R(-1) : R(0)); };
-        R gdp = 0, gdm = 0;
-        if (sel == 0) gdp = fac * gamma * sgnf(dp);
-        else if (sel == 1) gdm = fac * gamma * sgnf(dm);
-        else {
-            const R gc = fac * sgnf(dc) / (dxm + dxp);
-            gdp = gc * dxm;
-            gdm = gc * dxp;
-        }
-        out[dir] = SlopeD<R>{gdp, gdm, dxp, dxm};
-    }
-}
-
 // Forward pieces of one side's Riemann flux with what the reverse sweep needs.
 template <class R>
 struct Side {
@@ -310,18 +254,6 @@ __device__ __forceinline__ SrcFwd<R> src_fwd(const V &v, int vi, uint8_t bf, con
     f.sg1 = tiny_sgn(f.h_inv * (f.s[2] - f.vel1 * f.s[0]), ft);
     f.sg3 = tiny_sgn(f.vel1, ft);
     return f;
-}
-
-// d (depth slope) / d h at the neighbour across each side: the slope's derivative by dp or dm over
-// the centre distance.
-template <class R, class V>
-__device__ __forceinline__ void slope_quotients(const V &v, int vi, uint8_t bf, R gamma, R h, R q[4]) {
-    SlopeD<R> sd[2];
-    h_slope_deriv<R>(v, vi, bf, gamma, h, sd);
-    q[0] = sd[0].g_dp / sd[0].dxp;
-    q[2] = sd[0].g_dm / sd[0].dxm;
-    q[1] = sd[1].g_dp / sd[1].dxp;
-    q[3] = sd[1].g_dm / sd[1].dxm;
 }
 
 // get_f() gives the forward's quantities of the cell (computed, or handed over by the update), get_q(q)

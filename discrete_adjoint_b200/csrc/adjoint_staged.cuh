@@ -318,7 +318,7 @@ __device__ __forceinline__ void adj_gather_phase_staged(const MeshArgs &m, const
 }
 
 // The reverse step's source adjoint inside its staged update phase: lambda^{n+1} of a wet cell is
-// loaded before its update (FP64: with the slope derivatives the coefficient phase left), the slopes,
+// loaded before its update with the slope derivatives the coefficient phase left, the slopes,
 // velocities and friction signs are the update's own, the rest comes from the update's staged tile.
 template <class R, bool BATCH>
 struct SrcEpilogue {
@@ -331,7 +331,7 @@ struct SrcEpilogue {
     const R *kept;  // HaloArgs::kept
     struct Pre {
         R l[3];
-        R q[sizeof(R) == 8 ? 4 : 1];  // FP64: the slope derivatives the recording coefficient phase left
+        R q[4];  // the slope derivatives the recording coefficient phase left
     };
     __device__ __forceinline__ Pre pre(int i, bool wet) const {
         Pre p{};
@@ -339,9 +339,8 @@ struct SrcEpilogue {
             p.l[0] = Ln.h[i];
             p.l[1] = Ln.hu[i];
             p.l[2] = Ln.hv[i];
-            if constexpr (sizeof(R) == 8)
 #pragma unroll
-                for (int s = 0; s < 4; ++s) p.q[s] = kept[(size_t)(5 + s) * m.n + i];
+            for (int s = 0; s < 4; ++s) p.q[s] = kept[(size_t)(5 + s) * m.n + i];
         }
         return p;
     }
@@ -355,11 +354,8 @@ struct SrcEpilogue {
         adj_src_wet<R>(m, prev, gz, code, bf, p.l, cs, mci, aa, inst_tables<BATCH>(aa, ia, inst), dti, i,
                        [&]() -> const SrcFwd<R> & { return f; },
                        [&](R q[4]) {
-                           if constexpr (sizeof(R) == 8)
 #pragma unroll
-                               for (int s = 0; s < 4; ++s) q[s] = p.q[s];
-                           else
-                               slope_quotients<R>(v, c, bf, R(mci.gamma), prev[0], q);
+                           for (int s = 0; s < 4; ++s) q[s] = p.q[s];
                        });
     }
 };

@@ -97,7 +97,7 @@ __device__ __forceinline__ bool gather_stage64(GatherBuf64 &g, int t, int hoff, 
 
 template <bool FAST>
 struct QuotPolicy {
-    static __device__ __forceinline__ double div(double a, double b) { return fwd::Divisor<FAST>(b)(a); }
+    static __device__ __forceinline__ double div(double a, double b) { return fwd::Divisor<double, FAST>(b)(a); }
 };
 
 // A side of a face from the staged values (make_side).

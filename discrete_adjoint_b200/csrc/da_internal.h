@@ -174,10 +174,9 @@ struct da_ctx {
     int cur = 0;
     void *kact = nullptr;            // [n] Real
     // what the staged coefficient phase keeps of each wet cell for the update phase (staged_impl.cuh):
-    // FP64 [9][n] (depth slopes, velocities, wave speed, the depth slopes' derivatives) and the friction
-    // signs, FP32 [4][n] (slopes)
+    // [9][n] (depth slopes, velocities, wave speed, the depth slopes' derivatives) and the friction signs
     void *slopes = nullptr;
-    uint8_t *fsign = nullptr;        // [n] FP64 only
+    uint8_t *fsign = nullptr;        // [n] friction signs
     // segments: 32 consecutive cells (one warp), 8 per tile; arrays padded to whole tiles
     int nseg = 0;                    // ntiles * 8
     double *seg_vol = nullptr;       // [nseg] volume partial of each segment after its last update

@@ -10,19 +10,21 @@
 // identical; only where the operands come from changes.  Each cell's neighbour entries come from
 // the host-built table of tile-local slots (one 16-byte load per cell).
 //
-// FP64: what both phases need of a wet cell and of its wet neighbours is formed once per cell, in the
+// What both phases need of a wet cell and of its wet neighbours is formed once per cell, in the
 // coefficient phase: the velocities hu / h and hv / h and the flux's wave speed sqrt(k h g_z) go to
 // global memory, are staged with the tile, and replace k act/pass and g_z there, so the four side
 // fluxes of a cell take no division and no square root besides the HLL quotients; the four friction
-// signs (a byte) and the two depth slopes are all that the sources take from the slopes.  Quotients
-// that share a divisor are formed branch-free (quot.cuh) as long as every staged state is ordinary
+// signs (a byte) and the two depth slopes are all that the sources take from the slopes.
+// FP64 quotients that share a divisor are formed branch-free (quot.cuh) as long as every staged state is ordinary
 // there (tested as the copies land, folded into the tile's barrier); a tile with any other value, and
 // a mesh or material outside the range, takes the division operator.  The results are the
-// reference's bits either way.  Bound: not memory (740k wet cells: a third of HBM's rate) but the
+// reference's bits either way (FP32: the unstaged phases' bits).  Bound: not memory (740k wet cells: a third of HBM's rate) but the
 // instructions and the latency of one warp's FP64 chain.  46 divisions and 6 square roots per cell and
 // step became 13 divisors and 2 square roots: 2894 -> 2050 instructions per warp and step, 125 -> 95 us
 // per step on 740k wet cells (2 x 296 blocks), 14.0 -> 10.7 us on a flow of 18 tiles.  Three blocks
-// per SM with one buffer each (80 registers) took 100 us.
+// per SM with one buffer each (80 registers) took 100 us.  FP32 (approximate quotients): 1650 -> 1380
+// instructions, 137 -> 133 us on 2.1M wet cells (2 x 296 blocks), a flow on 262k cells 15.4 -> 13.9 us per
+// step and 26.2 -> 25.0 us per reverse step.
 //
 // Activity: a cell is updated when it or a face neighbour is wet.  The global path marks every
 // neighbour of a wet cell in the active bitmask with atomics; here the update phase recomputes
@@ -43,16 +45,16 @@ struct StageBuf {
     // the tile's own cells
     uint4 nl[kTileCells];                      // neighbour slots (8 x int16)
     uint8_t bf[kTileCells], mat[kTileCells];   // boundary flags, material
-    R sz[2][sizeof(R) == 8 ? kTileCells : 1];  // FP64: dx, dy (FP32: c0, c1 below)
+    R sz[2][kTileCells];                       // dx, dy (FP32: in the update phase)
     R src[6][kTileCells];                      // update phase: g_x, g_y, the gravity derivatives, curvatures
     // every slot
     R h[kSlots], hu[kSlots], hv[kSlots];
-    R c0[kSlots];  // FP64: x centre (coefficient phase), hu / h of wet cells (update phase); FP32: dx
-    R c1[kSlots];  // FP64: y centre, hv / h; FP32: dy
-    R a[sizeof(R) == 8 ? kSlots : 1];  // FP64: wave speed of wet cells (update phase)
-    // FP64: the tile's own cells only
-    R k[sizeof(R) == 8 ? kTileCells : kSlots];   // k act/pass (update phase)
-    R gz[sizeof(R) == 8 ? kTileCells : kSlots];  // g_z
+    R c0[kSlots];  // coefficient phase: x centre (FP32: dx); update phase: hu / h of wet cells
+    R c1[kSlots];  // y centre (FP32: dy); hv / h
+    R a[kSlots];   // wave speed of wet cells (update phase)
+    // the tile's own cells
+    R k[kTileCells];   // k act/pass (update phase)
+    R gz[kTileCells];  // g_z
 };
 
 template <class R>
@@ -73,10 +75,9 @@ struct HaloArgs {
     const int32_t *idx;   // halo cells, tile after tile
     const int16_t *nloc;  // [n][8] tile-local neighbour slots
     // written by the coefficient phase for each wet cell and read by the same step's update phase:
-    void *kept;           // FP64 [5][n]: d h / dx, d h / dy, hu / h, hv / h, sqrt(k h g_z), and when recording
-                          // [4][n] more, the derivatives of d h / dx and d h / dy by the neighbours' depths;
-                          // FP32 [4][n]: the limited slopes d h / dx, d hv / dx, d h / dy, d hu / dy
-    uint8_t *fsign;       // FP64 [n]: the four friction signs of the sources, two bits each (sign + 1)
+    void *kept;           // [5][n]: d h / dx, d h / dy, hu / h, hv / h, sqrt(k h g_z), and when recording
+                          // [4][n] more, the derivatives of d h / dx and d h / dy by the neighbours' depths
+    uint8_t *fsign;       // [n]: the four friction signs of the sources, two bits each (sign + 1)
     int fast;             // FP64: the mesh and the materials allow quot.cuh's quotients
 };
 
@@ -109,8 +110,6 @@ struct StagedView {
     __device__ __forceinline__ R h(int e) const { return b.h[e]; }
     __device__ __forceinline__ R hu(int e) const { return b.hu[e]; }
     __device__ __forceinline__ R hv(int e) const { return b.hv[e]; }
-    __device__ __forceinline__ R k(int e) const { return b.k[e]; }
-    __device__ __forceinline__ R gz(int e) const { return b.gz[e]; }
     __device__ __forceinline__ double coord(int dir, int e) const { return double(dir == 0 ? b.c0[e] : b.c1[e]); }
     __device__ __forceinline__ float size(int dir, int e) const { return float(dir == 0 ? b.c0[e] : b.c1[e]); }
 };
@@ -126,9 +125,9 @@ __device__ __forceinline__ void load_slots(const int16_t *nloc, int i, int nl[8]
     }
 }
 
-// Copies of one slot's values.  UPD: also what the update phase reads at neighbours (FP64: the
-// velocities and the wave speed, at the cell itself k act/pass and g_z; FP32: k act/pass and g_z).
-// The coefficient phase reads the centres instead (FP64).
+// Copies of one slot's values.  UPD: also what the update phase reads at neighbours (the velocities and
+// the wave speed, at the cell itself k act/pass and g_z).  The coefficient phase reads the centres (FP32:
+// the sizes) instead.
 template <class R, bool UPD>
 __device__ __forceinline__ void stage_slot(StageBuf<R> &b, int s, int e, bool own, const MeshArgs &m,
                                            const StateRef<R> &U, const R *kact, const HaloArgs &ha) {
@@ -136,27 +135,20 @@ __device__ __forceinline__ void stage_slot(StageBuf<R> &b, int s, int e, bool ow
     cp_async<B>(&b.h[s], U.h + e);
     cp_async<B>(&b.hu[s], U.hu + e);
     cp_async<B>(&b.hv[s], U.hv + e);
-    if constexpr (sizeof(R) == 8) {
-        if (own) cp_async<B>(&b.gz[s], m.g + (size_t)2 * m.n + e);
-        if (UPD) {
-            const R *kept = (const R *)ha.kept;
-            if (own) cp_async<B>(&b.k[s], kact + e);
-            cp_async<B>(&b.c0[s], kept + (size_t)2 * m.n + e);
-            cp_async<B>(&b.c1[s], kept + (size_t)3 * m.n + e);
-            cp_async<B>(&b.a[s], kept + (size_t)4 * m.n + e);
-        } else {
-            cp_async<B>(&b.c0[s], m.x + e);
-            cp_async<B>(&b.c1[s], m.y + e);
-        }
+    if (own) cp_async<B>(&b.gz[s], (sizeof(R) == 8 ? (const R *)m.g : (const R *)m.fg) + (size_t)2 * m.n + e);
+    if (UPD) {
+        const R *kept = (const R *)ha.kept;
+        if (own) cp_async<B>(&b.k[s], kact + e);
+        cp_async<B>(&b.c0[s], kept + (size_t)2 * m.n + e);
+        cp_async<B>(&b.c1[s], kept + (size_t)3 * m.n + e);
+        cp_async<B>(&b.a[s], kept + (size_t)4 * m.n + e);
     } else {
-        if (UPD) cp_async<B>(&b.k[s], kact + e);
-        if (UPD || own) cp_async<B>(&b.gz[s], m.fg + (size_t)2 * m.n + e);
-        cp_async<B>(&b.c0[s], m.fdx + e);
-        cp_async<B>(&b.c1[s], m.fdy + e);
+        cp_async<B>(&b.c0[s], sizeof(R) == 8 ? (const R *)m.x + e : (const R *)m.fdx + e);
+        cp_async<B>(&b.c1[s], sizeof(R) == 8 ? (const R *)m.y + e : (const R *)m.fdy + e);
     }
 }
 
-// What only the tile's own cells need: neighbour slots, sizes (FP64), source coefficients (UPD),
+// What only the tile's own cells need: neighbour slots, sizes, source coefficients (UPD),
 // and the tile's flag and material bytes in 16-byte pieces (the byte arrays are padded to tiles).
 template <class R, bool UPD>
 __device__ __forceinline__ void stage_own(StageBuf<R> &b, int t, const MeshArgs &m, const int16_t *nloc) {
@@ -165,9 +157,9 @@ __device__ __forceinline__ void stage_own(StageBuf<R> &b, int t, const MeshArgs 
     const int i = t * kTileCells + c;
     if (i < m.n) {
         cp_async<16>(&b.nl[c], nloc + (size_t)i * 8);
-        if constexpr (sizeof(R) == 8) {
-            cp_async<8>(&b.sz[0][c], m.dx + i);
-            cp_async<8>(&b.sz[1][c], m.dy + i);
+        if (sizeof(R) == 8 || UPD) {
+            cp_async<B>(&b.sz[0][c], sizeof(R) == 8 ? (const R *)m.dx + i : (const R *)m.fdx + i);
+            cp_async<B>(&b.sz[1][c], sizeof(R) == 8 ? (const R *)m.dy + i : (const R *)m.fdy + i);
         }
         if (UPD) {
             const R *g = sizeof(R) == 8 ? (const R *)m.g : (const R *)m.fg;
@@ -293,8 +285,8 @@ __device__ __forceinline__ void staged_tiles(const MeshArgs &m, const HaloArgs &
 // The cold path's division, out of line (the kernels stay small).
 __device__ __noinline__ double div_operator(double a, double b) { return a / b; }
 
-// A divisor and its quotients: FAST by quot.cuh, else the operator.
-template <bool FAST>
+// A divisor and its quotients.  FP64: FAST by quot.cuh, else the operator; FP32: its inverse.
+template <class R, bool FAST>
 struct Divisor {
     quot::Recip r;
     __device__ __forceinline__ explicit Divisor(double b) {
@@ -309,6 +301,12 @@ struct Divisor {
         else
             return div_operator(a, r.b);
     }
+};
+template <bool FAST>
+struct Divisor<float, FAST> {
+    float y;
+    __device__ __forceinline__ explicit Divisor(float b) : y(1.0f / b) {}
+    __device__ __forceinline__ float operator()(float a) const { return a * y; }
 };
 
 // cell_slopes (fv_device.cuh, FP64) with one divisor per centre distance.  DERIV: also the derivatives
@@ -329,7 +327,7 @@ __device__ __forceinline__ void staged_slopes64(const StagedView<double> &v, int
         const bool two_p = bf & (0x10 << dir), two_m = bf & (0x10 << (dir + 2));
         const double ci = v.coord(dir, i);
         const double dxp = v.coord(dir, ep) - ci, dxm = ci - v.coord(dir, em);
-        const Divisor<FAST> dvp(dxp), dvm(dxm), dvs(dxm + dxp);
+        const Divisor<double, FAST> dvp(dxp), dvm(dxm), dvs(dxm + dxp);
         const double up[3] = {v.h(ep), v.hu(ep), v.hv(ep)}, um[3] = {v.h(em), v.hu(em), v.hv(em)};
         double dp[3], dm[3];
 #pragma unroll
@@ -371,25 +369,32 @@ __device__ __forceinline__ void staged_slopes64(const StagedView<double> &v, int
     }
 }
 
-// What the coefficient phase forms of a wet cell (FP64).
-struct Coef64 {
-    double s[6];        // limited slopes
-    double vx, vy, a;   // hu / h, hv / h, sqrt(k h g_z)
-    double k, ev;       // k act/pass, largest wave speed
-    uint8_t code;       // branch of k act/pass
-    uint8_t sgn;        // friction signs, two bits each
-    double q[4];        // recording: derivatives of the depth slopes by the neighbours' depths
+// What the coefficient phase forms of a wet cell.
+template <class R>
+struct StagedCoef {
+    R s[6];        // limited slopes
+    R vx, vy, a;   // hu / h, hv / h, sqrt(k h g_z)
+    R k, ev;       // k act/pass, largest wave speed
+    uint8_t code;  // branch of k act/pass
+    uint8_t sgn;   // friction signs, two bits each
+    R q[4];        // recording: derivatives of the depth slopes by the neighbours' depths
 };
+
+// The four friction signs (-1, 0 or 1) in two bits each.
+__device__ __forceinline__ uint8_t pack_signs(int s0, int s1, int s2, int s3) {
+    return uint8_t((s0 + 1) | (s1 + 1) << 2 | (s2 + 1) << 4 | (s3 + 1) << 6);
+}
 
 // A cell with h > GEOFLOW_TINY: get_slopes, gmfggetcoef, eigen, and the velocities, wave speed and
 // friction signs that the corrector forms from the same values (update_cell).
 template <bool FAST, bool DERIV>
 __device__ __forceinline__ void staged_coef64(const StagedView<double> &v, int c, uint8_t bf, int mat, double gz,
-                                              const MatConsts &mc, double ft, const double ui[3], Coef64 &o) {
+                                              const MatConsts &mc, double ft, const double ui[3],
+                                              StagedCoef<double> &o) {
     staged_slopes64<FAST, DERIV>(v, c, bf, mc.gamma, ui, o.s, o.q);
     const double *s = o.s;
     const double h = ui[0], hu = ui[1], hv = ui[2];
-    const Divisor<FAST> dh(h), dhh(h * h);
+    const Divisor<double, FAST> dh(h), dhh(h * h);
     o.vx = dh(hu);
     o.vy = dh(hv);
     const double vel = dh(s[1]) - dhh(hu * s[0]) + dh(s[5]) - dhh(hv * s[3]);
@@ -407,32 +412,56 @@ __device__ __forceinline__ void staged_coef64(const StagedView<double> &v, int c
     const double h_inv = dh(1.0);
     const int s0 = int(tiny_sgn(h_inv * (s[4] - o.vx * s[3]), ft)), s2 = int(tiny_sgn(o.vx, ft));
     const int s1 = int(tiny_sgn(h_inv * (s[2] - o.vy * s[0]), ft)), s3 = int(tiny_sgn(o.vy, ft));
-    o.sgn = uint8_t((s0 + 1) | (s1 + 1) << 2 | (s2 + 1) << 4 | (s3 + 1) << 6);
+    o.sgn = pack_signs(s0, s1, s2, s3);
+}
+
+// The same in FP32, from the helpers of the unstaged phases (their operations, hence their bits).
+template <bool DERIV>
+__device__ __forceinline__ void staged_coef32(const StagedView<float> &v, int c, uint8_t bf, int mat, float gz,
+                                              const MatConsts &mc, float ft, const float ui[3], StagedCoef<float> &o) {
+    cell_slopes<float>(v, c, bf, float(mc.gamma), ui, o.s);
+    const float *s = o.s;
+    const float h = ui[0];
+    o.k = cell_kact<float>(mc, mat, h, ui[1], ui[2], s, &o.code);
+    o.vx = ui[1] / h;
+    o.vy = ui[2] / h;
+    const float cc = sqrt(o.k * gz * h);
+    o.a = sqrt(o.k * h * gz);
+    const float evx = dabs(o.vx) + cc, evy = dabs(o.vy) + cc;
+    o.ev = evx > evy ? evx : evy;
+    const float h_inv = 1.0f / h, vel0 = ui[1] * h_inv, vel1 = ui[2] * h_inv;
+    const int s0 = int(tiny_sgn(h_inv * (s[4] - vel0 * s[3]), ft)), s2 = int(tiny_sgn(vel0, ft));
+    const int s1 = int(tiny_sgn(h_inv * (s[2] - vel1 * s[0]), ft)), s3 = int(tiny_sgn(vel1, ft));
+    o.sgn = pack_signs(s0, s1, s2, s3);
+    if (DERIV) {
+        o.q[0] = o.q[1] = o.q[2] = o.q[3] = 0.0f;
+        if (!(bf & 0x0F)) slope_quotients<float>(v, c, bf, float(mc.gamma), h, o.q);
+    }
 }
 
 // A side of a Riemann problem from the staged values (dirflux): zero for a dry cell.
-struct Side64 {
-    double u[3], f[3], s0, s1, s2;
+template <class R>
+struct StagedSide {
+    R u[3], f[3], s0, s1, s2;
 };
 
-template <int DIR>
-__device__ __forceinline__ Side64 staged_side64(const StageBuf<double> &b, int e) {
-    Side64 o;
-    const double h = b.h[e];
-    const bool wet = !(h < DA_TINY);
-    o.u[0] = wet ? h : 0.0;
-    o.u[1] = wet ? b.hu[e] : 0.0;
-    o.u[2] = wet ? b.hv[e] : 0.0;
-    const double vel = wet ? (DIR == 0 ? b.c0[e] : b.c1[e]) : 0.0, a = wet ? b.a[e] : 0.0;
-    const double p = 0.5 * a * a * o.u[0];
+template <class R, int DIR>
+__device__ __forceinline__ StagedSide<R> staged_side(const StageBuf<R> &b, int e) {
+    StagedSide<R> o;
+    const R h = b.h[e];
+    const bool wet = !(h < R(DA_TINY));
+    o.u[0] = wet ? h : R(0);
+    o.u[1] = wet ? b.hu[e] : R(0);
+    o.u[2] = wet ? b.hv[e] : R(0);
+    const R vel = wet ? (DIR == 0 ? b.c0[e] : b.c1[e]) : R(0), a = wet ? b.a[e] : R(0);
     if (DIR == 0) {
         o.f[0] = o.u[1];
-        o.f[1] = o.u[1] * vel + p;
+        o.f[1] = o.u[1] * vel + R(0.5) * a * a * o.u[0];
         o.f[2] = o.u[2] * vel;
     } else {
         o.f[0] = o.u[2];
         o.f[1] = o.u[1] * vel;
-        o.f[2] = o.u[2] * vel + p;
+        o.f[2] = o.u[2] * vel + R(0.5) * a * a * o.u[0];
     }
     o.s0 = vel - a;
     o.s1 = vel;
@@ -442,86 +471,111 @@ __device__ __forceinline__ Side64 staged_side64(const StageBuf<double> &b, int e
 
 // riemann (fv_device.cuh) with one divisor for the three components.  Two dry sides give zero speeds,
 // hence the left flux, which is zero.
-template <bool FAST>
-__device__ __forceinline__ void riemann64(const Side64 &l, const Side64 &r, double F[3]) {
-    const bool ld = l.u[0] == 0.0, rd = r.u[0] == 0.0;
-    const double a0 = 2.0 * r.s0 - r.s1, a2 = 2.0 * r.s2 - r.s1;
-    const double b0 = 2.0 * l.s0 - l.s1, b2 = 2.0 * l.s2 - l.s1;
-    const double lo = ld ? a0 : (rd ? b0 : rmin(l.s0, r.s0));
-    const double hi = ld ? a2 : (rd ? b2 : rmax(l.s2, r.s2));
-    const double sl = rmin(0.0, lo), sr = rmax(0.0, hi);
-    if (sl >= 0.0) {
+template <class R, bool FAST>
+__device__ __forceinline__ void staged_riemann(const StagedSide<R> &l, const StagedSide<R> &r, R F[3]) {
+    const bool ld = l.u[0] == R(0), rd = r.u[0] == R(0);
+    const R a0 = R(2.0) * r.s0 - r.s1, a2 = R(2.0) * r.s2 - r.s1;
+    const R b0 = R(2.0) * l.s0 - l.s1, b2 = R(2.0) * l.s2 - l.s1;
+    const R lo = ld ? a0 : (rd ? b0 : rmin(l.s0, r.s0));
+    const R hi = ld ? a2 : (rd ? b2 : rmax(l.s2, r.s2));
+    const R sl = rmin(R(0), lo), sr = rmax(R(0), hi);
+    if (sl >= R(0)) {
         F[0] = l.f[0]; F[1] = l.f[1]; F[2] = l.f[2];
-    } else if (sr <= 0.0) {
+    } else if (sr <= R(0)) {
         F[0] = r.f[0]; F[1] = r.f[1]; F[2] = r.f[2];
     } else {
-        const Divisor<FAST> den(sr - sl);
+        const Divisor<R, FAST> den(sr - sl);
 #pragma unroll
         for (int v = 0; v < 3; ++v) F[v] = den(sr * l.f[v] - sl * r.f[v] + sl * sr * (r.u[v] - l.u[v]));
     }
 }
 
 // F(+side) - F(-side) in direction DIR of cell c (flux_div).
-template <bool FAST, int DIR>
-__device__ __forceinline__ void staged_div64(const StagedView<double> &v, int c, uint8_t bf, double div[3]) {
+template <class R, bool FAST, int DIR>
+__device__ __forceinline__ void staged_div(const StagedView<R> &v, int c, uint8_t bf, R div[3]) {
     if (bf & ((1 << DIR) | (1 << (DIR + 2)))) {
-        div[0] = div[1] = div[2] = 0.0;
+        div[0] = div[1] = div[2] = R(0);
         return;
     }
-    const Side64 self = staged_side64<DIR>(v.b, c);
-    double Fm[3], Fp[3];
-    riemann64<FAST>(staged_side64<DIR>(v.b, v.nl[DIR + 2]), self, Fm);
-    riemann64<FAST>(self, staged_side64<DIR>(v.b, v.nl[DIR]), Fp);
+    const StagedSide<R> self = staged_side<R, DIR>(v.b, c);
+    R Fm[3], Fp[3];
+    staged_riemann<R, FAST>(staged_side<R, DIR>(v.b, v.nl[DIR + 2]), self, Fm);
+    staged_riemann<R, FAST>(self, staged_side<R, DIR>(v.b, v.nl[DIR]), Fp);
     if (bf & (0x10 << (DIR + 2))) {
-        double F2[3];
-        riemann64<FAST>(staged_side64<DIR>(v.b, v.nl[DIR + 6]), self, F2);
+        R F2[3];
+        staged_riemann<R, FAST>(staged_side<R, DIR>(v.b, v.nl[DIR + 6]), self, F2);
 #pragma unroll
-        for (int q = 0; q < 3; ++q) Fm[q] = 0.5 * (Fm[q] + F2[q]);
+        for (int q = 0; q < 3; ++q) Fm[q] = R(0.5) * (Fm[q] + F2[q]);
     }
     if (bf & (0x10 << DIR)) {
-        double F2[3];
-        riemann64<FAST>(self, staged_side64<DIR>(v.b, v.nl[DIR + 4]), F2);
+        R F2[3];
+        staged_riemann<R, FAST>(self, staged_side<R, DIR>(v.b, v.nl[DIR + 4]), F2);
 #pragma unroll
-        for (int q = 0; q < 3; ++q) Fp[q] = 0.5 * (Fp[q] + F2[q]);
+        for (int q = 0; q < 3; ++q) Fp[q] = R(0.5) * (Fp[q] + F2[q]);
     }
 #pragma unroll
     for (int q = 0; q < 3; ++q) div[q] = Fp[q] - Fm[q];
 }
 
 // What the update phase loads of a cell ahead of the fluxes.
-struct Kept64 {
-    double sx, sy;  // depth slopes
+template <class R>
+struct Kept {
+    R sx, sy;  // depth slopes
     uint8_t sgn;
 };
 
+// g_z ds + dg h of the internal friction; FP32 with the one rounding that the compiler's contraction gives
+// update_cell (which of the two products is rounded is its choice, so it is spelled out here).
+template <class R>
+__device__ __forceinline__ R slope_term(R gz, R ds, R dg, R h) {
+    if constexpr (sizeof(R) == 8)
+        return gz * ds + dg * h;
+    else
+        return __fmaf_rn(dg, h, __fmul_rn(gz, ds));
+}
+
 // update_cell (forward_impl.cuh) of an active cell from the staged and kept values.
-template <bool FAST, class Hook>
-__device__ __forceinline__ bool staged_update64(const StagedView<double> &v, int c, uint8_t bf, const CellSrc<double> &cs,
-                                                const MatConsts &mc, double dt, const double prev[3], double dxc,
-                                                double dyc, double st[3], const Kept64 &kp, const Hook &hook) {
-    double dx3[3], dy3[3];
-    staged_div64<FAST, 0>(v, c, bf, dx3);
-    staged_div64<FAST, 1>(v, c, bf, dy3);
-    const double dtdx = dt / dxc;
-    const double dtdy = dyc == dxc ? dtdx : dt / dyc;
+template <class R, bool FAST, class Hook>
+__device__ __forceinline__ bool staged_update(const StagedView<R> &v, int c, uint8_t bf, const CellSrc<R> &cs,
+                                              const MatConsts &mc, R dt, const R prev[3], R dxc, R dyc, R st[3],
+                                              const Kept<R> &kp, const Hook &hook) {
+    R dx3[3], dy3[3];
+    staged_div<R, FAST, 0>(v, c, bf, dx3);
+    staged_div<R, FAST, 1>(v, c, bf, dy3);
+    R dtdx, dtdy;
+    if constexpr (sizeof(R) == 8) {
+        dtdx = dt / dxc;
+        dtdy = dyc == dxc ? dtdx : dt / dyc;
+    } else {
+        dtdx = dt * (1.0f / dxc);
+        dtdy = dt * (1.0f / dyc);
+    }
 #pragma unroll
     for (int q = 0; q < 3; ++q) st[q] = prev[q] - dtdx * dx3[q] - dtdy * dy3[q];
-    const bool clamped = st[0] < 0.0;
-    if (clamped) st[0] = 0.0;
-    if (prev[0] > DA_TINY) {
-        const double vel0 = v.b.c0[c], vel1 = v.b.c1[c];
-        auto sg = [&](int q) { return double(int((kp.sgn >> (2 * q)) & 3) - 1); };
-        const double sg0 = sg(0), sg1 = sg(1), sg2 = sg(2), sg3 = sg(3);
-        hook(SrcFwd<double>{{kp.sx, 0.0, 0.0, kp.sy, 0.0, 0.0}, vel0, vel1, 0.0, sg0, sg1, sg2, sg3}, clamped);
-        const double ki = v.b.k[c], gz = v.b.gz[c];
-        const double sin_int = mc.sin_int, tan_bed = mc.tan_bed[cs.mat];
-        double s1 = cs.g[0] * prev[0];
-        double s2 = sg0 * prev[0] * ki * (gz * kp.sy + cs.dg[1] * prev[0]) * sin_int;
-        double s3 = sg2 * rmax(gz * prev[0] + vel0 * prev[1] * cs.cv[0], 0.0) * tan_bed;
+    const bool clamped = st[0] < R(0);
+    if (clamped) st[0] = R(0);
+    if (prev[0] > R(DA_TINY)) {
+        R vel0, vel1;
+        if constexpr (sizeof(R) == 8) {
+            vel0 = v.b.c0[c];
+            vel1 = v.b.c1[c];
+        } else {  // the sources' velocities are products with 1 / h
+            const float h_inv = 1.0f / prev[0];
+            vel0 = prev[1] * h_inv;
+            vel1 = prev[2] * h_inv;
+        }
+        auto sg = [&](int q) { return R(int((kp.sgn >> (2 * q)) & 3) - 1); };
+        const R sg0 = sg(0), sg1 = sg(1), sg2 = sg(2), sg3 = sg(3);
+        hook(SrcFwd<R>{{kp.sx, R(0), R(0), kp.sy, R(0), R(0)}, vel0, vel1, R(0), sg0, sg1, sg2, sg3}, clamped);
+        const R ki = v.b.k[c], gz = v.b.gz[c];
+        const R sin_int = R(mc.sin_int), tan_bed = R(mc.tan_bed[cs.mat]);
+        R s1 = cs.g[0] * prev[0];
+        R s2 = sg0 * prev[0] * ki * slope_term(gz, kp.sy, cs.dg[1], prev[0]) * sin_int;
+        R s3 = sg2 * rmax(gz * prev[0] + vel0 * prev[1] * cs.cv[0], R(0)) * tan_bed;
         st[1] += dt * (s1 - s2 - s3);
         s1 = cs.g[1] * prev[0];
-        s2 = sg1 * prev[0] * ki * (gz * kp.sx + cs.dg[0] * prev[0]) * sin_int;
-        s3 = sg3 * rmax(gz * prev[0] + vel1 * prev[2] * cs.cv[1], 0.0) * tan_bed;
+        s2 = sg1 * prev[0] * ki * slope_term(gz, kp.sx, cs.dg[0], prev[0]) * sin_int;
+        s3 = sg3 * rmax(gz * prev[0] + vel1 * prev[2] * cs.cv[1], R(0)) * tan_bed;
         st[2] += dt * (s1 - s2 - s3);
     }
     return clamped;
@@ -580,50 +634,35 @@ __device__ __forceinline__ void coef_phase_staged(const MeshArgs &m, const HaloA
                     }
                     const R ui[3] = {h, b.hu[c], b.hv[c]};
                     const R gz = b.gz[c];
+                    R *kept = (R *)ha.kept;
                     if (!(h > R(DA_TINY))) {  // h == GEOFLOW_TINY: dry for get_coef_and_eigen, wet for the fluxes
-                        kact[i] = R(mc.kact_rest);
-                        if constexpr (sizeof(R) == 8) {
-                            R *kept = (R *)ha.kept;
-                            kept[(size_t)2 * m.n + i] = ui[1] / h;
-                            kept[(size_t)3 * m.n + i] = ui[2] / h;
-                            kept[(size_t)4 * m.n + i] = sqrt(mc.kact_rest * h * gz);
-                        }
+                        const R k = R(mc.kact_rest);
+                        kact[i] = k;
+                        kept[(size_t)2 * m.n + i] = ui[1] / h;
+                        kept[(size_t)3 * m.n + i] = ui[2] / h;
+                        kept[(size_t)4 * m.n + i] = sqrt(k * h * gz);
                     } else {
-                        R ev;
-                        R *kept = (R *)ha.kept;
+                        StagedCoef<R> o;
                         if constexpr (sizeof(R) == 8) {
-                            Coef64 o;
                             if (fast)
                                 staged_coef64<true, RECORD>(v, c, bf, mat, gz, mc, ft, ui, o);
                             else
                                 staged_coef64<false, RECORD>(v, c, bf, mat, gz, mc, ft, ui, o);
-                            code = o.code;
-                            kact[i] = o.k;
-                            kept[i] = o.s[0];
-                            kept[(size_t)m.n + i] = o.s[3];
-                            kept[(size_t)2 * m.n + i] = o.vx;
-                            kept[(size_t)3 * m.n + i] = o.vy;
-                            kept[(size_t)4 * m.n + i] = o.a;
-                            ha.fsign[i] = o.sgn;
-                            if (RECORD)
-#pragma unroll
-                                for (int q = 0; q < 4; ++q) kept[(size_t)(5 + q) * m.n + i] = o.q[q];
-                            ev = o.ev;
                         } else {
-                            R s[6];
-                            cell_slopes<R>(v, c, bf, R(mc.gamma), ui, s);
-                            // kept for the update phase's source terms
-                            kept[i] = s[0];
-                            kept[(size_t)m.n + i] = s[2];
-                            kept[(size_t)2 * m.n + i] = s[3];
-                            kept[(size_t)3 * m.n + i] = s[4];
-                            const R k = cell_kact<R>(mc, mat, h, ui[1], ui[2], s, &code);
-                            kact[i] = k;
-                            const R vx = ui[1] / h, vy = ui[2] / h;
-                            const R cc = sqrt(k * gz * h);
-                            const R evx = dabs(vx) + cc, evy = dabs(vy) + cc;
-                            ev = evx > evy ? evx : evy;
+                            staged_coef32<RECORD>(v, c, bf, mat, gz, mc, ft, ui, o);
                         }
+                        code = o.code;
+                        kact[i] = o.k;
+                        kept[i] = o.s[0];
+                        kept[(size_t)m.n + i] = o.s[3];
+                        kept[(size_t)2 * m.n + i] = o.vx;
+                        kept[(size_t)3 * m.n + i] = o.vy;
+                        kept[(size_t)4 * m.n + i] = o.a;
+                        ha.fsign[i] = o.sgn;
+                        if (RECORD)
+#pragma unroll
+                            for (int q = 0; q < 4; ++q) kept[(size_t)(5 + q) * m.n + i] = o.q[q];
+                        const R ev = o.ev;
                         if (ev > R(1000000000.)) raise_err(sc, DA_ERR_EIGEN);
                         const unsigned long long rb = __double_as_longlong(double((dxm > dym ? dym : dxm) / ev));
                         const unsigned long long hb = __double_as_longlong(double(h));
@@ -700,19 +739,11 @@ __device__ __forceinline__ void update_phase_staged(const MeshArgs &m, const Hal
                 // what this step's coefficient phase left for a wet cell, loaded ahead of the fluxes
                 const bool wet = prev[0] > R(DA_TINY);
                 const R *kept = (const R *)ha.kept;
-                Kept64 kp{};
-                R pre_s[6] = {};
+                Kept<R> kp{};
                 if (wet) {
-                    if constexpr (sizeof(R) == 8) {
-                        kp.sx = kept[i];
-                        kp.sy = kept[(size_t)m.n + i];
-                        kp.sgn = ha.fsign[i];
-                    } else {
-                        pre_s[0] = kept[i];
-                        pre_s[2] = kept[(size_t)m.n + i];
-                        pre_s[3] = kept[(size_t)2 * m.n + i];
-                        pre_s[4] = kept[(size_t)3 * m.n + i];
-                    }
+                    kp.sx = kept[i];
+                    kp.sy = kept[(size_t)m.n + i];
+                    kp.sgn = ha.fsign[i];
                 }
                 const auto pre = epi.pre(i, wet);
                 const uint8_t bf = b.bf[c];
@@ -725,14 +756,7 @@ __device__ __forceinline__ void update_phase_staged(const MeshArgs &m, const Hal
                     act |= b.h[v.nl[s]] >= R(DA_TINY);
                     if (bf & (0x10 << s)) act |= b.h[v.nl[s + 4]] >= R(DA_TINY);
                 }
-                R dxc, dyc;
-                if constexpr (sizeof(R) == 8) {
-                    dxc = b.sz[0][c];
-                    dyc = b.sz[1][c];
-                } else {
-                    dxc = b.c0[c];
-                    dyc = b.c1[c];
-                }
+                const R dxc = b.sz[0][c], dyc = b.sz[1][c];
                 R st[3] = {prev[0], prev[1], prev[2]};
                 bool clamped = false;
                 const CellSrc<R> cs = staged_src(b, c);
@@ -745,12 +769,11 @@ __device__ __forceinline__ void update_phase_staged(const MeshArgs &m, const Hal
                 if (act) {
                     if constexpr (sizeof(R) == 8) {
                         if (fast)
-                            clamped = staged_update64<true>(v, c, bf, cs, mc, dt, prev, dxc, dyc, st, kp, hook);
+                            clamped = staged_update<R, true>(v, c, bf, cs, mc, dt, prev, dxc, dyc, st, kp, hook);
                         else
-                            clamped = staged_update64<false>(v, c, bf, cs, mc, dt, prev, dxc, dyc, st, kp, hook);
+                            clamped = staged_update<R, false>(v, c, bf, cs, mc, dt, prev, dxc, dyc, st, kp, hook);
                     } else {
-                        clamped = update_cell<R>(v, c, bf, cs, mc, dt, ft, prev, dxc, dyc, st, wet ? pre_s : nullptr,
-                                                 hook);
+                        clamped = staged_update<R, true>(v, c, bf, cs, mc, dt, prev, dxc, dyc, st, kp, hook);
                     }
                 }
                 const uint8_t code = RECORD ? uint8_t(kcode | (act ? 8 : 0) | (clamped ? 4 : 0)) : 0;
