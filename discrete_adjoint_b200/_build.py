@@ -36,6 +36,7 @@ UNITS = [
     ("ensemble.cu", []),
     ("dwr.cu", []),
     ("stats.cu", []),
+    ("tile_order.cu", []),
     ("mesh_host.cpp", []),
     ("solution_io.cpp", []),
     ("restart_io.cpp", []),

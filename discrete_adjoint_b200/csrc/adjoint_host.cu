@@ -222,12 +222,22 @@ struct Runner {
     // Consecutive forward advances (a chain of checkpoint stores between a restore and the next
     // reverse step) go out as one multi-step launch that stores the checkpoints on its way: the
     // advances wait here until a restore, a reverse step or the end of the sweep needs the state.
+    // The tiles in a new order, from the flags of the last step that ran, before a chain of forward steps:
+    // a flow needs some ten steps to cross a tile.
+    static constexpr int kOrderSteps = 64;
+    long long ordered_at = 0;
+    int order_tiles() {
+        if (fsteps - ordered_at < kOrderSteps) return DA_OK;
+        ordered_at = fsteps;
+        return launch_tile_order(ctx);
+    }
     int def_k = 0;
     void *def_pre = nullptr;
     MidStoreList def_mid;
     int flush() {
         if (def_k == 0) return DA_OK;
-        const int st = launch_forward_steps(ctx, def_k, def_pre, nullptr, &def_mid);
+        int st = order_tiles();
+        if (!st) st = launch_forward_steps(ctx, def_k, def_pre, nullptr, &def_mid);
         def_k = 0;
         def_pre = nullptr;
         def_mid.n = 0;
@@ -260,7 +270,10 @@ struct Runner {
         fsteps += k;
         pos += k;
         void *slot = store_slot >= 0 ? ctx->snaps[store_slot] : nullptr;
-        if (ctx->ninst > 0) return launch_forward_steps(ctx, k, take_pending(), slot);  // one launch each
+        if (ctx->ninst > 0) {  // one launch each
+            const int so = order_tiles();
+            return so ? so : launch_forward_steps(ctx, k, take_pending(), slot);
+        }
         int st = DA_OK;
         if (slot && def_mid.n == kMidStores) st = flush();
         if (def_k == 0) def_pre = take_pending();
@@ -449,7 +462,7 @@ std::vector<unsigned char> sweep_key(const da_ctx *ctx, const double *box, int n
     const void *ptrs[] = {ctx->U[0][0], ctx->U[0][1], ctx->U[0][2], ctx->U[1][0], ctx->U[1][1], ctx->U[1][2],
                           ctx->lam[0][0], ctx->lam[0][1], ctx->lam[0][2], ctx->lam[1][0], ctx->lam[1][1],
                           ctx->lam[1][2], ctx->kact, ctx->slopes, ctx->fsign, ctx->run_flags, ctx->active, ctx->seg_clean, ctx->seg_wet, ctx->seg_vol,
-                          ctx->seg_dirty, ctx->mask, ctx->tile_epoch, ctx->seg_act, ctx->lam_clean, ctx->adjA,
+                          ctx->seg_dirty, ctx->mask, ctx->tile_order, ctx->tile_epoch, ctx->seg_act, ctx->lam_clean, ctx->adjA,
                           ctx->adjB, ctx->gbed, ctx->gint, ctx->dk_tab, ctx->red_out, ctx->red_part, ctx->inst_J,
                           ctx->seg_J, ctx->dh0, ctx->dsc};
     put(ptrs, sizeof(ptrs));
@@ -500,6 +513,7 @@ int adjoint_sweep(da_ctx *ctx, const double *box, int32_t nsteps, int32_t nsnaps
         if (!s && r.dwr)
             s = cuda_check(ctx, cudaMemsetAsync(ctx->dwr.acc, 0, sizeof(double) * (size_t)ctx->mesh.n, ctx->stream), "memset");
         r.pos = 0;
+        if (!s) s = launch_tile_order(ctx);  // the store has formed every segment's wet flag
         if (!s) s = r.reverse(0, nsteps, 0);
         if (!s) s = r.flush();
         if (!s) s = r.flush_run();

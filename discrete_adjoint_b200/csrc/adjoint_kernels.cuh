@@ -98,11 +98,11 @@ template <class R, bool BATCH>
 __device__ __forceinline__ void gather_staged(const MeshArgs &m, const fwd::HaloArgs &ha, const StateRef<R> &U,
                                               const StateRef<R> &Ln, const StateOut<R> &Lo, const MatConsts &mc,
                                               const AdjArgs &aa, int rec_id, double dt, int *list, const InstArgs &ia,
-                                              void *smem, bool quarter) {
+                                              void *smem, bool quarter, const fwd::FirstTiles<R> &first) {
     if constexpr (sizeof(R) == 8)
-        adj_gather_phase64<BATCH>(m, ha, U, Ln, Lo, mc, aa, rec_id, dt, list, ia, *(GatherSmem64 *)smem, quarter);
+        adj_gather_phase64<BATCH>(m, ha, U, Ln, Lo, mc, aa, rec_id, dt, list, ia, *(GatherSmem64 *)smem, quarter, first);
     else
-        adj_gather_phase_staged<R, BATCH>(m, ha, U, Ln, Lo, mc, aa, rec_id, R(dt), list, ia, *(GatherSmem<R> *)smem, quarter);
+        adj_gather_phase_staged<R, BATCH>(m, ha, U, Ln, Lo, mc, aa, rec_id, R(dt), list, ia, *(GatherSmem<R> *)smem, quarter, first);
 }
 template <class R>
 constexpr size_t gather_staged_bytes() {
@@ -134,12 +134,17 @@ __global__ void __launch_bounds__(kBlock, OCC) k_youturn(MeshArgs m, fwd::StateP
     __shared__ int list[kBlock];
     extern __shared__ __align__(16) unsigned char dyn_smem[];
     fwd::StageSmem<R> &stg = *reinterpret_cast<fwd::StageSmem<R> *>(dyn_smem);
+    __shared__ fwd::FirstTiles<R> first;
+    const fwd::FirstLoad<R, BATCH> fl(ha, STAGED ? ntiles : 0);
     // the recording update counts its listed tiles from zero (the adds follow a barrier)
     if (blockIdx.x == 0 && threadIdx.x == 0) sc->listed = 0u;
     if (pre.mode != snap::NONE) {
         snap::snap_segments<R>(pre);
         snap::snap_scalars<R>(pre);
+        if (STAGED) fl.store(ha, first);
         if (!fwd::grid_sync(sc)) return;
+    } else if (STAGED) {
+        fl.store(ha, first);
     }
     const double time = __ldcg(&sc->time);
     const long long iter = __ldcg(&sc->iter);
@@ -148,7 +153,7 @@ __global__ void __launch_bounds__(kBlock, OCC) k_youturn(MeshArgs m, fwd::StateP
     unsigned long long my_min = 0x7FF0000000000000ull, my_max = 0ull;
     if (STAGED)
         fwd::coef_phase_staged<R, true, BATCH>(m, ha, U, kact, active, seg_wet, ntiles, cull, mc, sc, mask, list, my_min,
-                                               my_max, ia, stg, fwd::sign_threshold<R>(iter, tc, mc));
+                                               my_max, ia, stg, fwd::sign_threshold<R>(iter, tc, mc), first);
     else
         fwd::coef_phase<R, true, BATCH>(m, U, kact, active, seg_wet, ntiles, cull, mc, sc, mask, list, my_min, my_max,
                                         ia);
@@ -173,9 +178,9 @@ __global__ void __launch_bounds__(kBlock, OCC) k_youturn(MeshArgs m, fwd::StateP
         const SrcEpilogue<R, BATCH> src{m, Ln, mc, aa, ia, R(dt), (const R *)ha.kept};
         fwd::update_phase_staged<R, true, BATCH>(m, ha, U, O, kact, active, seg_clean, seg_wet, seg_vol, seg_dirty,
                                                  ntiles, cull, mc, sc, R(dt), ftr, mask, tile_epoch, seg_act, rec_id,
-                                                 list, ia, stg, src);
+                                                 list, ia, stg, first, src);
         if (!fwd::grid_sync(sc)) return;
-        gather_staged<R, BATCH>(m, ha, U, Ln, Lo, mc, aa, rec_id, dt, list, ia, dyn_smem, gather_quarters(sc, gsplit));
+        gather_staged<R, BATCH>(m, ha, U, Ln, Lo, mc, aa, rec_id, dt, list, ia, dyn_smem, gather_quarters(sc, gsplit), first);
         if (blockIdx.x == 0 && threadIdx.x == 0) {
             sc->iter = iter + 1;
             sc->frict_tiny = ft;
@@ -194,7 +199,7 @@ __global__ void __launch_bounds__(kBlock, OCC) k_youturn(MeshArgs m, fwd::StateP
     if (STAGED)
         fwd::update_phase_staged<R, true, BATCH>(m, ha, U, O, kact, active, seg_clean, seg_wet, seg_vol, seg_dirty,
                                                  ntiles, cull, mc, sc, R(dt), ftr, mask, tile_epoch, seg_act, rec_id,
-                                                 list, ia, stg);
+                                                 list, ia, stg, first);
     else
         fwd::update_phase<R, true, BATCH>(m, U, O, kact, active, seg_clean, seg_wet, seg_vol, seg_dirty, ntiles, cull,
                                           mc, sc, R(dt), ftr, mask, tile_epoch, seg_act, rec_id, list, ia);
@@ -206,7 +211,7 @@ __global__ void __launch_bounds__(kBlock, OCC) k_youturn(MeshArgs m, fwd::StateP
     adj_src_phase<R, BATCH>(m, U, Ln, mc, aa, R(dt), ftr, list, ia);
     if (!fwd::grid_sync(sc)) return;
     if (STAGED)
-        gather_staged<R, BATCH>(m, ha, U, Ln, Lo, mc, aa, rec_id, dt, list, ia, dyn_smem, gather_quarters(sc, gsplit));
+        gather_staged<R, BATCH>(m, ha, U, Ln, Lo, mc, aa, rec_id, dt, list, ia, dyn_smem, gather_quarters(sc, gsplit), first);
     else
         adj_gather_phase<R, BATCH>(m, U, Ln, Lo, mc, aa, R(dt), list, ia);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -320,6 +325,8 @@ __global__ void __launch_bounds__(kBlock, OCC) k_reverse_run(MeshArgs m, fwd::St
     extern __shared__ __align__(16) unsigned char dyn_smem[];
     fwd::StageSmem<R> &stg = *reinterpret_cast<fwd::StageSmem<R> *>(dyn_smem);
     const int t0 = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
+    __shared__ fwd::FirstTiles<R> first;
+    const fwd::FirstLoad<R, false> fl(ha, ntiles);
     for (int s = t0; s < ra.nseg; s += nt) {
         const uint8_t d = seg_dirty[s], w = seg_wet[s];
         ra.dirty[0][s] = ra.dirty[1][s] = d;
@@ -329,7 +336,10 @@ __global__ void __launch_bounds__(kBlock, OCC) k_reverse_run(MeshArgs m, fwd::St
     if (ra.slot[0]) {
         if (!fwd::grid_sync(sc)) return;
         run_restore<R>(ra, 0, cur, S, m.n);
+        fl.store(ha, first);
         if (!fwd::grid_sync(sc)) return;
+    } else {
+        fl.store(ha, first);
     }
     for (int k = 0; k < ra.n; ++k) {
         const int p = (cur + k) & 1, rec_id = rec_id0 + k;
@@ -347,7 +357,7 @@ __global__ void __launch_bounds__(kBlock, OCC) k_reverse_run(MeshArgs m, fwd::St
         if (blockIdx.x == 0 && threadIdx.x == 0) sc->listed = 0u;
         unsigned long long my_min = 0x7FF0000000000000ull, my_max = 0ull;
         fwd::coef_phase_staged<R, true>(m, ha, U, kact, active, ra.slot[k] ? ra.wet[p] : seg_wet, ntiles, cull, mc, sc,
-                                        mask, list, my_min, my_max, InstArgs{}, stg, ftr);
+                                        mask, list, my_min, my_max, InstArgs{}, stg, ftr, first);
         fwd::push_minmax(my_min, my_max, acc_min, acc_max);
         if (!fwd::grid_sync(sc)) return;
         const double min_dxe = __longlong_as_double(__ldcg(acc_min)), hmax = __longlong_as_double(__ldcg(acc_max));
@@ -362,10 +372,10 @@ __global__ void __launch_bounds__(kBlock, OCC) k_reverse_run(MeshArgs m, fwd::St
         const SrcEpilogue<R, false> src{m, Ln, mc, aa, InstArgs{}, R(dt), (const R *)ha.kept};
         fwd::update_phase_staged<R, true, false, false>(m, ha, U, StateOut<R>{}, kact, active, nullptr, nullptr, nullptr,
                                                         nullptr, ntiles, cull, mc, sc, R(dt), ftr, mask, tile_epoch,
-                                                        seg_act, rec_id, list, InstArgs{}, stg, src);
+                                                        seg_act, rec_id, list, InstArgs{}, stg, first, src);
         if (!fwd::grid_sync(sc)) return;
         gather_staged<R, false>(m, ha, U, Ln, Lo, mc, aa, rec_id, dt, list, InstArgs{}, dyn_smem,
-                                gather_quarters(sc, gsplit));
+                                gather_quarters(sc, gsplit), first);
         if (k + 1 < ra.n) {
             run_restore<R>(ra, k + 1, p ^ 1, S, m.n);
             if (!fwd::grid_sync(sc)) return;

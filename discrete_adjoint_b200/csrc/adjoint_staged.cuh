@@ -214,12 +214,13 @@ __device__ __forceinline__ void adj_gather_phase_staged(const MeshArgs &m, const
                                                         const StateRef<R> &U, const StateRef<R> &Lnext,
                                                         const StateOut<R> &Lout, const MatConsts &mc0,
                                                         const AdjArgs &aa, int rec_id, R dt0, int *list,
-                                                        const InstArgs &ia, GatherSmem<R> &S, bool quarter) {
+                                                        const InstArgs &ia, GatherSmem<R> &S, bool quarter, const fwd::FirstTiles<R> &first) {
     GatherBuf<R> &g = S.g;
     const int lane = threadIdx.x & 31;
     const int nunits = quarter ? 4 * aa.ntiles : aa.ntiles;
     for (int round = 0; sched_more(round, nunits); ++round) {
-        const int uq = sched_tile(round);
+        const int uq = quarter ? fwd::staged_quarter<R, BATCH>(ha, round, first, aa.ntiles)
+                               : fwd::staged_tile<R, BATCH>(ha, round, first, aa.ntiles);
         const int tq = quarter ? uq >> 2 : uq;
         bool need = false;
         if (uq < nunits) {

@@ -178,12 +178,13 @@ template <bool BATCH>
 __device__ __forceinline__ void adj_gather_phase64(const MeshArgs &m, const fwd::HaloArgs &ha, const StateRef<double> &U,
                                                    const StateRef<double> &Lnext, const StateOut<double> &Lout,
                                                    const MatConsts &mc0, const AdjArgs &aa, int rec_id, double dt0,
-                                                   int *list, const InstArgs &ia, GatherSmem64 &S, bool quarter) {
+                                                   int *list, const InstArgs &ia, GatherSmem64 &S, bool quarter, const fwd::FirstTiles<double> &first) {
     const GatherBuf64 &g = S.g;
     const int lane = threadIdx.x & 31, s = lane & 3;
     const int nunits = quarter ? 4 * aa.ntiles : aa.ntiles;
     for (int round = 0; sched_more(round, nunits); ++round) {
-        const int uq = sched_tile(round);
+        const int uq = quarter ? fwd::staged_quarter<double, BATCH>(ha, round, first, aa.ntiles)
+                               : fwd::staged_tile<double, BATCH>(ha, round, first, aa.ntiles);
         const int tq = quarter ? uq >> 2 : uq;
         bool need = false;
         if (uq < nunits) {

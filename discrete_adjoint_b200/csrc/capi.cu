@@ -171,6 +171,8 @@ static void free_state(da_ctx *ctx) {
     dfree(ctx->stage);
     dfree(ctx->dd_bounds);
     dfree(ctx->tile_epoch);
+    dfree(ctx->tile_order);
+    ctx->tile_ordered = false;
     dfree(ctx->seg_act);
     dfree(ctx->lam_clean);
     ctx->have_state = false;

@@ -203,6 +203,8 @@ struct da_ctx {
     da::OutlineGrid outline;          // maximum-depth map (da_outline_init)
     double *stats_mem = nullptr;      // partial sums and result of the flow statistics (stats.cu)
     double *stats_host = nullptr;     // pinned copy of the result
+    int *tile_order = nullptr;       // [ntiles] the order in which the staged phases take the tiles
+    bool tile_ordered = false;       // other than plain
     int *tile_epoch = nullptr;       // [ntiles] id of the last recording step that listed the tile
     uint8_t *seg_act = nullptr;      // [nseg] the segment had an active cell in that step
     uint8_t *lam_clean = nullptr;    // [nseg] both adjoint buffers hold the same segment
@@ -278,6 +280,8 @@ int copy_d2h(da_ctx *ctx, void *host, const void *dev, size_t bytes, const char 
 void fill_consts(const da_params &p, MatConsts *mc, TimeConsts *tc);
 // every k act/pass value of the table zero or within [2^-60, 2^60] (quot.cuh)
 bool kact_ordinary(const MatConsts &mc);
+int plain_tile_order(da_ctx *ctx);
+int launch_tile_order(da_ctx *ctx);
 
 // forward_fp64.cu / forward_fp32.cu
 // record_mask (optional): branch codes of the step for the adjoint (listed tiles; tile_epoch)

@@ -59,6 +59,8 @@ int forward_alloc(da_ctx *ctx) {
     if (!st) st = cuda_check(ctx, cudaMalloc(&ctx->slopes, 9 * rs * n), "cudaMalloc(slopes)");
     if (!st) st = cuda_check(ctx, cudaMalloc((void **)&ctx->fsign, n), "cudaMalloc(signs)");
     if (!st) st = cuda_check(ctx, cudaMalloc((void **)&ctx->seg_wet, nseg), "cudaMalloc(seg_wet)");
+    if (!st) st = cuda_check(ctx, cudaMalloc((void **)&ctx->tile_order, sizeof(int) * ctx->ntiles), "cudaMalloc(order)");
+    if (!st) st = plain_tile_order(ctx);
     if (!st) st = cuda_check(ctx, cudaMalloc((void **)&ctx->tile_epoch, sizeof(int) * ctx->ntiles), "cudaMalloc(epoch)");
     if (!st) st = cuda_check(ctx, cudaMemsetAsync(ctx->tile_epoch, 0xff, sizeof(int) * ctx->ntiles, ctx->stream), "memset");
     if (!st) st = cuda_check(ctx, cudaMalloc((void **)&ctx->seg_act, nseg), "cudaMalloc(seg_act)");

@@ -592,11 +592,16 @@ __global__ void __launch_bounds__(kBlock, OCC) k_steps(MeshArgs m, StatePair<R> 
     __shared__ int list[kBlock];
     extern __shared__ __align__(16) unsigned char dyn_smem[];
     StageSmem<R> &stg = *reinterpret_cast<StageSmem<R> *>(dyn_smem);
+    __shared__ FirstTiles<R> first;
+    const FirstLoad<R, BATCH> fl(ha, STAGED ? ntiles : 0);
     if (pre.mode != snap::NONE) {
         // a checkpoint restore first (both buffers, flags, scalars), then a barrier
         snap::snap_segments<R>(pre);
         snap::snap_scalars<R>(pre);
+        if (STAGED) fl.store(ha, first);
         if (!grid_sync(sc)) return;
+    } else if (STAGED) {
+        fl.store(ha, first);
     }
     double time = __ldcg(&sc->time);
     long long iter = __ldcg(&sc->iter);
@@ -612,7 +617,7 @@ __global__ void __launch_bounds__(kBlock, OCC) k_steps(MeshArgs m, StatePair<R> 
         unsigned long long my_min = 0x7FF0000000000000ull, my_max = 0ull;
         if (STAGED)
             coef_phase_staged<R, false, BATCH>(m, ha, U, kact, active, seg_wet, ntiles, cull, mc, sc, nullptr, list,
-                                               my_min, my_max, ia, stg, sign_threshold<R>(iter, tc, mc));
+                                               my_min, my_max, ia, stg, sign_threshold<R>(iter, tc, mc), first);
         else
             coef_phase<R, false, BATCH>(m, U, kact, active, seg_wet, ntiles, cull, mc, sc, nullptr, list, my_min,
                                         my_max, ia);
@@ -640,7 +645,7 @@ __global__ void __launch_bounds__(kBlock, OCC) k_steps(MeshArgs m, StatePair<R> 
         if (STAGED)
             update_phase_staged<R, false, BATCH>(m, ha, U, O, kact, active, seg_clean, seg_wet, seg_vol, seg_dirty,
                                                  ntiles, cull, mc, sc, R(dt), ftr, nullptr, nullptr, nullptr, 0, list,
-                                                 ia, stg);
+                                                 ia, stg, first);
         else
             update_phase<R, false, BATCH>(m, U, O, kact, active, seg_clean, seg_wet, seg_vol, seg_dirty, ntiles, cull,
                                           mc, sc, R(dt), ftr, nullptr, nullptr, nullptr, 0, list, ia);

@@ -79,12 +79,70 @@ struct HaloArgs {
                           // [4][n] more, the derivatives of d h / dx and d h / dy by the neighbours' depths
     uint8_t *fsign;       // [n]: the four friction signs of the sources, two bits each (sign + 1)
     int fast;             // FP64: the mesh and the materials allow quot.cuh's quotients
+    const int *order;     // [ntiles] the order of the tiles (tile_order.cu), null: plain
 };
 
 inline HaloArgs halo_args(const da_ctx *ctx) {
     const bool kact = ctx->ninst > 0 ? ctx->inst_ordinary : kact_ordinary(ctx->mc);
     return HaloArgs{ctx->mesh.halo_off, ctx->mesh.halo_idx, ctx->mesh.nloc,
-                    ctx->slopes,        ctx->fsign,         ctx->mesh.ordinary && kact ? 1 : 0};
+                    ctx->slopes,        ctx->fsign,         ctx->mesh.ordinary && kact ? 1 : 0,
+                    ctx->tile_ordered ? ctx->tile_order : nullptr};
+}
+
+// Which kernels take the tiles in the order of tile_order.cu: those of an ensemble, whose members' flows fall
+// on the same blocks (24 members, 310 wet of 6212 tiles: step 37 -> 31 us, reverse step 92 -> 64 us), and the
+// FP32 ones (13 wet of 1024 tiles: 13.7 -> 12.0 and 24.9 -> 20.7 us).  The FP64 kernels of a single flow have
+// no register left for it: there it cost every step 0.3 us of 11, more than it gives a compact flow.
+template <class R, bool BATCH>
+constexpr bool kOrdered = BATCH || sizeof(R) == 4;
+
+// The tile at entry q of the list (q itself past its end).
+__device__ __forceinline__ int ordered_tile(const HaloArgs &ha, int q, int ntiles) {
+    return ha.order != nullptr && q < ntiles ? ha.order[q] : q;
+}
+
+// A thread's tile of round 0 (and in FP32 that of its first quarter tile) is the same in every phase of a
+// launch and waits in shared memory: read from memory it cost each phase 0.2 us, and so did a register, which
+// spilled.  It is loaded before a launch's restore and stored after it; waited for at its start it cost 3 us.
+template <class R>
+struct FirstTiles {
+    uint16_t tile[kTileCells], quarter[sizeof(R) == 4 ? kTileCells : 1];  // an ordered list has at most 2^16 tiles
+};
+template <class R, bool BATCH>
+struct FirstLoad {
+    int tile = 0, quarter = 0;
+    __device__ __forceinline__ FirstLoad(const HaloArgs &ha, int ntiles) {
+        if constexpr (kOrdered<R, BATCH>) tile = ordered_tile(ha, sched_tile(0), ntiles);
+        if constexpr (sizeof(R) == 4) quarter = ordered_tile(ha, sched_tile(0) >> 2, ntiles);
+    }
+    __device__ __forceinline__ void store(const HaloArgs &ha, FirstTiles<R> &first) const {
+        if constexpr (kOrdered<R, BATCH>) {
+            if (ha.order == nullptr) return;
+            first.tile[threadIdx.x] = uint16_t(min(tile, 0xffff));
+            if constexpr (sizeof(R) == 4) first.quarter[threadIdx.x] = uint16_t(min(quarter, 0xffff));
+        }
+    }
+};
+
+// The thread's tile of a round, and its unit 4 t + quarter of a gather by quarter tiles.
+template <class R, bool BATCH>
+__device__ __forceinline__ int staged_tile(const HaloArgs &ha, int round, const FirstTiles<R> &first, int ntiles) {
+    const int q = sched_tile(round);
+    if constexpr (kOrdered<R, BATCH>) {
+        if (ha.order != nullptr) return round == 0 ? first.tile[threadIdx.x] : ordered_tile(ha, q, ntiles);
+    }
+    return q;
+}
+template <class R, bool BATCH>
+__device__ __forceinline__ int staged_quarter(const HaloArgs &ha, int round, const FirstTiles<R> &first, int ntiles) {
+    const int q = sched_tile(round);
+    if constexpr (sizeof(R) == 4) {
+        if (ha.order != nullptr)
+            return 4 * (round == 0 ? first.quarter[threadIdx.x] : ordered_tile(ha, q >> 2, ntiles)) + (q & 3);
+    } else if constexpr (BATCH) {
+        if (ha.order != nullptr) return 4 * ordered_tile(ha, q >> 2, ntiles) + (q & 3);
+    }
+    return q;
 }
 
 // The staged phases run when the parameters ask for them, the mesh's halo tables exist and the
@@ -587,9 +645,9 @@ __device__ __forceinline__ void coef_phase_staged(const MeshArgs &m, const HaloA
                                                   R *kact, unsigned *active, const uint8_t *seg_wet, int ntiles,
                                                   int cull, const MatConsts &mc0, DevScalars *sc, uint8_t *mask,
                                                   int *list, unsigned long long &my_min, unsigned long long &my_max,
-                                                  const InstArgs &ia, StageSmem<R> &S, R ft) {
+                                                  const InstArgs &ia, StageSmem<R> &S, R ft, const FirstTiles<R> &first) {
     for (int round = 0; sched_more(round, ntiles); ++round) {
-        const int tq = sched_tile(round);
+        const int tq = staged_tile<R, BATCH>(ha, round, first, ntiles);
         const bool need = tq < ntiles && (!cull || seg_flags(seg_wet, tq) != 0ull);
         int ho, hc;
         halo_range(ha, tq, ntiles, ho, hc);
@@ -707,10 +765,10 @@ __device__ __forceinline__ void update_phase_staged(const MeshArgs &m, const Hal
                                                     uint8_t *seg_dirty, int ntiles, int cull, const MatConsts &mc0,
                                                     DevScalars *sc, R dt0, R ft, uint8_t *mask, int *tile_epoch,
                                                     uint8_t *seg_act, int rec_id, int *list, const InstArgs &ia,
-                                                    StageSmem<R> &S, const Epi &epi = Epi{}) {
+                                                    StageSmem<R> &S, const FirstTiles<R> &first, const Epi &epi = Epi{}) {
     const int lane = threadIdx.x & 31;
     for (int round = 0; sched_more(round, ntiles); ++round) {
-        const int tq = sched_tile(round);
+        const int tq = staged_tile<R, BATCH>(ha, round, first, ntiles);
         bool need = false;
         if (tq < ntiles) {
             // the clean flags and the bitmask words of the tile, loaded together
