@@ -186,16 +186,17 @@ def bytes_per_cell_update(precision: str) -> dict:
     arrays of the committed layout (csrc/da_internal.h), r = 8 (FP64) / 4 (FP32-split) bytes per real:
       forward:  state in 3r + state out 3r + g (3), d_gravity (2), curvature (2) 7r + material and
                 boundary flags 2 + neighbour table 4 x int32 16 + cell sizes 2r (+ centres 2 x 8 in
-                FP64, whose slopes take centre differences as the reference does) + the six limited
-                slopes the coefficient phase writes and the update phase reads back 12r
+                FP64, whose slopes take centre differences as the reference does) + what the
+                coefficient phase writes and the update phase reads back: two depth slopes, two
+                velocities, the wave speed 10r and the friction signs 2
       adjoint:  lambda in 3r + U 3r + the same statics, flags, neighbours, sizes (and centres) +
-                branch byte 1 + lambda out 3r
-    FP64: forward 250 B, adjoint 179 B; FP32-split: 126 B and 91 B.  (Without the kept slopes, the
+                branch byte 1 + lambda out 3r + the depth slopes' four derivatives, kept likewise 8r
+    FP64: forward 236 B, adjoint 243 B; FP32-split: 120 B and 123 B.  (Without what is kept, the
     one-pass figures of the path: FP64 154 B, FP32-split 78 B per forward cell-update.)"""
     r = 8 if precision == "fp64" else 4
     xy = 16 if precision == "fp64" else 0
     statics = 7 * r + 2 + 16 + 2 * r + xy
-    return {"forward": 6 * r + statics + 12 * r, "adjoint": 9 * r + statics + 1}
+    return {"forward": 6 * r + statics + 10 * r + 2, "adjoint": 9 * r + statics + 1 + 8 * r}
 
 
 def algorithmic_bytes(precision: str, n_act: float) -> dict:
