@@ -211,19 +211,19 @@ def algorithmic_bytes(precision: str, n_act: float) -> dict:
 
 
 # DRAM bytes (read + write) from the committed ncu captures (the headline traffic and the dense
-# k_steps summaries under profiles/).  Sparse headline kernels: bytes per active cell of a
-# launch captured in the steady flow (k_youturn: reverse steps of iterations 256 and 255 of the
-# 512-step sweep, 4372 and 4344 active cells; k_steps: one launch of 32 steps after 256, 4553
-# active cells per step on average), scaled by the active cells of the traced run; the dense case:
-# bytes per time step of a 10-step launch with every cell wet.
+# k_steps summaries under profiles/).  Sparse headline kernels: bytes per active cell and step of a
+# launch captured in the steady flow (k_youturn, i.e. the launches of reverse steps: one k_reverse_run of
+# the 23 steps of iterations 258 to 236 of the 512-step sweep, 4272 active cells per step on average;
+# k_steps: one launch of 32 steps after 256, 4553 active cells per step on average), scaled by the active
+# cells of the traced run; the dense case: bytes per time step of a 10-step launch with every cell wet.
 TRAFFIC_PER_ACTIVE_CELL = {
-    ("fp64", "k_youturn"): 0.5 * (2206976 / 4372 + 2181632 / 4344),
-    ("fp32", "k_youturn"): 0.5 * (1372672 / 4372 + 1368832 / 4344),
-    ("fp64", "k_steps"): (1511680 + 15104) / (32 * 4552.6),
+    ("fp64", "k_youturn"): (5538048 + 94464) / (23 * 4271.6),
+    ("fp32", "k_youturn"): (3543296 + 55808) / (23 * 4271.1),
+    ("fp64", "k_steps"): (1582848 + 20736) / (32 * 4552.6),
 }
 TRAFFIC_DENSE_PER_STEP = {
-    "fp32": (4.958934e9 + 1.516130e9) / 10,
-    "fp64": (9.034467e9 + 3.031311e9) / 10,
+    "fp32": (5.144700e9 + 1.404057e9) / 10,
+    "fp64": (9.414111e9 + 2.799996e9) / 10,
 }
 
 
