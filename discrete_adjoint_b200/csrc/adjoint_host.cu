@@ -11,7 +11,6 @@
 // the recursion of binomial checkpointing (Griewank's revolve), solved by dynamic programming.
 #include <cuda_runtime.h>
 
-#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -95,9 +94,6 @@ int adj_alloc(da_ctx *ctx, int nsnap) {
     const size_t rs = rsize(ctx);
     int st = DA_OK;
     const int nouts = (ctx->ninst > 0 ? ctx->ninst : 1) * (DA_MAX_MATERIALS + 1 + DA_MAX_PILES);
-    // partial sums: the single instance's, or (n_materials + 2) outputs of every member
-    const size_t nparts = std::max((size_t)kAdjReduceParts * (DA_MAX_MATERIALS + 1 + DA_MAX_PILES),
-                                   (size_t)kAdjInstParts * ctx->ninst * (ctx->p.n_materials + 2));
     if (ctx->adj_n != (int)n || ctx->adj_ninst != ctx->ninst) {
         auto fr = [](void *p) { if (p) cudaFree(p); };
         fr(ctx->mask); fr(ctx->run_flags); fr(ctx->adjA); fr(ctx->adjB); fr(ctx->gbed); fr(ctx->gint); fr(ctx->dk_tab);
@@ -119,7 +115,7 @@ int adj_alloc(da_ctx *ctx, int nsnap) {
         if (!st) st = cuda_check(ctx, cudaMalloc((void **)&ctx->gint, sizeof(double) * n), "cudaMalloc(gint)");
         if (!st) st = cuda_check(ctx, cudaMalloc((void **)&ctx->dk_tab, sizeof(double) * 2 * DA_MAX_MATERIALS * 3), "cudaMalloc");
         if (!st) st = cuda_check(ctx, cudaMalloc((void **)&ctx->red_out, sizeof(double) * nouts), "cudaMalloc");
-        if (!st) st = cuda_check(ctx, cudaMalloc((void **)&ctx->red_part, sizeof(double) * nparts), "cudaMalloc");
+        if (!st) st = cuda_check(ctx, cudaMalloc((void **)&ctx->red_part, sizeof(double) * adj_part_doubles(ctx->ninst)), "cudaMalloc");
         if (!st) st = cuda_check(ctx, cudaMalloc((void **)&ctx->inst_J, sizeof(double) * (ctx->ninst > 0 ? ctx->ninst : 1)), "cudaMalloc");
         if (!st) st = cuda_check(ctx, cudaMalloc((void **)&ctx->seg_J, sizeof(double) * ctx->nseg), "cudaMalloc");
         if (st) return st;

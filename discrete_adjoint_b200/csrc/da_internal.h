@@ -35,6 +35,14 @@ struct MatConsts {
 constexpr int kAdjReduceParts = 128;  // cell ranges of the gradient reduction
 constexpr int kAdjInstParts = 32;     // the same of each ensemble member
 
+// Doubles of the reduction's partial sums: a single instance's, or n_materials + 2 outputs of every
+// member, by the most materials that da_set_params can give a context (the buffer outlives the call).
+constexpr size_t adj_part_doubles(int ninst) {
+    const size_t single = (size_t)kAdjReduceParts * (DA_MAX_MATERIALS + 1 + DA_MAX_PILES);
+    const size_t members = (size_t)kAdjInstParts * (ninst > 0 ? ninst : 0) * (DA_MAX_MATERIALS + 2);
+    return single > members ? single : members;
+}
+
 struct DevScalars {
     double time;          // TimeProps::time
     double dt;            // last dt
