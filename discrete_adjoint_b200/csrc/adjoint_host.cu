@@ -714,8 +714,10 @@ int da_adjoint_run_dwr(da_ctx *ctx, const da_functional *f, int32_t nsteps, int3
     int st = cuda_check(ctx, cudaStreamSynchronize(ctx->stream), "sync");
     if (!st) st = copy_d2h(ctx, ctx->hsc, ctx->dsc, sizeof(DevScalars), "read scalars");
     const long long iter_begin = ctx->hsc->iter;
+    if (!st) st = dwr_clear_error(ctx);
     if (!st) st = dwr_accumulators(ctx, nsteps);
     if (!st) st = adjoint_run_impl(ctx, f, nsteps, nsnapshots, dh0_dpile, n_piles, out, lambda0, &iter_begin);
+    if (!st) st = dwr_error(ctx, "da_adjoint_run_dwr");
     if (!st) st = copy_d2h(ctx, cell_error, ctx->dwr.acc, sizeof(double) * n, "copy dwr cells");
     if (!st) st = copy_d2h(ctx, step_sums, ctx->dwr.step_sums, sizeof(double) * 2 * (size_t)nsteps, "copy dwr sums");
     return st;

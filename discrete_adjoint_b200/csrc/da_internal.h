@@ -61,6 +61,7 @@ struct DevScalars {
     unsigned long long bar;       // grid barrier of the cooperative kernels: arrivals since the launch
                                   // began (barrier k of a grid of G blocks opens at G (k + 1))
     unsigned long long bar_exit;  // blocks that have left the launch; the last one restarts both at 0
+    int dwr_err;          // first DA_ERR_* of the error grid's steps since the host cleared it (dwr.cu)
 };
 
 // Time-clipping targets (TimeProps::ndnextoutput / ndnextsave / ndmaxtime) and the
@@ -346,7 +347,10 @@ int copy_lambda_out(da_ctx *ctx, int buf, double *host);
 // dwr.cu: the indicator of the step U[un] -> U[unext] with adjoint lam[lam], queued on the stream after
 // the kernel that made the step (iter0 the iteration before it; its dt and time are read from the
 // device scalars): the totals into out[2] (device), the estimate per coarse cell added to acc (or null);
-// the accumulators of a sweep; release of the error grid
+// the accumulators of a sweep; the error grid's error of the last sweep or step, from hsc (dwr_clear_error
+// before it, with hsc just read); release of the error grid
+int dwr_clear_error(da_ctx *ctx);
+int dwr_error(da_ctx *ctx, const char *where);
 int dwr_indicator(da_ctx *ctx, int un, int unext, int lam, long long iter0, double *acc, double *out);
 int dwr_accumulators(da_ctx *ctx, int nsteps);
 void dwr_release(da_ctx *ctx);

@@ -16,6 +16,9 @@
 // the reverse sweep's indicator steps queue up behind its kernels (three launches a step; with a
 // host round trip for dt, iteration and totals, a dt array allocated and freed and the sums' 256 parts
 // added by one thread, a step of 10k coarse cells took 210 us).
+// An error that the error grid's step raises (a barrier wait that ran out, a state that is not finite, a
+// wave speed above the bound) is carried into the coarse scalars, where the end of the sweep or step reads
+// it; the next indicator step starts without it.
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -42,16 +45,22 @@ __global__ void __launch_bounds__(kBlock) k_dwr_interp(int nf, const int32_t *__
                                                        Fields<R> lam, R *fh, R *fhu, R *fhv,
                                                        double *__restrict__ ut_next, double *__restrict__ lamt,
                                                        uint8_t *__restrict__ seg_clean, uint8_t *__restrict__ seg_wet,
-                                                       int nseg, const DevScalars *__restrict__ coarse,
+                                                       unsigned *__restrict__ active, int nseg,
+                                                       const DevScalars *__restrict__ coarse,
                                                        DevScalars *__restrict__ fine) {
-    // the error grid's state is new everywhere, its time that of the step's beginning
+    // the error grid's state is new everywhere, its time that of the step's beginning; nothing of a
+    // step that did not end is left (no kernel of the error grid runs beside this one)
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < nseg; s += gridDim.x * blockDim.x) {
         seg_clean[s] = 0;
         seg_wet[s] = 1;
+        active[s] = 0u;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         fine->time = coarse->time - coarse->dt;  // enters the step only through clipping, which the replay skips
         fine->iter = coarse->iter - 1;
+        fine->err = 0;
+        fine->bar = 0ull;
+        fine->bar_exit = 0ull;
     }
     for (int f = blockIdx.x * blockDim.x + threadIdx.x; f < nf; f += gridDim.x * blockDim.x) {
         double a[3] = {0, 0, 0}, b[3] = {0, 0, 0}, c[3] = {0, 0, 0};
@@ -119,7 +128,8 @@ __global__ void __launch_bounds__(kBlock) k_dwr_residual(int n, int nf, const in
                                                          const double *__restrict__ lamt, Fields<R> lam,
                                                          double *__restrict__ err, double *__restrict__ cell,
                                                          double *__restrict__ acc, double *parts, unsigned *done,
-                                                         double *__restrict__ out) {
+                                                         double *__restrict__ out, const DevScalars *__restrict__ fine,
+                                                         DevScalars *__restrict__ coarse) {
     __shared__ double red[kBlock / 32][2];
     __shared__ bool last;
     const int per = (n + kParts - 1) / kParts;
@@ -171,6 +181,7 @@ __global__ void __launch_bounds__(kBlock) k_dwr_residual(int n, int nf, const in
         out[0] = es + ec;
         out[1] = cs + cc;
         *done = 0u;
+        if (fine->err != 0 && coarse->dwr_err == 0) coarse->dwr_err = fine->err;
     }
 }
 
@@ -187,7 +198,8 @@ int run_t(da_ctx *ctx, DwrState &d, int un, int unext, int lam, long long iter0,
     k_dwr_interp<R><<<grid, kBlock, 0, ctx->stream>>>(nf, d.interp, d.weight, fields<R>(ctx->U[un]),
                                                       fields<R>(ctx->U[unext]), fields<R>(ctx->lam[lam]),
                                                       (R *)fc->U[0][0], (R *)fc->U[0][1], (R *)fc->U[0][2], d.ut_next,
-                                                      d.lamt, fc->seg_clean, fc->seg_wet, fc->nseg, ctx->dsc, fc->dsc);
+                                                      d.lamt, fc->seg_clean, fc->seg_wet, fc->active, fc->nseg, ctx->dsc,
+                                                      fc->dsc);
     int st = cuda_check(ctx, cudaGetLastError(), "dwr interpolation");
     fc->have_state = true;
     // one step of the error grid from U~^n with the coarse dt, read where the coarse step left it
@@ -201,7 +213,7 @@ int run_t(da_ctx *ctx, DwrState &d, int un, int unext, int lam, long long iter0,
     if (!st) {
         k_dwr_residual<R><<<kParts, kBlock, 0, ctx->stream>>>(ctx->mesh.n, nf, d.children, fields<R>(fc->U[fc->cur]),
                                                               d.ut_next, d.lamt, fields<R>(ctx->lam[lam]), d.err, d.cell,
-                                                              acc, d.parts, d.done, out);
+                                                              acc, d.parts, d.done, out, fc->dsc, ctx->dsc);
         st = cuda_check(ctx, cudaGetLastError(), "dwr residual");
     }
     return st;
@@ -238,6 +250,16 @@ void dwr_release(da_ctx *ctx) { free_dwr(ctx); }
 int dwr_indicator(da_ctx *ctx, int un, int unext, int lam, long long iter0, double *acc, double *out) {
     return ctx->p.precision == DA_PREC_FP64 ? run_t<double>(ctx, ctx->dwr, un, unext, lam, iter0, acc, out)
                                             : run_t<float>(ctx, ctx->dwr, un, unext, lam, iter0, acc, out);
+}
+
+int dwr_clear_error(da_ctx *ctx) {
+    if (ctx->hsc->dwr_err == 0) return DA_OK;
+    return cuda_check(ctx, cudaMemsetAsync(&ctx->dsc->dwr_err, 0, sizeof(int), ctx->stream), "memset");
+}
+
+int dwr_error(da_ctx *ctx, const char *where) {
+    const int code = ctx->hsc->dwr_err;
+    return code ? set_error(ctx, code, std::string(where) + ": the error grid's step: " + da_strerror(code)) : DA_OK;
 }
 
 int dwr_accumulators(da_ctx *ctx, int nsteps) {
@@ -338,13 +360,15 @@ int da_dwr_step(da_ctx *ctx, const double *lambda_next, double *el_error, double
     // the coarse step n -> n+1 from a base checkpoint, put back afterwards
     if (!st) st = launch_snapshot(ctx, ctx->snaps[0], true);
     if (!st) st = read_scalars(ctx);
+    if (!st) st = dwr_clear_error(ctx);
     const long long iter0 = ctx->hsc->iter;
     if (!st) st = launch_single_step(ctx);
     if (!st) st = read_scalars(ctx);
     if (!st) st = device_error(ctx, "da_dwr_step: the coarse step");
     if (!st) st = dwr_indicator(ctx, 1 - ctx->cur, ctx->cur, 0, iter0, nullptr, ctx->dwr.sums);
     if (!st) st = launch_snapshot(ctx, ctx->snaps[0], false);
-    if (!st) st = cuda_check(ctx, cudaStreamSynchronize(ctx->stream), "sync");
+    if (!st) st = read_scalars(ctx);
+    if (!st) st = dwr_error(ctx, "da_dwr_step");
     const int nf = ctx->dwr.nf;
     if (!st && el_error) st = copy_d2h(ctx, el_error, ctx->dwr.err, 8 * (size_t)nf, "copy");
     if (!st && cell_error) st = copy_d2h(ctx, cell_error, ctx->dwr.cell, 8 * n, "copy");

@@ -349,7 +349,9 @@ int da_refine_info(da_ctx *ctx, double *el_error, uint8_t *flags, double *geo_ta
  * da_dwr_step evaluates the indicator of the step from the context's current state U^n, with
  * lambda_next = dJ/dU^{n+1} (host [3][n]); the coarse step is taken and undone.  Outputs
  * (optional): el_error per fine cell [nf], its sum over each coarse cell's children [n], and
- * sums[2] = total el_error and total correction (compensated FP64 sums in a fixed order). */
+ * sums[2] = total el_error and total correction (compensated FP64 sums in a fixed order).  An error
+ * that the step of the refined grid raises is the status of the call (here and in
+ * da_adjoint_run_dwr); the context itself stays as it was. */
 int da_dwr_setup(da_ctx *ctx, const da_mesh_soa *fine, const int32_t *parent, const int32_t *interp,
                  const double *weight);
 int da_dwr_step(da_ctx *ctx, const double *lambda_next, double *el_error, double *cell_error, double *sums);
