@@ -230,7 +230,7 @@ void free_dwr(da_ctx *ctx) {
     DwrState &d = ctx->dwr;
     if (d.fine) {
         if (ctx->stream) cudaStreamSynchronize(ctx->stream);
-        d.fine->stream = d.fine_stream;  // its own again
+        if (d.fine_stream) d.fine->stream = d.fine_stream;  // its own again
         da_destroy(d.fine);
         // a captured sweep may hold launches on the error grid
         if (ctx->sweep_graph) cudaGraphExecDestroy(ctx->sweep_graph);

@@ -52,3 +52,21 @@ def test_error_of_the_error_grid_is_reported_and_does_not_last():
             for a, b in zip(got, ref):
                 assert np.array_equal(a, b)
             assert np.array_equal(run.dwr_cell, ref_run.dwr_cell) and np.array_equal(run.dwr_steps, ref_run.dwr_steps)
+
+
+def test_failed_setups_leave_nothing_behind():
+    # the error grid's context, its stream included, goes with a setup that fails in the mesh's checks: a
+    # stream left behind takes half a megabyte of device memory
+    import torch
+    w = inputs.test_case(seed=1)
+    g = error_grid(w)
+    g.fine.material[0] = 99
+    g.fine._soa = None
+    with GeoflowContext(w.mat, TimeProps()) as c:
+        c.upload_mesh(w.mesh)
+        free = []
+        for k in range(102):
+            with pytest.raises(_ffi.DAError):
+                Indicator(c, g)
+            free.append(torch.cuda.mem_get_info()[0])
+        assert free[1] - free[-1] < 8 << 20
