@@ -187,13 +187,11 @@ struct Runner {
     // (U^n, U^{n+1} and lambda^{n+1} all resident) the indicator of that step, as the reference's
     // dual_solver calls error_compute after each adjoint step (dual_solver.C:206-230).
     bool dwr = false;
-    long long iter_begin = 0;  // iteration of U^0
-    int left = 0;              // reverse steps still to come
+    int left = 0;  // reverse steps still to come
     int dwr_step() {
         --left;
         if (!dwr) return DA_OK;
-        return dwr_indicator(ctx, ctx->cur ^ 1, ctx->cur, lam_cur, iter_begin + left, ctx->dwr.acc,
-                             ctx->dwr.step_sums + 2 * (size_t)left);
+        return dwr_indicator(ctx, ctx->cur ^ 1, ctx->cur, lam_cur, ctx->dwr.acc, ctx->dwr.step_sums + 2 * (size_t)left);
     }
     Schedule sch;
     std::vector<int> free_slots;
@@ -470,17 +468,19 @@ std::vector<unsigned char> sweep_key(const da_ctx *ctx, const double *box, int n
 // over nsteps steps from the current state, reverse steps back to step 0, the state put back,
 // J and the gradient sums launched (single: red_out[n_mat + 1 + n_piles]; ensemble: per member).
 // lam0 receives the buffer that holds lambda^0.
-// Without tracing, the sweep's thousand or so launches (the DWR indicator's among them) are captured once as a CUDA graph and replayed while nothing
-// they depend on changes: a graph starts its cooperative kernels back to back, without the few
-// microseconds of idle GPU between stream launches.  The recording ids the capture gave the
-// reverse steps repeat on a replay, so the graph first clears the tiles' recording ids.
+// Without tracing, the sweep's thousand or so launches (the DWR indicator's among them) are captured once
+// as a CUDA graph and replayed while nothing they depend on changes: a graph starts its cooperative
+// kernels back to back, without the few microseconds of idle GPU between stream launches.  A sweep with
+// the indicator has a graph of its own beside the plain one's, so that a program which takes both in
+// turn captures each once; time and iteration are read on the device and are not part of the key.
+// The recording ids the capture gave the reverse steps repeat on a replay, so the graph first clears the
+// tiles' recording ids.
 int adjoint_sweep(da_ctx *ctx, const double *box, int32_t nsteps, int32_t nsnapshots, int32_t n_piles, int *lam0,
-                  long long *fsteps, float *dev_ms, const long long *dwr_iter0, const double *lambda_end) {
+                  long long *fsteps, float *dev_ms, bool dwr, const double *lambda_end) {
     int st = adj_alloc(ctx, nsnapshots + 1);
     Runner r;
     r.ctx = ctx;
-    r.dwr = dwr_iter0 != nullptr;
-    r.iter_begin = r.dwr ? *dwr_iter0 : 0;
+    r.dwr = dwr;
     r.left = nsteps;
     if (box)
         for (int q = 0; q < 4; ++q) r.box[q] = box[q];
@@ -519,16 +519,14 @@ int adjoint_sweep(da_ctx *ctx, const double *box, int32_t nsteps, int32_t nsnaps
         return s;
     };
     bool graph = !ctx->trace.on && ctx->p.jacobian_mode == DA_JAC_EXACT;
+    SweepGraph &sg = ctx->sweeps[r.dwr ? 1 : 0];
     if (graph) {
         std::vector<unsigned char> key = sweep_key(ctx, box, nsteps, nsnapshots, n_piles, r.seeded, r.sec2, r.cos_int);
         // the error grid's own tables are fixed until it is released, which drops the graph
-        const long long dwr_key[4] = {r.dwr, r.iter_begin, (long long)(uintptr_t)(r.dwr ? ctx->dwr.acc : nullptr),
-                                      (long long)(uintptr_t)(r.dwr ? ctx->dwr.step_sums : nullptr)};
-        key.insert(key.end(), (const unsigned char *)dwr_key, (const unsigned char *)(dwr_key + 4));
-        if (!ctx->sweep_graph || key != ctx->sweep_key) {
-            if (ctx->sweep_graph) cudaGraphExecDestroy(ctx->sweep_graph);
-            ctx->sweep_graph = nullptr;
-            ctx->sweep_key.clear();
+        const void *dwr_key[2] = {r.dwr ? ctx->dwr.acc : nullptr, r.dwr ? ctx->dwr.step_sums : nullptr};
+        key.insert(key.end(), (const unsigned char *)dwr_key, (const unsigned char *)(dwr_key + 2));
+        if (!sg.exec || key != sg.key) {
+            sg.drop();
             // capture: nothing runs; the host-side state the launches leave is kept for replays
             const Runner r0 = r;
             const int cur0 = ctx->cur;
@@ -542,16 +540,15 @@ int adjoint_sweep(da_ctx *ctx, const double *box, int32_t nsteps, int32_t nsnaps
                 const cudaError_t e = cudaStreamEndCapture(ctx->stream, &g);
                 s = s2 ? s2 : cuda_check(ctx, e, "end capture");
             }
-            if (!s) s = cuda_check(ctx, cudaGraphInstantiate(&ctx->sweep_graph, g, 0), "instantiate");
+            if (!s) s = cuda_check(ctx, cudaGraphInstantiate(&sg.exec, g, 0), "instantiate");
             if (g) cudaGraphDestroy(g);
             if (!s) {
-                ctx->sweep_key = key;
-                ctx->sweep_lam = r.lam_cur;
-                ctx->sweep_fsteps = r.fsteps;
+                sg.key = key;
+                sg.lam = r.lam_cur;
+                sg.fsteps = r.fsteps;
             } else {
                 // the launches one by one instead
-                if (ctx->sweep_graph) cudaGraphExecDestroy(ctx->sweep_graph);
-                ctx->sweep_graph = nullptr;
+                sg.drop();
                 cudaGetLastError();
                 ctx->err.clear();
                 graph = false;
@@ -566,9 +563,9 @@ int adjoint_sweep(da_ctx *ctx, const double *box, int32_t nsteps, int32_t nsnaps
     cudaEventRecord(e0, ctx->stream);
     if (graph) {
         // the gradient sums are in the timed region
-        st = cuda_check(ctx, cudaGraphLaunch(ctx->sweep_graph, ctx->stream), "sweep graph launch");
-        r.lam_cur = ctx->sweep_lam;
-        r.fsteps = ctx->sweep_fsteps;
+        st = cuda_check(ctx, cudaGraphLaunch(sg.exec, ctx->stream), "sweep graph launch");
+        r.lam_cur = sg.lam;
+        r.fsteps = sg.fsteps;
     } else {
         st = sweep();
     }
@@ -648,7 +645,7 @@ int da_adjoint_step(da_ctx *ctx, const double *lambda_next, double *lambda_out, 
 namespace {
 
 int adjoint_run_impl(da_ctx *ctx, const da_functional *f, int32_t nsteps, int32_t nsnapshots, const double *dh0_dpile,
-                     int32_t n_piles, da_gradient *out, double *lambda0, const long long *dwr,
+                     int32_t n_piles, da_gradient *out, double *lambda0, bool dwr,
                      const double *lambda_end = nullptr) {
     if (!ctx || (!f && !lambda_end) || nsteps <= 0 || nsnapshots < 0 || n_piles < 0 || n_piles > DA_MAX_PILES ||
         (n_piles > 0 && !dh0_dpile) || (f && f->kind != DA_FUNC_H2_BOX))
@@ -693,13 +690,13 @@ extern "C" {
 
 int da_adjoint_run(da_ctx *ctx, const da_functional *f, int32_t nsteps, int32_t nsnapshots, const double *dh0_dpile,
                    int32_t n_piles, da_gradient *out, double *lambda0) {
-    return adjoint_run_impl(ctx, f, nsteps, nsnapshots, dh0_dpile, n_piles, out, lambda0, nullptr);
+    return adjoint_run_impl(ctx, f, nsteps, nsnapshots, dh0_dpile, n_piles, out, lambda0, false);
 }
 
 int da_adjoint_run_seeded(da_ctx *ctx, const double *lambda_end, int32_t nsteps, int32_t nsnapshots,
                           const double *dh0_dpile, int32_t n_piles, da_gradient *out, double *lambda0) {
     if (!lambda_end) return DA_ERR_INVALID;
-    return adjoint_run_impl(ctx, nullptr, nsteps, nsnapshots, dh0_dpile, n_piles, out, lambda0, nullptr, lambda_end);
+    return adjoint_run_impl(ctx, nullptr, nsteps, nsnapshots, dh0_dpile, n_piles, out, lambda0, false, lambda_end);
 }
 
 int da_adjoint_run_dwr(da_ctx *ctx, const da_functional *f, int32_t nsteps, int32_t nsnapshots,
@@ -713,10 +710,9 @@ int da_adjoint_run_dwr(da_ctx *ctx, const da_functional *f, int32_t nsteps, int3
     for (int k = 0; k < 2 * nsteps; ++k) step_sums[k] = 0.0;
     int st = cuda_check(ctx, cudaStreamSynchronize(ctx->stream), "sync");
     if (!st) st = copy_d2h(ctx, ctx->hsc, ctx->dsc, sizeof(DevScalars), "read scalars");
-    const long long iter_begin = ctx->hsc->iter;
     if (!st) st = dwr_clear_error(ctx);
     if (!st) st = dwr_accumulators(ctx, nsteps);
-    if (!st) st = adjoint_run_impl(ctx, f, nsteps, nsnapshots, dh0_dpile, n_piles, out, lambda0, &iter_begin);
+    if (!st) st = adjoint_run_impl(ctx, f, nsteps, nsnapshots, dh0_dpile, n_piles, out, lambda0, true);
     if (!st) st = dwr_error(ctx, "da_adjoint_run_dwr");
     if (!st) st = copy_d2h(ctx, cell_error, ctx->dwr.acc, sizeof(double) * n, "copy dwr cells");
     if (!st) st = copy_d2h(ctx, step_sums, ctx->dwr.step_sums, sizeof(double) * 2 * (size_t)nsteps, "copy dwr sums");

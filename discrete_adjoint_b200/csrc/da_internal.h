@@ -66,6 +66,7 @@ struct DevScalars {
 
 // Time-clipping targets (TimeProps::ndnextoutput / ndnextsave / ndmaxtime) and the
 // frict_tiny schedule (hpfem.C:232-235), passed by value to the dt kernel.
+constexpr long long kReplayOne = -1;
 struct TimeConsts {
     double next_output, next_save, max_time, influx_dt;
     double gravity_scale, epsilon;
@@ -73,7 +74,7 @@ struct TimeConsts {
     long long frict_tiny_iters;
     const double *dt_replay;  // when set, step k takes dt_replay[k - iter0] instead of the CFL dt
     long long iter0;
-    long long n_replay;
+    long long n_replay;       // kReplayOne: every step takes *dt_replay
 };
 
 // Ensemble (batched) mode: the mesh is the members' meshes one after another, each padded to
@@ -101,6 +102,20 @@ struct OutlineGrid {
     int nx = 0, ny = 0;
     double x0 = 0, y0 = 0, dx = 0, dy = 0;
     unsigned long long *map = nullptr;  // [ny][nx]
+};
+
+// A reverse sweep's launches captured as a CUDA graph (adjoint_host.cu), with the inputs its kernels were
+// given (key) and the host-side results of building it.
+struct SweepGraph {
+    cudaGraphExec_t exec = nullptr;
+    std::vector<unsigned char> key;
+    int lam = 0;
+    long long fsteps = 0;
+    void drop() {
+        if (exec) cudaGraphExecDestroy(exec);
+        exec = nullptr;
+        key.clear();
+    }
 };
 
 // Dual-weighted-residual indicator: the error grid's own context and the device tables (dwr.cu).
@@ -252,12 +267,7 @@ struct da_ctx {
     std::vector<int> sched_split;
     int sched_n = -1, sched_c = -1;
     std::vector<void *> snaps;       // checkpoint slots, 3 state arrays each
-    // the reverse sweep's launches captured as a CUDA graph (adjoint_host.cu), with the inputs its
-    // kernels were given (sweep_key) and the host-side results of building it
-    cudaGraphExec_t sweep_graph = nullptr;
-    std::vector<unsigned char> sweep_key;
-    int sweep_lam = 0;
-    long long sweep_fsteps = 0;
+    da::SweepGraph sweeps[2];        // the reverse sweep without and with the DWR indicator
     double *dt_replay = nullptr;     // device copy of a frozen time-step sequence
     void *refadj_mem = nullptr;      // workspace of the reference-mode adjoint (adjoint_ref.cu)
     int refadj_n = 0;                // the mesh size it was allocated for
@@ -337,21 +347,19 @@ int forward_state_changed(da_ctx *ctx);
 // adjoint_host.cu: d kact / d phi_bed and d phi_int of each material's three branches
 void kact_derivatives(const da_params &p, double *dkb, double *dki);
 // adjoint_host.cu: the checkpointed reverse sweep (see there)
-// dwr_iter0 (or null): also the DWR indicator of every reverse step, into the context's accumulators,
-// iteration *dwr_iter0 at the beginning
+// dwr: also the DWR indicator of every reverse step, into the context's accumulators
 // lambda_end (or null): lambda^N given instead of the functional's seed (host [3][n])
 int adjoint_sweep(da_ctx *ctx, const double *box, int32_t nsteps, int32_t nsnapshots, int32_t n_piles, int *lam0,
-                  long long *fsteps, float *dev_ms, const long long *dwr_iter0 = nullptr,
+                  long long *fsteps, float *dev_ms, bool dwr = false,
                   const double *lambda_end = nullptr);
 int copy_lambda_out(da_ctx *ctx, int buf, double *host);
 // dwr.cu: the indicator of the step U[un] -> U[unext] with adjoint lam[lam], queued on the stream after
-// the kernel that made the step (iter0 the iteration before it; its dt and time are read from the
-// device scalars): the totals into out[2] (device), the estimate per coarse cell added to acc (or null);
+// the kernel that made the step (its dt, time and iteration are read from the device scalars): the totals into out[2] (device), the estimate per coarse cell added to acc (or null);
 // the accumulators of a sweep; the error grid's error of the last sweep or step, from hsc (dwr_clear_error
 // before it, with hsc just read); release of the error grid
 int dwr_clear_error(da_ctx *ctx);
 int dwr_error(da_ctx *ctx, const char *where);
-int dwr_indicator(da_ctx *ctx, int un, int unext, int lam, long long iter0, double *acc, double *out);
+int dwr_indicator(da_ctx *ctx, int un, int unext, int lam, double *acc, double *out);
 int dwr_accumulators(da_ctx *ctx, int nsteps);
 void dwr_release(da_ctx *ctx);
 // adjoint_host.cu: adjoint buffers and one checkpoint slot

@@ -191,7 +191,7 @@ Fields<R> fields(void *const U[3]) {
 }
 
 template <class R>
-int run_t(da_ctx *ctx, DwrState &d, int un, int unext, int lam, long long iter0, double *acc, double *out) {
+int run_t(da_ctx *ctx, DwrState &d, int un, int unext, int lam, double *acc, double *out) {
     da_ctx *fc = d.fine;
     const int nf = fc->mesh.n, grid = (ctx->sm_count > 0 ? ctx->sm_count : 148) * 8;
     fc->cur = 0;  // every indicator step uses the same buffers
@@ -204,8 +204,7 @@ int run_t(da_ctx *ctx, DwrState &d, int un, int unext, int lam, long long iter0,
     fc->have_state = true;
     // one step of the error grid from U~^n with the coarse dt, read where the coarse step left it
     fc->tc.dt_replay = &ctx->dsc->dt;
-    fc->tc.iter0 = iter0;
-    fc->tc.n_replay = 1;
+    fc->tc.n_replay = kReplayOne;
     if (!st) {
         st = launch_single_step(fc);
         if (st) set_error(ctx, st, std::string("dwr step of the error grid: ") + da_last_error(fc));
@@ -232,10 +231,7 @@ void free_dwr(da_ctx *ctx) {
         if (ctx->stream) cudaStreamSynchronize(ctx->stream);
         if (d.fine_stream) d.fine->stream = d.fine_stream;  // its own again
         da_destroy(d.fine);
-        // a captured sweep may hold launches on the error grid
-        if (ctx->sweep_graph) cudaGraphExecDestroy(ctx->sweep_graph);
-        ctx->sweep_graph = nullptr;
-        ctx->sweep_key.clear();
+        ctx->sweeps[1].drop();  // it holds launches on the error grid
     }
     if (d.mem) cudaFree(d.mem);
     if (d.acc) cudaFree(d.acc);
@@ -247,9 +243,9 @@ void free_dwr(da_ctx *ctx) {
 
 void dwr_release(da_ctx *ctx) { free_dwr(ctx); }
 
-int dwr_indicator(da_ctx *ctx, int un, int unext, int lam, long long iter0, double *acc, double *out) {
-    return ctx->p.precision == DA_PREC_FP64 ? run_t<double>(ctx, ctx->dwr, un, unext, lam, iter0, acc, out)
-                                            : run_t<float>(ctx, ctx->dwr, un, unext, lam, iter0, acc, out);
+int dwr_indicator(da_ctx *ctx, int un, int unext, int lam, double *acc, double *out) {
+    return ctx->p.precision == DA_PREC_FP64 ? run_t<double>(ctx, ctx->dwr, un, unext, lam, acc, out)
+                                            : run_t<float>(ctx, ctx->dwr, un, unext, lam, acc, out);
 }
 
 int dwr_clear_error(da_ctx *ctx) {
@@ -361,11 +357,10 @@ int da_dwr_step(da_ctx *ctx, const double *lambda_next, double *el_error, double
     if (!st) st = launch_snapshot(ctx, ctx->snaps[0], true);
     if (!st) st = read_scalars(ctx);
     if (!st) st = dwr_clear_error(ctx);
-    const long long iter0 = ctx->hsc->iter;
     if (!st) st = launch_single_step(ctx);
     if (!st) st = read_scalars(ctx);
     if (!st) st = device_error(ctx, "da_dwr_step: the coarse step");
-    if (!st) st = dwr_indicator(ctx, 1 - ctx->cur, ctx->cur, 0, iter0, nullptr, ctx->dwr.sums);
+    if (!st) st = dwr_indicator(ctx, 1 - ctx->cur, ctx->cur, 0, nullptr, ctx->dwr.sums);
     if (!st) st = launch_snapshot(ctx, ctx->snaps[0], false);
     if (!st) st = read_scalars(ctx);
     if (!st) st = dwr_error(ctx, "da_dwr_step");

@@ -56,7 +56,7 @@ __device__ __forceinline__ void step_dt(double min_dxe, double hmax, double time
     if (tc.dt_replay) {
         // frozen time-step sequence (tangent/finite-difference checks of the adjoint)
         const long long k = iter - tc.iter0;
-        dt = (k >= 0 && k < tc.n_replay) ? tc.dt_replay[k] : 0.0;
+        dt = tc.n_replay == kReplayOne ? *tc.dt_replay : (k >= 0 && k < tc.n_replay) ? tc.dt_replay[k] : 0.0;
     }
     dt_out = dt;
     ft_out = iter < tc.frict_tiny_iters ? tc.frict_tiny_early : tc.frict_tiny_late;
