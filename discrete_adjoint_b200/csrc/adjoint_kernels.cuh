@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(kBlock, OCC) k_youturn(MeshArgs m, fwd::StateP
         // the source adjoint of each wet cell right after its update, from the tile and halo
         // staged for it (its own branches and lambda^{n+1}, U^n around it: nothing another cell
         // writes in this phase), so the reverse step needs no source phase of its own
-        const SrcEpilogue<R, BATCH> src{m, Ln, mc, aa, ia, R(dt), (const R *)ha.kept};
+        const SrcEpilogue<R, BATCH> src{m, Ln, mc, aa, ia, R(dt)};
         fwd::update_phase_staged<R, true, BATCH>(m, ha, U, O, kact, active, seg_clean, seg_wet, seg_vol, seg_dirty,
                                                  ntiles, cull, mc, sc, R(dt), ftr, mask, tile_epoch, seg_act, rec_id,
                                                  list, ia, stg, first, src);
@@ -369,7 +369,7 @@ __global__ void __launch_bounds__(kBlock, OCC) k_reverse_run(MeshArgs m, fwd::St
             *(k & 1 ? &sc->acc_min_dxe : &sc->acc_alt_min_dxe) = fwd::kMinDxeStart;
             *(k & 1 ? &sc->acc_hmax : &sc->acc_alt_hmax) = 0ull;
         }
-        const SrcEpilogue<R, false> src{m, Ln, mc, aa, InstArgs{}, R(dt), (const R *)ha.kept};
+        const SrcEpilogue<R, false> src{m, Ln, mc, aa, InstArgs{}, R(dt)};
         fwd::update_phase_staged<R, true, false, false>(m, ha, U, StateOut<R>{}, kact, active, nullptr, nullptr, nullptr,
                                                         nullptr, ntiles, cull, mc, sc, R(dt), ftr, mask, tile_epoch,
                                                         seg_act, rec_id, list, InstArgs{}, stg, first, src);

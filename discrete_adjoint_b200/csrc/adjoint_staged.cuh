@@ -329,7 +329,6 @@ struct SrcEpilogue {
     const AdjArgs &aa;
     const InstArgs &ia;
     R dt;
-    const R *kept;  // HaloArgs::kept
     struct Pre {
         R l[3];
         R q[4];  // the slope derivatives the recording coefficient phase left
@@ -341,7 +340,7 @@ struct SrcEpilogue {
             p.l[1] = Ln.hu[i];
             p.l[2] = Ln.hv[i];
 #pragma unroll
-            for (int s = 0; s < 4; ++s) p.q[s] = kept[(size_t)(5 + s) * m.n + i];
+            for (int s = 0; s < 4; ++s) p.q[s] = *fwd::kept_deriv<R>(aa.B, s, m.n, i);
         }
         return p;
     }

@@ -198,7 +198,7 @@ struct da_ctx {
     int cur = 0;
     void *kact = nullptr;            // [n] Real
     // what the staged coefficient phase keeps of each wet cell for the update phase (staged_impl.cuh):
-    // [9][n] (depth slopes, velocities, wave speed, the depth slopes' derivatives) and the friction signs
+    // [5][n] (depth slopes, velocities, wave speed) and the friction signs
     void *slopes = nullptr;
     uint8_t *fsign = nullptr;        // [n] friction signs
     // segments: 32 consecutive cells (one warp), 8 per tile; arrays padded to whole tiles

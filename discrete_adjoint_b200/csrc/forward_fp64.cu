@@ -56,7 +56,7 @@ int forward_alloc(da_ctx *ctx) {
             if (!st) st = cuda_check(ctx, cudaMemsetAsync(ctx->U[b][v], 0, rs * n, ctx->stream), "memset");
         }
     if (!st) st = cuda_check(ctx, cudaMalloc(&ctx->kact, rs * n), "cudaMalloc(kact)");
-    if (!st) st = cuda_check(ctx, cudaMalloc(&ctx->slopes, 9 * rs * n), "cudaMalloc(slopes)");
+    if (!st) st = cuda_check(ctx, cudaMalloc(&ctx->slopes, 5 * rs * n), "cudaMalloc(slopes)");
     if (!st) st = cuda_check(ctx, cudaMalloc((void **)&ctx->fsign, n), "cudaMalloc(signs)");
     if (!st) st = cuda_check(ctx, cudaMalloc((void **)&ctx->seg_wet, nseg), "cudaMalloc(seg_wet)");
     if (!st) st = cuda_check(ctx, cudaMalloc((void **)&ctx->tile_order, sizeof(int) * ctx->ntiles), "cudaMalloc(order)");

@@ -75,9 +75,11 @@ struct HaloArgs {
     const int32_t *idx;   // halo cells, tile after tile
     const int16_t *nloc;  // [n][8] tile-local neighbour slots
     // written by the coefficient phase for each wet cell and read by the same step's update phase:
-    void *kept;           // [5][n]: d h / dx, d h / dy, hu / h, hv / h, sqrt(k h g_z), and when recording
-                          // [4][n] more, the derivatives of d h / dx and d h / dy by the neighbours' depths
+    void *kept;           // [5][n]: d h / dx, d h / dy, hu / h, hv / h, sqrt(k h g_z)
     uint8_t *fsign;       // [n]: the four friction signs of the sources, two bits each (sign + 1)
+    double *deriv;        // [4][n]: when recording, the derivatives of d h / dx and d h / dy by the neighbours'
+                          // depths (kept_deriv): the adjoint's array B, whose entry of a wet cell the update
+                          // phase writes after it has read this one (no memory of their own: 32 B a cell)
     int fast;             // FP64: the mesh and the materials allow quot.cuh's quotients
     const int *order;     // [ntiles] the order of the tiles (tile_order.cu), null: plain
 };
@@ -85,8 +87,14 @@ struct HaloArgs {
 inline HaloArgs halo_args(const da_ctx *ctx) {
     const bool kact = ctx->ninst > 0 ? ctx->inst_ordinary : kact_ordinary(ctx->mc);
     return HaloArgs{ctx->mesh.halo_off, ctx->mesh.halo_idx, ctx->mesh.nloc,
-                    ctx->slopes,        ctx->fsign,         ctx->mesh.ordinary && kact ? 1 : 0,
-                    ctx->tile_ordered ? ctx->tile_order : nullptr};
+                    ctx->slopes,        ctx->fsign,         ctx->adjB,
+                    ctx->mesh.ordinary && kact ? 1 : 0,     ctx->tile_ordered ? ctx->tile_order : nullptr};
+}
+
+// The place of side q's kept derivative of cell i: the first bytes of B's own entry.
+template <class R>
+__device__ __forceinline__ R *kept_deriv(double *deriv, int q, int n, int i) {
+    return reinterpret_cast<R *>(deriv + (size_t)q * n + i);
 }
 
 // Which kernels take the tiles in the order of tile_order.cu: those of an ensemble, whose members' flows fall
@@ -719,7 +727,7 @@ __device__ __forceinline__ void coef_phase_staged(const MeshArgs &m, const HaloA
                         ha.fsign[i] = o.sgn;
                         if (RECORD)
 #pragma unroll
-                            for (int q = 0; q < 4; ++q) kept[(size_t)(5 + q) * m.n + i] = o.q[q];
+                            for (int q = 0; q < 4; ++q) *kept_deriv<R>(ha.deriv, q, m.n, i) = o.q[q];
                         const R ev = o.ev;
                         if (ev > R(1000000000.)) raise_err(sc, DA_ERR_EIGEN);
                         const unsigned long long rb = __double_as_longlong(double((dxm > dym ? dym : dxm) / ev));
