@@ -222,7 +222,8 @@ struct da_ctx {
     std::vector<int32_t> inst_npile;  // [ninst] piles of each member (0 or 1)
     void *inst_mem = nullptr;         // one allocation holding every InstArgs table
     double *inst_vol = nullptr;       // [ninst] members' volumes (stats)
-    void *inst_init[3] = {nullptr, nullptr, nullptr};  // [n] members' initial states, concatenated (restart)
+    // [n] members' initial states, concatenated (restart); null: zero everywhere
+    void *inst_init[3] = {nullptr, nullptr, nullptr};
     da::DwrState dwr;                 // error grid of the DWR indicator (da_dwr_setup)
     da::OutlineGrid outline;          // maximum-depth map (da_outline_init)
     double *stats_mem = nullptr;      // partial sums and result of the flow statistics (stats.cu)

@@ -215,11 +215,14 @@ int da_ensemble_upload(da_ctx *ctx, const da_member *members, int32_t n_members)
         ctx->inst_nmat.push_back(members[k].n_materials);
         ctx->inst_npile.push_back(members[k].dh0_dpile ? 1 : 0);
     }
-    // the initial states stay on the device for da_ensemble_restart
+    // the initial states stay on the device for da_ensemble_restart; an array of zeros (most piles
+    // start at rest) takes no memory
     const size_t rs = ctx->p.precision == DA_PREC_FP64 ? sizeof(double) : sizeof(float);
     for (int v = 0; v < 3 && !st; ++v) {
+        const double *a = init.data() + (size_t)v * N;
+        if (std::all_of(a, a + N, [](double x) { return x == 0.0 && !std::signbit(x); })) continue;
         st = cuda_check(ctx, cudaMalloc(&ctx->inst_init[v], rs * N), "cudaMalloc(initial states)");
-        if (!st) st = upload_real(ctx, ctx->inst_init[v], init.data() + (size_t)v * N);
+        if (!st) st = upload_real(ctx, ctx->inst_init[v], a);
         // the staging buffer and the host array are reused
         if (!st) st = cuda_check(ctx, cudaStreamSynchronize(ctx->stream), "sync");
     }
@@ -240,8 +243,10 @@ int da_ensemble_restart(da_ctx *ctx) {
     const size_t N = (size_t)ctx->mesh.n, rs = ctx->p.precision == DA_PREC_FP64 ? sizeof(double) : sizeof(float);
     int st = DA_OK;
     for (int v = 0; v < 3 && !st; ++v)
-        st = cuda_check(ctx, cudaMemcpyAsync(ctx->U[ctx->cur][v], ctx->inst_init[v], rs * N, cudaMemcpyDeviceToDevice,
-                                             ctx->stream), "initial states");
+        st = cuda_check(ctx, ctx->inst_init[v] ? cudaMemcpyAsync(ctx->U[ctx->cur][v], ctx->inst_init[v], rs * N,
+                                                                 cudaMemcpyDeviceToDevice, ctx->stream)
+                                               : cudaMemsetAsync(ctx->U[ctx->cur][v], 0, rs * N, ctx->stream),
+                        "initial states");
     if (!st) st = forward_state_changed(ctx);
     if (!st) ctx->have_state = true;
     if (!st) st = da_set_time(ctx, 0.0, 0);
