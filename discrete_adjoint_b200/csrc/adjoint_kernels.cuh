@@ -258,8 +258,9 @@ int reverse_grid(const da_ctx *ctx, int cap) {
 // cells in FP32 3.31 -> 3.14 ms, 24 steps of 191k wet cells 4.03 -> 3.88 ms.
 //
 // The two state buffers are tracked on their own: dirty[b] the segments of buffer b that may differ
-// from the base checkpoint, wet[b] those with a wet cell (of the base where they do not differ).
-// Afterwards the live dirty flags cover both buffers too, as the restore that follows every run expects.
+// from the base checkpoint, wet[b] those with a wet cell (of the base where they do not differ).  The
+// live dirty flags cover both buffers at every moment, as the restore that follows every run expects:
+// also the one after a run that a barrier timeout has cut short.
 constexpr int kRunMax = 32;  // steps of a launch
 
 template <class R>
@@ -275,7 +276,8 @@ struct RunArgs {
 
 // Checkpoint k of the run into state buffer b (snap_segments' division of the work).
 template <class R>
-__device__ __forceinline__ void run_restore(const RunArgs<R> &ra, int k, int b, const fwd::StatePair<R> &S, int n) {
+__device__ __forceinline__ void run_restore(const RunArgs<R> &ra, int k, int b, const fwd::StatePair<R> &S, int n,
+                                            uint8_t *seg_dirty) {
     const int lane = threadIdx.x & 31;
     const int W = (gridDim.x * blockDim.x) >> 5;
     const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -291,6 +293,7 @@ __device__ __forceinline__ void run_restore(const RunArgs<R> &ra, int k, int b, 
             flag = !is_base && snap_dirty[s] != 0;
             work = flag || dirty[s];
             if (work) dirty[s] = flag;
+            if (flag) seg_dirty[s] = 1;
         }
         unsigned bits = __ballot_sync(0xffffffffu, work);
         const unsigned from = __ballot_sync(0xffffffffu, flag);
@@ -335,7 +338,7 @@ __global__ void __launch_bounds__(kBlock, OCC) k_reverse_run(MeshArgs m, fwd::St
     // the first step's state: live (its wet flags too), or its checkpoint after a barrier
     if (ra.slot[0]) {
         if (!fwd::grid_sync(sc)) return;
-        run_restore<R>(ra, 0, cur, S, m.n);
+        run_restore<R>(ra, 0, cur, S, m.n, seg_dirty);
         fl.store(ha, first);
         if (!fwd::grid_sync(sc)) return;
     } else {
@@ -377,7 +380,7 @@ __global__ void __launch_bounds__(kBlock, OCC) k_reverse_run(MeshArgs m, fwd::St
         gather_staged<R, false>(m, ha, U, Ln, Lo, mc, aa, rec_id, dt, list, InstArgs{}, dyn_smem,
                                 gather_quarters(sc, gsplit), first);
         if (k + 1 < ra.n) {
-            run_restore<R>(ra, k + 1, p ^ 1, S, m.n);
+            run_restore<R>(ra, k + 1, p ^ 1, S, m.n, seg_dirty);
             if (!fwd::grid_sync(sc)) return;
         } else if (blockIdx.x == 0 && threadIdx.x == 0) {
             // the last step's scalars, as a launch of its own leaves them
@@ -391,9 +394,6 @@ __global__ void __launch_bounds__(kBlock, OCC) k_reverse_run(MeshArgs m, fwd::St
             sc->acc_hmax = sc->acc_alt_hmax = 0ull;
         }
     }
-    // Every segment that either buffer or the flags of the live state differ on from the base (the last
-    // restores wrote theirs before a barrier).
-    for (int s = t0; s < ra.nseg; s += nt) seg_dirty[s] |= ra.dirty[0][s] | ra.dirty[1][s];
     fwd::grid_exit(sc);
 }
 
