@@ -254,14 +254,10 @@ __device__ __forceinline__ void flux_div(const V &v, int i, uint8_t bf, const R 
 }
 
 // Full corrector update of one active cell (fluxes + sources), reference order.  c is the cell in
-// the view; cs its source coefficients (read only for a wet cell, h > GEOFLOW_TINY); hook(f,
-// clamped) runs for a wet cell with the slopes, velocities and friction signs of its sources.
-// pre_s (or null): the cell's limited slopes as the coefficient phase computed them from the same
-// state (the same bits cell_slopes gives here).
-template <class R, class V, class Hook = NoSrcHook>
+// the view; cs its source coefficients (read only for a wet cell, h > GEOFLOW_TINY).
+template <class R, class V>
 __device__ __forceinline__ bool update_cell(const V &v, int c, uint8_t bf, const CellSrc<R> &cs, const MatConsts &mc,
-                                            R dt, R ft, const R prev[3], R dxc, R dyc, R st[3],
-                                            const R *pre_s = nullptr, const Hook &hook = Hook{}) {
+                                            R dt, R ft, const R prev[3], R dxc, R dyc, R st[3]) {
     const R ki = prev[0] >= R(DA_TINY) ? v.k(c) : R(0);
     const R gz = v.gz(c);
     const R g0 = cs.g[0], g1 = cs.g[1], dg0 = cs.dg[0], dg1 = cs.dg[1], cv0 = cs.cv[0], cv1 = cs.cv[1];
@@ -282,12 +278,7 @@ __device__ __forceinline__ bool update_cell(const V &v, int c, uint8_t bf, const
     if (clamped) st[0] = R(0);
     if (prev[0] > R(DA_TINY)) {
         R s[6];
-        if (pre_s) {
-#pragma unroll
-            for (int j = 0; j < 6; ++j) s[j] = pre_s[j];
-        } else {
-            cell_slopes<R>(v, c, bf, R(mc.gamma), prev, s);
-        }
+        cell_slopes<R>(v, c, bf, R(mc.gamma), prev, s);
         R vel0, vel1, h_inv;
         if constexpr (sizeof(R) == 8) {
             vel0 = prev[1] / prev[0];
@@ -304,16 +295,14 @@ __device__ __forceinline__ bool update_cell(const V &v, int c, uint8_t bf, const
         tmp = h_inv * (s[2] - vel1 * s[0]);
         const R sg1 = tiny_sgn(tmp, ft);
         const R sg3 = tiny_sgn(vel1, ft);
-        // the reverse step's source adjoint of this cell, from these same values (its branches)
-        hook(SrcFwd<R>{{s[0], s[1], s[2], s[3], s[4], s[5]}, vel0, vel1, h_inv, sg0, sg1, sg2, sg3}, clamped);
         const R sin_int = R(mc.sin_int);
         const R tan_bed = R(mc.tan_bed[mat]);
         R s1 = g0 * prev[0];
-        R s2 = sg0 * prev[0] * ki * (gz * s[3] + dg1 * prev[0]) * sin_int;
+        R s2 = sg0 * prev[0] * ki * slope_term(gz, s[3], dg1, prev[0]) * sin_int;
         R s3 = sg2 * rmax(gz * prev[0] + vel0 * prev[1] * cv0, R(0.0)) * tan_bed;
         st[1] += dt * (s1 - s2 - s3);
         s1 = g1 * prev[0];
-        s2 = sg1 * prev[0] * ki * (gz * s[0] + dg0 * prev[0]) * sin_int;
+        s2 = sg1 * prev[0] * ki * slope_term(gz, s[0], dg0, prev[0]) * sin_int;
         s3 = sg3 * rmax(gz * prev[0] + vel1 * prev[2] * cv1, R(0.0)) * tan_bed;
         st[2] += dt * (s1 - s2 - s3);
     }

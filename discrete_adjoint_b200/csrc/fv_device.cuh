@@ -134,11 +134,16 @@ struct SrcFwd {
     R sg0, sg1, sg2, sg3;
 };
 
-// No hook (the forward alone).
-struct NoSrcHook {
-    template <class... A>
-    __device__ __forceinline__ void operator()(A &&...) const {}
-};
+// g_z ds + dg h of the internal friction.  FP32 contracts it; which of the two products is rounded would be
+// the compiler's choice at each place, so it is spelled out for the staged and the global update (the same
+// bits in both).
+template <class R>
+__device__ __forceinline__ R slope_term(R gz, R ds, R dg, R h) {
+    if constexpr (sizeof(R) == 8)
+        return gz * ds + dg * h;
+    else
+        return __fmaf_rn(dg, h, __fmul_rn(gz, ds));
+}
 
 // What the per-cell numerics read about a cell and its neighbours goes through a view: nb(s, c)
 // the cell across neighbour entry s of cell c, and the values of a cell.  GlobalView reads the

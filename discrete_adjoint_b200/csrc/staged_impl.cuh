@@ -376,7 +376,7 @@ struct Divisor<float, FAST> {
 };
 
 // cell_slopes (fv_device.cuh, FP64) with one divisor per centre distance.  DERIV: also the derivatives
-// of the depth slopes by the depth across each side, q[s] (h_slope_deriv, adjoint_impl.cuh: the
+// of the depth slopes by the depth across each side, q[s] (h_slope_deriv, fv_device.cuh: the
 // slope's derivative by dp or dm over the centre distance).
 template <bool FAST, bool DERIV>
 __device__ __forceinline__ void staged_slopes64(const StagedView<double> &v, int i, uint8_t bf, double gamma,
@@ -589,16 +589,6 @@ struct Kept {
     R sx, sy;  // depth slopes
     uint8_t sgn;
 };
-
-// g_z ds + dg h of the internal friction; FP32 with the one rounding that the compiler's contraction gives
-// update_cell (which of the two products is rounded is its choice, so it is spelled out here).
-template <class R>
-__device__ __forceinline__ R slope_term(R gz, R ds, R dg, R h) {
-    if constexpr (sizeof(R) == 8)
-        return gz * ds + dg * h;
-    else
-        return __fmaf_rn(dg, h, __fmul_rn(gz, ds));
-}
 
 // update_cell (forward_impl.cuh) of an active cell from the staged and kept values.
 template <class R, bool FAST, class Hook>
