@@ -199,31 +199,36 @@ def bytes_per_cell_update(precision: str) -> dict:
     return {"forward": 6 * r + statics + 10 * r + 2, "adjoint": 9 * r + statics + 1 + 8 * r}
 
 
+# the launches of reverse steps, which the trace counts together: runs of them (k_reverse_run; 31 of the
+# headline's 32) and single ones (k_youturn)
+REVERSE = "k_reverse_run + k_youturn"
+
+
 def algorithmic_bytes(precision: str, n_act: float) -> dict:
     """Algorithmic bytes of one launch of each kernel per time step it covers, over the cells the
     step actually processes (n_act: wet cells and their face neighbours; tile culling leaves the
-    others untouched): k_steps one forward step, k_youturn one reverse step (the replayed forward
+    others untouched): k_steps one forward step, REVERSE one reverse step (the replayed forward
     step and the adjoint step), a checkpoint copy the state of those cells each way."""
     b = bytes_per_cell_update(precision)
     r = 8 if precision == "fp64" else 4
-    return {"k_steps": b["forward"] * n_act, "k_youturn": (b["forward"] + b["adjoint"]) * n_act,
+    return {"k_steps": b["forward"] * n_act, REVERSE: (b["forward"] + b["adjoint"]) * n_act,
             "snapshot_copy": 2 * 3 * r * n_act}
 
 
 # DRAM bytes (read + write) from the committed ncu captures (the headline traffic and the dense
 # k_steps summaries under profiles/).  Sparse headline kernels: bytes per active cell and step of a
-# launch captured in the steady flow (k_youturn, i.e. the launches of reverse steps: one k_reverse_run of
+# launch captured in the steady flow (reverse steps: one k_reverse_run of
 # the 23 steps of iterations 258 to 236 of the 512-step sweep, 4272 active cells per step on average;
 # k_steps: one launch of 32 steps after 256, 4553 active cells per step on average), scaled by the active
 # cells of the traced run; the dense case: bytes per time step of a 10-step launch with every cell wet.
 TRAFFIC_PER_ACTIVE_CELL = {
-    ("fp64", "k_youturn"): (5538048 + 94464) / (23 * 4271.6),
-    ("fp32", "k_youturn"): (3543296 + 55808) / (23 * 4271.1),
-    ("fp64", "k_steps"): (1582848 + 20736) / (32 * 4552.6),
+    ("fp64", REVERSE): (5517056 + 96768) / (23 * 4271.6),
+    ("fp32", REVERSE): (3655424 + 90112) / (23 * 4271.1),
+    ("fp64", "k_steps"): (1583104 + 25600) / (32 * 4552.6),
 }
 TRAFFIC_DENSE_PER_STEP = {
-    "fp32": (5.144700e9 + 1.404057e9) / 10,
-    "fp64": (9.414111e9 + 2.799996e9) / 10,
+    "fp32": (5.144393e9 + 1.404350e9) / 10,
+    "fp64": (9.412916e9 + 2.800689e9) / 10,
 }
 
 
@@ -364,7 +369,7 @@ def fwdadj(args, ws, local):
         # per-kernel device times of one traced run
         c.set_tracing(True)
         adjoint_run(c, box, HORIZON, SNAPSHOTS, m.dh0_dpile)
-        res["trace"] = c.trace(with_steps=True)
+        res["trace"] = {REVERSE if k == "k_youturn" else k: v for k, v in c.trace(with_steps=True).items()}
         c.set_tracing(False)
         # e2e through the C ABI with pinned host buffers: H2D of the initial state and the pile
         # derivative, the run, D2H of the gradients and lambda^0

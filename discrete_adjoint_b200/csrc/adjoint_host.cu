@@ -213,11 +213,9 @@ struct Runner {
         pending = slot;
         return st;
     }
-    // Consecutive forward advances (a chain of checkpoint stores between a restore and the next
-    // reverse step) go out as one multi-step launch that stores the checkpoints on its way: the
-    // advances wait here until a restore, a reverse step or the end of the sweep needs the state.
-    // The tiles in a new order, from the flags of the last step that ran, before a chain of forward steps:
-    // a flow needs some ten steps to cross a tile.
+    // The tiles in a new order before a chain of forward steps, from the live flags: those of the last
+    // chain's end or the last restore (runs of reverse steps write none of them), which may be some steps
+    // older than the state; a flow needs some ten steps to cross a tile.
     static constexpr int kOrderSteps = 64;
     long long ordered_at = 0;
     int order_tiles() {
@@ -225,6 +223,9 @@ struct Runner {
         ordered_at = fsteps;
         return launch_tile_order(ctx);
     }
+    // Consecutive forward advances (a chain of checkpoint stores between a restore and the next
+    // reverse step) go out as one multi-step launch that stores the checkpoints on its way: the
+    // advances wait here until a restore, a reverse step or the end of the sweep needs the state.
     int def_k = 0;
     void *def_pre = nullptr;
     MidStoreList def_mid;

@@ -6,8 +6,8 @@
 // reciprocal of its own each time and a range test with a branch, which also keeps the compiler from
 // interleaving neighbouring quotients: one after another they are most of a cell's latency.  Here
 // the reciprocal is formed once per divisor (an estimate and three Newton steps) and each quotient is one
-// multiplication and four fused multiply-adds (both as in Markstein, "Computation of elementary functions on the IBM RISC System/6000
-// processor", IBM J. Res. Dev. 34, 1990):
+// multiplication and four fused multiply-adds (both as in Markstein, "Computation of elementary functions on
+// the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990):
 //   q0 = a y,  r0 = b q0 - a,  q1 = q0 - r0 y,  r1 = b q1 - a,  q = q1 - r1 y.
 // With y within half an ulp of 1/b, q1 is within one ulp of a/b; then r1 is exact, and q is a/b
 // rounded to nearest: where a/b lies next to the middle m of two neighbours, q1 is half an ulp
