@@ -5,9 +5,9 @@
 // bits need every quotient rounded as the division operator rounds it.  The operator costs a
 // reciprocal of its own each time and a range test with a branch, which also keeps the compiler from
 // interleaving neighbouring quotients: one after another they are most of a cell's latency.  Here
-// the reciprocal is formed once per divisor (an estimate and three Newton steps) and each quotient is one
-// multiplication and four fused multiply-adds (both as in Markstein, "Computation of elementary functions on
-// the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990):
+// the reciprocal is formed once per divisor and each quotient is one multiplication and four fused
+// multiply-adds (Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor",
+// IBM J. Res. Dev. 34, 1990):
 //   q0 = a y,  r0 = b q0 - a,  q1 = q0 - r0 y,  r1 = b q1 - a,  q = q1 - r1 y.
 // With y within half an ulp of 1/b, q1 is within one ulp of a/b; then r1 is exact, and q is a/b
 // rounded to nearest: where a/b lies next to the middle m of two neighbours, q1 is half an ulp
@@ -21,7 +21,7 @@
 // zero or within [2^-760, 2^760], every divisor within [2^-250, 2^250] and every quotient zero or above
 // 2^-910.  Anything else takes the division operator.
 //
-// Three quotients of one divisor, chained, one warp: 118 cycles a round against 382 with the operator.
+// Three quotients of one divisor, chained, one warp: 112 cycles a round against 382 with the operator.
 #pragma once
 #include <stdint.h>
 
@@ -47,15 +47,18 @@ DA_QUOT_FN double mul(double a, double b) { return a * b; }
 DA_QUOT_FN double mul_add(double a, double b, double c) { return std::fma(a, b, c); }
 #endif
 
-// Newton's step for 1/b: the relative error e of y becomes e^2 before rounding.
-DA_QUOT_FN double newton(double b, double y) { return mul_add(mul_add(-b, y, 1.0), y, y); }
-
-// 1/b from an estimate y0 by three Newton steps (the reciprocal iteration of the same paper).  The hardware's
-// estimate is documented to read the upper 32 bits of b and to return the upper 32 bits of its result, the
-// others zero: each cut costs up to 2^-20, taken as 2^-19 in all.  Two steps leave 2^-76 before
-// rounding, hence y within an ulp; the third starts there, its own residual is exact, and it leaves 2^-105
-// before rounding, which is y within half an ulp (and 2^-53 of that).
-DA_QUOT_FN Recip refine(double b, double y0) { return Recip{b, newton(b, newton(b, newton(b, y0)))}; }
+// 1/b from an estimate y0.  The hardware's is documented to read the upper 32 bits of b and to return the
+// upper 32 bits of its result, the others zero: each cut costs up to 2^-20, taken as |e| < 2^-19 in all.
+// Two steps of Goldschmidt's iteration (Applications of division by convergence, MIT, 1964: y (1 + e) (1 + e^2),
+// whose factors do not wait for one another) leave e^4 < 2^-76 and the rounding of two results, an ulp; a
+// Newton step (Markstein's, as above) from there leaves 2^-104 before its own rounding, which is y within
+// half an ulp (and 2^-51 of that).  Three Newton steps are one multiply-add longer in their chain.
+DA_QUOT_FN Recip refine(double b, double y0) {
+    const double e = mul_add(-b, y0, 1.0);
+    const double y1 = mul_add(e, y0, y0), e2 = mul(e, e);
+    const double y2 = mul_add(e2, y1, y1);
+    return Recip{b, mul_add(mul_add(-b, y2, 1.0), y2, y2)};
+}
 
 // a / b, rounded to nearest
 DA_QUOT_FN double div(double a, const Recip &r) {
