@@ -18,9 +18,10 @@
 // FP64 quotients that share a divisor are formed branch-free (quot.cuh) as long as every staged state is ordinary
 // there (tested as the copies land, folded into the tile's barrier); a tile with any other value, and
 // a mesh or material outside the range, takes the division operator.  The results are the
-// reference's bits either way (FP32: the unstaged phases' bits).  Bound: not memory (740k wet cells: a third of HBM's rate) but the
+// reference's bits either way (FP32: the unstaged phases' bits).  A recording step also keeps the depth
+// slopes' derivatives for the source adjoint (kept_deriv).  Bound: not memory (740k wet cells: a third of HBM's rate) but the
 // instructions and the latency of one warp's FP64 chain.  46 divisions and 6 square roots per cell and
-// step became 13 divisors and 2 square roots: 2894 -> 2050 instructions per warp and step, 125 -> 95 us
+// step became 13 divisors and 2 square roots: 2894 -> 2060 instructions per warp and step, 125 -> 95 us
 // per step on 740k wet cells (2 x 296 blocks), 14.0 -> 10.7 us on a flow of 18 tiles.  Three blocks
 // per SM with one buffer each (80 registers) took 100 us.  FP32 (approximate quotients): 1650 -> 1380
 // instructions, 137 -> 133 us on 2.1M wet cells (2 x 296 blocks), a flow on 262k cells 15.4 -> 13.9 us per
