@@ -71,12 +71,12 @@ int reduce_inst_t(da_ctx *ctx, int lam0) {
     const MeshArgs m = mesh_args(ctx);
     StateRef<R> L{(const R *)ctx->lam[lam0][0], (const R *)ctx->lam[lam0][1], (const R *)ctx->lam[lam0][2]};
     trace_begin(ctx, TR_ADJ_REDUCE);
-    const int nout = ctx->p.n_materials + 2, n = ctx->ninst * nout;
+    const int nout = ctx->inst_mat + 2, n = ctx->ninst * nout;
     // a launch takes at most 65535 members across
     for (int k0 = 0; k0 < ctx->ninst; k0 += 65535) {
         const int nk = ctx->ninst - k0 < 65535 ? ctx->ninst - k0 : 65535;
         k_adj_reduce_inst<R><<<dim3(kInstParts, nk, nout), kBlock, 0, ctx->stream>>>(
-            m, L, ctx->gbed, ctx->gint, ctx->dh0, ctx->p.n_materials, ctx->ia.seg0 + k0,
+            m, L, ctx->gbed, ctx->gint, ctx->dh0, ctx->inst_mat, ctx->ia.seg0 + k0,
             ctx->red_part + (size_t)k0 * nout * kInstParts);
     }
     k_adj_reduce_inst_final<<<(n * 32 + kBlock - 1) / kBlock, kBlock, 0, ctx->stream>>>(ctx->red_part, n, ctx->red_out);

@@ -219,6 +219,7 @@ struct da_ctx {
     std::vector<int32_t> inst_cell0;  // [ninst + 1] first cell of each member (multiple of 256)
     std::vector<int32_t> inst_ncell;  // [ninst] cells of each member before padding
     std::vector<int32_t> inst_nmat;   // [ninst] materials of each member
+    int inst_mat = 0;                 // the most of them, whatever the parameters are set to later
     std::vector<int32_t> inst_npile;  // [ninst] piles of each member (0 or 1)
     void *inst_mem = nullptr;         // one allocation holding every InstArgs table
     double *inst_vol = nullptr;       // [ninst] members' volumes (stats)

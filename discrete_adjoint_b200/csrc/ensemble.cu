@@ -209,6 +209,7 @@ int da_ensemble_upload(da_ctx *ctx, const da_member *members, int32_t n_members)
     ia.seg0 = (const int32_t *)(b + o_seg0);
     ctx->ninst = nm;
     ctx->inst_ordinary = ordinary;
+    ctx->inst_mat = max_mat;
     ctx->inst_cell0 = cell0;
     for (int k = 0; k < nm; ++k) {
         ctx->inst_ncell.push_back(members[k].mesh.n_cells);
@@ -326,7 +327,7 @@ int da_ensemble_adjoint(da_ctx *ctx, int32_t nsteps, int32_t nsnapshots, da_grad
     if (ctx->p.jacobian_mode != DA_JAC_EXACT)
         return set_error(ctx, DA_ERR_UNSUPPORTED, "da_ensemble_adjoint: ensembles use the exact adjoint");
     cudaSetDevice(ctx->device);
-    const int nm = ctx->ninst, nout = ctx->p.n_materials + 2;
+    const int nm = ctx->ninst, nout = ctx->inst_mat + 2;
     int lam0 = 0;
     long long fsteps = 0;
     float ms = 0.f;
@@ -340,8 +341,8 @@ int da_ensemble_adjoint(da_ctx *ctx, int32_t nsteps, int32_t nsnapshots, da_grad
         std::memset(&g, 0, sizeof(g));
         g.J = J[k];
         for (int m = 0; m < ctx->inst_nmat[k]; ++m) g.dJ_dbedfrict[m] = red[(size_t)k * nout + m];
-        g.dJ_dintfrict = red[(size_t)k * nout + ctx->p.n_materials];
-        if (ctx->inst_npile[k]) g.dJ_dpile[0] = red[(size_t)k * nout + ctx->p.n_materials + 1];
+        g.dJ_dintfrict = red[(size_t)k * nout + ctx->inst_mat];
+        if (ctx->inst_npile[k]) g.dJ_dpile[0] = red[(size_t)k * nout + ctx->inst_mat + 1];
         g.forward_steps = fsteps;
         g.snapshots = nsnapshots;
         g.device_ms = ms;
